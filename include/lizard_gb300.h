@@ -112,15 +112,15 @@ int lizg_ldpc_decode_noalloc(const int8_t *d_llr, const int32_t *d_rate, int cou
 
 // No counterpart in the reference (its decoder has one form a build): the decoder's kernel variants and their
 // choice. Each code has a few variants that decode bit for bit alike and differ in the warps a codeword takes (1, 2
-// or 4) and in the layer form (messages held in registers, or recomputed in a loop). Variant 0 is the default on
-// every device. lizg_ldpc_autotune times every variant of every code on the current device over a seeded batch of
+// or 4) and in the layer form (two codewords at once, messages held in registers, or recomputed in a loop). Variant 0
+// is the default on every device. lizg_ldpc_autotune times every variant of every code on the current device over a seeded batch of
 // `count` codewords, codeword c at ebn0_db[c mod n_ebn0] (BPSK/AWGN, the batch's LLR quantisation), and keeps the
 // fastest per code for that device; choice[4] (may be NULL) receives the indices in code order 7/8, 3/4, 2/3, 1/2.
 // Every later decode on the device (plans, the single-codeword call, the receiver, the allocation-free call) uses
 // the kept variant.
 // lizg_ldpc_set_variant fixes one by hand; lizg_ldpc_variant returns the current index and its warps a codeword and
-// form (bit 0: the loop form; bit 1: the pair form, two checks a thread in 16-bit halves); lizg_ldpc_variants the
-// number of variants of a rate.
+// form (bit 0: the loop form; bit 1: the pair form, two checks a thread in 16-bit halves; bit 2: the two-codeword form,
+// two codewords a CTA of four warps in 16-bit halves); lizg_ldpc_variants the number of variants of a rate.
 int lizg_ldpc_autotune(int count, const float *ebn0_db, int n_ebn0, int32_t *choice);
 int lizg_ldpc_variants(int rate);
 int lizg_ldpc_variant(int rate, int32_t *wpc, int32_t *loop_form);

@@ -1,17 +1,18 @@
 // Layered normalised min-sum LDPC decoding of the four LIZARD codes plus the block's CRC-32C check, on sm_103a.
 //
-// A codeword is decoded by a group of 1, 2 or 4 warps. A block row (a layer) has z = 128 checks that share no bit;
-// in the scalar form lane l of the group's warp w takes checks l + 32 t of every layer (t over the warp's share of
-// 0..3) and keeps their min1 / min2 / sign in registers between the layer's two passes; in the pair form a thread
-// takes checks i and i + 64 as the two 16-bit halves of one register (the layout is described at layer_pair). The
-// codeword's posteriors (int16) and check-to-bit messages (int8) live in the group's slice of shared memory for the
-// whole decode; global memory is touched once to read the LLRs and once to write the packed hard bits, so the
-// kernel is bound by the ALU pipe (every min/max form issues there) and shared-memory latency, not by HBM.
+// A block row (a layer) has z = 128 checks that share no bit. In the two-codeword form, the default, a CTA of 128
+// threads decodes two codewords at once in the halves of f16x2 registers, a check a thread (described at layer_dual).
+// In the integer forms a codeword is decoded by a group of 1, 2 or 4 warps: in the scalar form lane l of the group's
+// warp w takes checks l + 32 t of every layer (t over the warp's share of 0..3) and keeps their min1 / min2 / sign in
+// registers between the layer's two passes; in the pair form a thread takes checks i and i + 64 as the two 16-bit
+// halves of one register (the layout is described at layer_pair). In every form the codeword's posteriors and
+// check-to-bit messages live in shared memory for the whole decode; global memory is touched once to read the LLRs
+// and once to write the packed hard bits, so the kernels are bound by instruction issue, not by HBM.
 //
-// Persistent grid: one CTA per SM (its shared memory holds as many codewords as fit), groups pull codeword indices
-// from a work counter, so codewords that stop early free their group for the next one. Each code has several
-// variants (warps a codeword, registers or a loop over the row's slots, scalar or pair form), all bit-identical;
-// one per code runs, chosen by timing on the device or by hand.
+// Persistent grid (as many CTAs as an SM's shared memory holds): codeword indices come from a work counter, so
+// codewords that stop early free their place for the next one. Each code has several variants (the two-codeword form;
+// the integer forms by warps a codeword, registers or a loop over the row's slots, scalar or pair), all
+// bit-identical; one per code runs, the default, or chosen by timing on the device or by hand.
 //
 // Arithmetic: the reference's four-times kernel, liblizard/src/ldpc.c:340-423 (and its NEON original, 300-328):
 // the extrinsic L - R saturated to a byte held at [-127, 127]; min1/min2 over byte magnitudes; (x * 13) >> 4 capped
@@ -735,6 +736,432 @@ __global__ void __launch_bounds__(kMixThreads, 1) ldpc_mixed_kernel(const __grid
   }
 }
 
+// ---------------------------------------------------------------- the two-codeword form
+//
+// A CTA of 128 threads decodes two codewords of one code at a time, thread i owning check i of every layer, the two
+// codewords riding in the halves of f16x2 registers. Every value of the decode is a whole number of magnitude under
+// 2048 (a posterior is its LLR plus at most 11 messages of magnitude 103 or less), so half precision holds it exactly
+// and the decode is the integer form's bit for bit. What the halves buy, per edge of both codewords:
+//   - min.xorsign.abs gives the least magnitude and the sign product in one instruction, max.xorsign.abs the other
+//     half of the second minimum: three instructions an edge for both minima and the sign;
+//   - the choice between the two scaled minima is s2 - sat(|q| - min1) (s2 - s1), on the FMA pipe (the magnitudes are
+//     whole, so the saturated difference is 0 at the least magnitude and 1 elsewhere), the check's sign folded in;
+//   - no half is swapped or sign-extended: both codewords' columns sit in one word of shared memory.
+// Messages are a byte a codeword (+128), two edges of two codewords a word of shared memory. A layer's code is the same
+// for every row (its circulants read from constant memory, uniform over the CTA): with the rows unrolled and the
+// messages in registers instead, 30-80 KB of code, the instruction fetch bound the kernel (no_instruction the top
+// stall; the 1/2 code 3.75 ms on the case below).
+//
+// Bound: instruction issue (62-77% of cycles issue, ALU pipe 43-56%, shared memory 45%), 25 instructions an edge of
+// two codewords against 37-58 an edge of one in the integer forms. Measured, 16,384 codewords of one code at Eb/N0
+// 1.0-4.0 dB, the best integer form and this one, ms: 7/8 4.77, 1.71; 3/4 4.37, 1.71; 2/3 4.01, 1.79; 1/2 4.14, 2.31;
+// and 12 codewords (one a CTA, latency alone), us: 410, 73; 384, 93; 323, 112; 310, 128.
+__device__ __forceinline__ uint32_t hadd2(uint32_t a, uint32_t b) { uint32_t d; asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
+__device__ __forceinline__ uint32_t hsub2(uint32_t a, uint32_t b) { uint32_t d; asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
+__device__ __forceinline__ uint32_t hsub2_sat(uint32_t a, uint32_t b) { uint32_t d; asm("sub.rn.sat.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
+__device__ __forceinline__ uint32_t hmul2(uint32_t a, uint32_t b) { uint32_t d; asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
+__device__ __forceinline__ uint32_t hfma2(uint32_t a, uint32_t b, uint32_t c) { uint32_t d; asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c)); return d; }
+__device__ __forceinline__ uint32_t hfma2_sat(uint32_t a, uint32_t b, uint32_t c) { uint32_t d; asm("fma.rn.sat.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c)); return d; }
+__device__ __forceinline__ uint32_t habs2(uint32_t a) { uint32_t d; asm("abs.f16x2 %0, %1;" : "=r"(d) : "r"(a)); return d; }
+__device__ __forceinline__ uint32_t hmin2(uint32_t a, uint32_t b) { uint32_t d; asm("min.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
+// magnitudes compared, the result's sign the product of both signs
+__device__ __forceinline__ uint32_t hminx2(uint32_t a, uint32_t b) { uint32_t d; asm("min.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
+__device__ __forceinline__ uint32_t hmaxx2(uint32_t a, uint32_t b) { uint32_t d; asm("max.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
+__device__ __forceinline__ uint32_t prmt2(uint32_t a, uint32_t b, uint32_t s) { uint32_t d; asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(s)); return d; }
+
+constexpr int kDualThreads = 128;
+constexpr uint32_t kH1152 = 0x64806480u, kH1024 = 0x64006400u, kH127 = 0x57F057F0u, kHSign = 0x80008000u;
+constexpr uint32_t kHm13 = 0xCA80CA80u, kH13_16 = 0x3A803A80u, kH16 = 0x4C004C00u, kHBytes = 0x64646464u;
+
+// Circulants as the two-codeword layers read them, uniform over the CTA, two an entry: (x, y) and (z, w) each a column's
+// byte offset in the posteriors and the shift in bytes; rows of (NDMAX + 1) / 2 entries, what a row lacks unused.
+__constant__ uint4 c_dual[5 * 11 + 10 * 7 + 15 * 5 + 30 * 3];
+template <int C> __host__ __device__ constexpr int dual_first() { return C == 0 ? 0 : C == 1 ? 55 : C == 2 ? 125 : 200; }
+__host__ __device__ constexpr uint32_t full_rows(const uint8_t *rowptr, int mb, int ndmax) {
+  uint32_t m = 0;
+  for (int r = 0; r < mb; r++)
+    if (rowptr[r + 1] - rowptr[r] == ndmax) m |= 1u << r;
+  return m;
+}
+// The rows that have all NDMAX circulants.
+template <int C> struct FullRows {
+  static constexpr uint32_t mask = full_rows(C == 0 ? LIZG_R78_ROWPTR : C == 1 ? LIZG_R34_ROWPTR : C == 2 ? LIZG_R23_ROWPTR : LIZG_R12_ROWPTR,
+                                             Code<C>::MB, Code<C>::NDMAX);
+  static constexpr bool all = mask == (uint32_t)((1ull << Code<C>::MB) - 1);
+};
+// A row's message words: the staircase's two slots, then the circulants two a word.
+template <int C> __host__ __device__ constexpr int row_words() { return 1 + (Code<C>::NDMAX + 1) / 2; }
+
+// floor(13 m / 16) of both halves, m whole in 0..127: 13 m / 16 rounded to a whole number, less one where that rounded up.
+__device__ __forceinline__ uint32_t scaled13(uint32_t m) {
+  const uint32_t r = hsub2(hfma2(m, kH13_16, kH1024), kH1024);
+  return hsub2(r, hfma2_sat(r, kH16, hmul2(m, kHm13)));
+}
+// Edge k's (0 or 1) messages of a word, as whole numbers.
+template <int K>
+__device__ __forceinline__ uint32_t message(uint32_t w) { return hsub2(prmt2(w, kHBytes, K ? 0x4342u : 0x4140u), kH1152); }
+
+// What a thread needs of a layer before the posteriors: the byte offsets of its columns and its messages.
+template <int C> struct RowFetch {
+  uint32_t at[Code<C>::NDMAX], R[row_words<C>()];
+};
+template <int C>
+__device__ __forceinline__ void fetch_row(RowFetch<C> &x, const uint32_t *R, int r, uint32_t i4) {
+  constexpr int ND = Code<C>::NDMAX;
+#pragma unroll
+  for (int e = 0; e < ND; e += 2) {
+    const uint4 c = c_dual[dual_first<C>() + r * ((ND + 1) / 2) + e / 2];
+    x.at[e] = ((i4 - c.y) & 508u) | c.x;
+    if (e + 1 < ND) x.at[e + 1 < ND ? e + 1 : 0] = ((i4 - c.w) & 508u) | c.z;
+  }
+#pragma unroll
+  for (int w = 0; w < row_words<C>(); w++) x.R[w] = R[(r * row_words<C>() + w) * 128];
+}
+
+// Layer r for thread i's check of both codewords. L: the posteriors (a word a column, the codewords in its halves); R:
+// the thread's messages; x: the layer's fetch, replaced by layer rn's before the call ends (its messages, which are
+// the thread's own, and its columns' places, so that only the posteriors are left to read past the barrier).
+template <int C>
+__device__ __forceinline__ void layer_dual(uint32_t *L, uint32_t *R, RowFetch<C> &x, int r, int rn, int i) {
+  using T = Code<C>;
+  constexpr int ND = T::NDMAX;
+  uint8_t *Lb = reinterpret_cast<uint8_t *>(L);
+  const bool last = FullRows<C>::all || ((FullRows<C>::mask >> r) & 1);
+  uint32_t *own = L + T::K + r * 128 + i;
+  uint32_t *prev = r > 0 ? own - 128 : L + T::K + (T::MB - 1) * 128 + ((i - 1) & 127);
+  uint32_t q[ND + 2];
+  q[ND] = hsub2(*prev, message<0>(x.R[0]));
+  if (r == 0 && i == 0) q[ND] = kH1024;   // check 0 has no previous parity bit: a certain zero, past every cap
+  q[ND + 1] = hsub2(*own, message<1>(x.R[0]));
+  uint32_t a1 = q[ND], a2 = kH127, b1 = q[ND + 1], b2 = kH127;   // the second least's cap from the start
+#pragma unroll
+  for (int e = 0; e < ND; e++) {
+    if (e < ND - 1 || last) {
+      const uint32_t l = *reinterpret_cast<uint32_t *>(Lb + x.at[e]), w = x.R[1 + e / 2];
+      const uint32_t v = hsub2(l, (e & 1) ? message<1>(w) : message<0>(w));
+      q[e] = v;
+      if (e & 1) { b2 = hminx2(b2, hmaxx2(b1, v)); b1 = hminx2(b1, v); }
+      else { a2 = hminx2(a2, hmaxx2(a1, v)); a1 = hminx2(a1, v); }
+    }
+  }
+  const uint32_t m1s = hminx2(a1, b1), sg = m1s & kHSign;
+  const uint32_t m1 = hmin2(habs2(m1s), kH127), m2 = habs2(hminx2(hmaxx2(a1, b1), hminx2(a2, b2)));
+  const uint32_t s1 = scaled13(m1), s2 = scaled13(m2);
+  const uint32_t s2s = s2 ^ sg, nds = hsub2(s1, s2) ^ sg;   // the check's sign folded in
+  // an edge's message: s2 where its magnitude is the least, else s1, times the other edges' signs; held biased
+  uint32_t hb = 0;
+  auto send = [&](uint32_t v) -> uint32_t {
+    const uint32_t m = hfma2(nds, hsub2_sat(habs2(v), m1), s2s) ^ (v & kHSign);
+    hb = hadd2(m, kH1152);
+    return hadd2(v, m);
+  };
+  uint32_t *Rr = R + r * row_words<C>() * 128;
+#pragma unroll
+  for (int e = 0; e < ND; e += 2) {
+    if (e < ND - 1 || last) {
+      *reinterpret_cast<uint32_t *>(Lb + x.at[e]) = send(q[e]);
+      const uint32_t h0 = hb;
+      if (e + 1 < ND && (e + 1 < ND - 1 || last)) *reinterpret_cast<uint32_t *>(Lb + x.at[e + 1]) = send(q[e + 1]);
+      Rr[(1 + e / 2) * 128] = prmt2(h0, hb, 0x6420u);
+    }
+  }
+  const uint32_t lp = send(q[ND]), h0 = hb;
+  if (r > 0 || i != 0) *prev = lp;   // check 0's would be another check's column
+  *own = send(q[ND + 1]);
+  Rr[0] = prmt2(h0, hb, 0x6420u);
+  fetch_row<C>(x, R, rn, 4 * i);
+}
+
+// The sign bits (15 and 31) set where check i of block row r is violated.
+template <int C>
+__device__ __forceinline__ uint32_t check_dual(const uint32_t *L, int r, int i) {
+  using T = Code<C>;
+  const bool last = FullRows<C>::all || ((FullRows<C>::mask >> r) & 1);
+  const uint32_t *own = L + T::K + r * 128 + i;
+  uint32_t x = *own;
+  if (r > 0) x ^= own[-128];
+  else if (i != 0) x ^= L[T::K + (T::MB - 1) * 128 + i - 1];
+  constexpr int ND = T::NDMAX;
+  const uint8_t *Lb = reinterpret_cast<const uint8_t *>(L);
+#pragma unroll
+  for (int e = 0; e < ND; e += 2) {
+    const uint4 c = c_dual[dual_first<C>() + r * ((ND + 1) / 2) + e / 2];
+    if (e < ND - 1 || last) x ^= *reinterpret_cast<const uint32_t *>(Lb + (((4u * i - c.y) & 508u) | c.x));
+    if (e + 1 < ND && (e + 1 < ND - 1 || last)) x ^= *reinterpret_cast<const uint32_t *>(Lb + (((4u * i - c.w) & 508u) | c.z));
+  }
+  return x;
+}
+
+// x^(8 (476 - 4 j)) mod P for word j of a block, then the all-ones init's term: CRC-32C as a sum of word products.
+__device__ uint32_t g_crc_words[kBlockBytes / 4 + 1];
+
+// Whether the batch's next codeword is copied to a line of shared memory while the pair decodes (the 2/3 code's would
+// leave an SM two CTAs instead of three).
+template <int C> __host__ __device__ constexpr bool dual_stages() { return C != 2; }
+template <int C>
+struct DualShared {
+  uint32_t L[Code<C>::N];            // posteriors: data columns in code order, then parity bit k + c (c = i mb + r) at [r][i]
+  uint32_t R[Code<C>::MB * row_words<C>() * 128];
+  alignas(16) uint32_t pk[Code<C>::N / 32];
+  alignas(16) int8_t next[dual_stages<C>() ? Code<C>::N : 16];
+  uint32_t par[128], red[2][4], crc[4];
+  int item;
+};
+// CTAs an SM holds, by shared memory (a CTA's and the 1 KB the system keeps of each).
+template <int C> __host__ __device__ constexpr int dual_ctas() { return 228 * 1024 / ((int)sizeof(DualShared<C>) + 1024); }
+static_assert(dual_ctas<0>() == 4 && dual_ctas<1>() == 3 && dual_ctas<2>() == 3 && dual_ctas<3>() == 2, "the two-codeword CTAs an SM");
+
+// One half's column written: a whole number as f16.
+__device__ __forceinline__ void put_half(uint32_t *L, int word, int h, int8_t x) {
+  const uint32_t v = hsub2(0x6400u | ((uint32_t)(uint8_t)x ^ 0x80u), kH1152);
+  reinterpret_cast<uint16_t *>(L)[2 * word + h] = (uint16_t)v;
+}
+
+// Item `item`'s soft values into half h (next: the staged codeword, or its place in the batch). Every thread takes part;
+// the caller synchronises.
+template <int C>
+__device__ __forceinline__ void load_dual(const LdpcLaunch &a, int item, const int8_t *next, uint32_t *L, int h) {
+  using T = Code<C>;
+  const int tid = threadIdx.x;
+  if (a.rx.llrf) {
+    // the receiver's slots through the bit map, whitening off by sign, never-sent bits 0, known zeros 127 (as
+    // decode_item)
+    const int f = item / a.fd.tier_blocks[a.tier], b = a.fd.tier_first[a.tier] + item % a.fd.tier_blocks[a.tier];
+    const int s0 = a.fd.block_slot[b], nt = a.fd.tier_nt[a.tier];
+    const int8_t *sl = a.rx.llrf + f * a.rx.llr_stride + s0;
+    const uint8_t *wh = a.fd.white + s0;
+    const int16_t *perm = a.fd.perm[a.tier];
+    constexpr int U = 15;   // nt is 35, 40, 45 or 60 times 128
+    for (int i0 = tid; i0 < nt; i0 += U * kDualThreads) {
+      int v[U];
+      int8_t x[U];
+      uint8_t w[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int i = i0 + u * kDualThreads;
+        v[u] = i < nt ? perm[i] : -1; x[u] = i < nt ? sl[i] : 0; w[u] = i < nt ? wh[i] : 0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (v[u] >= 0) put_half(L, lpos<C, false>(v[u]), h, w[u] ? (int8_t)(-x[u]) : x[u]);
+    }
+    for (int v = LIZG_INFO_BITS + tid; v < T::K; v += kDualThreads) put_half(L, v, h, 127);
+  } else {
+    // data bits a byte a lane (the half-words stored on distinct banks), then thread i's mb parity bits
+    constexpr int U = C == 0 ? 31 : 10;
+#pragma unroll
+    for (int k = 0; k < T::K / kDualThreads; k += U) {
+      int8_t x[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) x[u] = next[(k + u) * kDualThreads + tid];
+#pragma unroll
+      for (int u = 0; u < U; u++) put_half(L, (k + u) * kDualThreads + tid, h, x[u]);
+    }
+    int8_t x[T::MB];
+#pragma unroll
+    for (int r = 0; r < T::MB; r++) x[r] = next[T::K + tid * T::MB + r];
+#pragma unroll
+    for (int r = 0; r < T::MB; r++) put_half(L, T::K + r * 128 + tid, h, x[r]);
+  }
+}
+
+// Half h's decision: hard bits packed MSB first, the block's CRC-32C, the verdict. Every thread takes part; the caller
+// synchronises before the shared words are written again.
+template <int C>
+__device__ __forceinline__ void finish_dual(const LdpcLaunch &a, int item, int used, DualShared<C> &s, int h) {
+  using T = Code<C>;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t sign = h ? 0x80000000u : 0x8000u;
+  uint32_t mine = 0;   // lane j keeps the warp's word j, stored together
+  constexpr int PW = T::K / 128;
+#pragma unroll
+  for (int j = 0; j < PW; j++) {
+    const uint32_t b = __ballot_sync(0xffffffffu, (s.L[128 * j + tid] & sign) != 0);
+    if (lane == j) mine = b;
+  }
+  if (lane < PW) s.pk[4 * lane + warp] = __byte_perm(__brev(mine), 0u, 0x0123u);
+  if (!a.rx.llrf) {   // thread i's mb parity bits are consecutive in code order: bits i mb .. i mb + mb - 1
+    uint32_t m = 0;
+#pragma unroll
+    for (int r = 0; r < T::MB; r++) m |= (s.L[T::K + r * 128 + tid] & sign) ? 1u << r : 0u;
+    s.par[tid] = m;
+  }
+  __syncthreads();
+  uint32_t c = 0;
+  if (tid < kBlockBytes / 4) c = gf_mul(s.pk[tid], g_crc_words[tid]);
+  c = __reduce_xor_sync(0xffffffffu, c);
+  if (lane == 0) s.crc[warp] = c;
+  if (!a.rx.llrf && tid < 4 * T::MB) {
+    uint32_t b = 0;
+    for (int i = 32 * tid / T::MB; i < 128 && i * T::MB < 32 * tid + 32; i++) {
+      const int at = i * T::MB - 32 * tid;
+      b |= at >= 0 ? s.par[i] << at : s.par[i] >> -at;
+    }
+    s.pk[T::K / 32 + tid] = __byte_perm(__brev(b), 0u, 0x0123u);
+  }
+  __syncthreads();
+  const uint32_t crc = ~(s.crc[0] ^ s.crc[1] ^ s.crc[2] ^ s.crc[3] ^ g_crc_words[kBlockBytes / 4]);
+  const bool match = crc == __byte_perm(s.pk[kBlockBytes / 4], 0u, 0x0123u);
+  if (a.rx.llrf) {
+    const int f = item / a.fd.tier_blocks[a.tier], gi = f * a.fd.blocks + a.fd.tier_first[a.tier] + item % a.fd.tier_blocks[a.tier];
+    if (tid == 0) { a.its[gi] = used; a.ok[gi] = used > 0 && match; }   // only a decoded block is verified
+    uint8_t *dst = a.rx.blocks + (int64_t)gi * kBlockBytes;
+    if ((reinterpret_cast<uintptr_t>(dst) & 3) == 0) {
+      if (tid < kBlockBytes / 4) reinterpret_cast<uint32_t *>(dst)[tid] = s.pk[tid];
+    } else {
+      for (int t = tid; t < kBlockBytes; t += kDualThreads) dst[t] = reinterpret_cast<const uint8_t *>(s.pk)[t];
+    }
+  } else {
+    const int cw = a.list[item];
+    if (tid == 0) { a.its[cw] = used; a.ok[cw] = match; }   // the batch reports the CRC of whatever was decided
+    int4 *dst = reinterpret_cast<int4 *>(a.bits + a.off[cw] / 8);
+    for (int t = tid; t < T::N / 128; t += kDualThreads) dst[t] = reinterpret_cast<const int4 *>(s.pk)[t];
+  }
+}
+
+// The persistent kernel, a pair a CTA. A CTA's own first items are blockIdx.x and blockIdx.x + gridDim.x, so two
+// codewords share a CTA only where every CTA has one; later items come from the counter. A half that finishes takes
+// its next codeword at the next even iteration (the layers run forwards on even iterations and backwards on odd ones,
+// so both halves must agree); its partner goes on.
+template <int C>
+__global__ void __launch_bounds__(kDualThreads, dual_ctas<C>()) ldpc_dual_kernel(LdpcLaunch a) {
+  using T = Code<C>;
+  extern __shared__ __align__(16) uint8_t smem[];
+  DualShared<C> &s = *reinterpret_cast<DualShared<C> *>(smem);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int count = a.count_dev ? *a.count_dev : a.count;
+  const bool counter = 2 * (int)gridDim.x < count;   // else every item is some CTA's own
+  int item[2] = {-1, -1}, it[2] = {0, 0}, first[2] = {0, 0};
+  int own = 0, staged = -1, buf = 0;
+  bool more = true;
+  uint32_t *R = s.R + tid;
+  for (int k = tid; k < T::N; k += kDualThreads) s.L[k] = 0;   // an idle half holds zeros or its last codeword
+  for (int k = 0; k < T::MB * row_words<C>(); k++) R[k * 128] = 0x80808080u;
+  auto pull = [&]() -> int {   // the next item, waited for
+    if (own < 2) return (int)(blockIdx.x + gridDim.x * own++);
+    if (!counter) return count;
+    if (tid == 0) s.item = 2 * (int)gridDim.x + atomicAdd(a.counter, 1);
+    __syncthreads();
+    const int next = s.item;
+    __syncthreads();
+    return next;
+  };
+  auto stage = [&](int next) {   // a batch item on its way to the staging line
+    if (next >= count) { more = false; return; }
+    staged = next;
+    if (!dual_stages<C>()) return;
+    const int8_t *src = a.llr + a.off[a.list[next]];
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s.next);
+    for (int t = tid; t < T::N / 16; t += kDualThreads)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * t), "l"(src + 16 * t) : "memory");
+  };
+  __syncthreads();
+  for (int step = 0;; step ^= 1) {   // the iteration's direction
+    if (item[0] < 0 && item[1] < 0) step = 0;
+    if (step == 0) {
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        if (item[h] >= 0) continue;
+        if (a.rx.llrf) {
+          while (item[h] < 0 && more) {
+            const int next = pull();
+            if (next >= count) { more = false; break; }
+            const int f = next / a.fd.tier_blocks[a.tier], gi = f * a.fd.blocks + a.fd.tier_first[a.tier] + next % a.fd.tier_blocks[a.tier];
+            if (a.rx.decl[gi]) {   // a declined block is not tried
+              if (tid == 0) { a.its[gi] = -2; a.ok[gi] = 0; }
+            } else {
+              item[h] = next;
+            }
+          }
+        } else {
+          if (staged < 0 && more) stage(pull());
+          if (staged >= 0) {
+            if (dual_stages<C>()) {
+              asm volatile("cp.async.wait_all;" ::: "memory");
+              __syncthreads();
+            }
+            item[h] = staged;
+            staged = -1;
+          }
+        }
+        if (item[h] >= 0) {
+          it[h] = 0;
+          load_dual<C>(a, item[h], a.rx.llrf ? nullptr : dual_stages<C>() ? s.next : a.llr + a.off[a.list[item[h]]], s.L, h);
+          const uint32_t keep = h ? 0x00FF00FFu : 0xFF00FF00u;
+#pragma unroll 5
+          for (int k = 0; k < T::MB * row_words<C>(); k++) R[k * 128] = (R[k * 128] & keep) | (0x80808080u & ~keep);
+          if (dual_stages<C>() && !a.rx.llrf) __syncthreads();   // the staging line is read
+        }
+      }
+      if (item[0] < 0 && item[1] < 0) break;
+      __syncthreads();
+    }
+    // the batch's next codeword asked for and copied in under this iteration
+    const bool ask = !a.rx.llrf && staged < 0 && more;
+    int asked = 0;
+    if (ask) {
+      if (own < 2) stage(pull());
+      else if (tid == 0 && counter) asked = atomicAdd(a.counter, 1);
+    }
+    RowFetch<C> x;
+    fetch_row<C>(x, R, step ? T::MB - 1 : 0, 4 * tid);
+#pragma unroll 1
+    for (int k = 0; k < T::MB; k++) {
+      const int r = step ? T::MB - 1 - k : k, rn = step ? max(r - 1, 0) : min(r + 1, T::MB - 1);
+      layer_dual<C>(s.L, R, x, r, rn, tid);
+      __syncthreads();
+    }
+    // violated checks: counted where the stall rule reads the count (after the first iteration and at stall_it), else
+    // looked for until both live halves have one, in the order the iteration updated them
+    uint32_t live = 0;
+    bool counted = false;
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+      if (item[h] >= 0) {
+        live |= h ? 0x80000000u : 0x8000u;
+        counted |= a.stall_it > 1 && (it[h] == 0 || it[h] == a.stall_it - 1);
+      }
+    uint32_t acc = 0;
+    if (counted) {
+      for (int r = 0; r < T::MB; r++) acc += (check_dual<C>(s.L, r, tid) >> 15) & 0x00010001u;
+      acc = __reduce_add_sync(0xffffffffu, acc);
+    } else {
+      for (int k = 0; k < T::MB; k++) {
+        acc |= check_dual<C>(s.L, step ? T::MB - 1 - k : k, tid) & kHSign;
+        if ((k & (k + 1)) == 0 || k == T::MB - 1) {   // looks after 1, 2, 4, 8, ... rows
+          acc = __reduce_or_sync(0xffffffffu, acc);
+          if ((acc & live) == live) break;
+        }
+      }
+    }
+    if (lane == 0) s.red[buf][warp] = acc;
+    if (tid == 0) s.item = 2 * (int)gridDim.x + asked;
+    __syncthreads();
+    if (ask && staged < 0 && more) stage(counter ? s.item : count);
+    uint32_t all = 0;
+#pragma unroll
+    for (int w = 0; w < 4; w++) { const uint32_t v = s.red[buf][w]; all = counted ? all + v : all | v; }
+    buf ^= 1;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      if (item[h] < 0) continue;
+      const int bad = counted ? (int)(h ? all >> 16 : all & 0xffffu) : (all & (h ? 0x80000000u : 0x8000u)) != 0;
+      int used = 0;
+      if (bad == 0) used = it[h] + 1;
+      else if (a.stall_it > 1 && it[h] == a.stall_it - 1) {
+        if ((float)bad > __fmul_rn(a.stall_ratio, (float)first[h])) used = -3;
+      } else if (it[h] == 0 && a.stall_it > 1) first[h] = bad;
+      if (used == 0 && it[h] + 1 >= a.max_iter) used = -1;
+      it[h]++;
+      if (used) {
+        finish_dual<C>(a, item[h], used, s, h);
+        item[h] = -1;
+        __syncthreads();
+      }
+    }
+  }
+}
+
 // x^(8 k) mod P, reflected.
 static uint32_t xpow8(int k) {
   uint32_t r = 0x80000000u;
@@ -759,7 +1186,23 @@ cudaError_t ldpc_upload_tables() {
   uint32_t k[33];
   for (int l = 0; l < 32; l++) { const int end = 15 * l + 15 < kBlockBytes ? 15 * l + 15 : kBlockBytes; k[l] = xpow8(kBlockBytes - end); }
   k[32] = host_gf_mul(0xffffffffu, xpow8(kBlockBytes));
-  return cudaMemcpyToSymbol(c_crc_shift, k, sizeof k);
+  if ((err = cudaMemcpyToSymbol(c_crc_shift, k, sizeof k)) != cudaSuccess) return err;
+  std::vector<uint4> dual;
+  for (int c = 0; c < 4; c++) {
+    const lizg_code_def_t &d = LIZG_CODES[c];
+    const int ndmax = c == 0 ? Code<0>::NDMAX : c == 1 ? Code<1>::NDMAX : c == 2 ? Code<2>::NDMAX : Code<3>::NDMAX;
+    for (int r = 0; r < d.mb; r++)
+      for (int e = 0; e < ndmax; e += 2) {
+        auto circ = [&](int j) { return d.rowptr[r] + j < d.rowptr[r + 1] ? (uint32_t)d.circ[d.rowptr[r] + j] : 0u; };
+        const uint32_t p = circ(e), q = circ(e + 1);
+        dual.push_back(make_uint4((p >> 8) * 512u, (p & 255) * 4u, (q >> 8) * 512u, (q & 255) * 4u));
+      }
+  }
+  if ((err = cudaMemcpyToSymbol(c_dual, dual.data(), dual.size() * sizeof(uint4))) != cudaSuccess) return err;
+  uint32_t kw[kBlockBytes / 4 + 1];
+  for (int j = 0; j < kBlockBytes / 4; j++) kw[j] = xpow8(kBlockBytes - 4 * j);
+  kw[kBlockBytes / 4] = k[32];
+  return cudaMemcpyToSymbol(g_crc_words, kw, sizeof kw);
 }
 
 // ---------------------------------------------------------------- kernel variants and their choice
@@ -770,15 +1213,15 @@ cudaError_t ldpc_upload_tables() {
 // and keeps the fastest per code.
 struct Variant {
   int wpc;
-  bool loop, pair;
+  bool loop, pair, dual;
 };
 constexpr int kMaxVariants = 8;
 static const Variant kVariants[4][kMaxVariants] = {
-    // 7/8: 21-circulant rows, the loop form; the pair form first (the fastest on a GB300)
-    {{2, true, true}, {1, true, false}, {2, false, false}, {2, true, false}, {2, false, true}, {1, true, true}},
-    {{2, false, false}, {1, true, false}, {4, false, false}, {2, true, false}, {2, false, true}, {1, false, true}},   // 3/4
-    {{2, false, false}, {1, true, false}, {4, false, false}, {2, false, true}, {1, false, true}},                     // 2/3
-    {{4, false, false}, {2, false, false}, {1, false, false}, {2, false, true}, {1, false, true}},                    // 1/2
+    // the two-codeword form first: the fastest of every code on a GB300, at every batch size
+    {{4, true, false, true}, {2, true, true}, {1, true, false}, {2, true, false}, {2, false, true}, {1, true, true}},      // 7/8
+    {{4, true, false, true}, {2, false, false}, {4, false, false}, {2, true, false}, {2, false, true}, {1, false, true}},   // 3/4
+    {{4, true, false, true}, {2, false, false}, {4, false, false}, {2, false, true}, {1, false, true}},                     // 2/3
+    {{4, true, false, true}, {4, false, false}, {2, false, false}, {2, false, true}, {1, false, true}},                     // 1/2
 };
 static int variant_count(int code) {
   int k = 0;
@@ -797,6 +1240,16 @@ static int choice_of(int code) {
   return dev >= 0 && dev < kMaxDevices ? g_choice[dev][code] : 0;
 }
 
+template <int C>
+static cudaError_t launch_dual(const LdpcLaunch &a, int sms, cudaStream_t st) {
+  constexpr int smem = (int)sizeof(DualShared<C>);
+  static SmemOptIn opt;
+  if (cudaError_t e = opt.set(reinterpret_cast<const void *>(ldpc_dual_kernel<C>), smem)) return e;
+  const int most = sms * dual_ctas<C>();
+  ldpc_dual_kernel<C><<<a.count < most ? a.count : most, kDualThreads, smem, st>>>(a);
+  return cudaGetLastError();
+}
+
 template <int C, int WPC, bool LOOP, bool PAIR>
 static cudaError_t launch_v(const LdpcLaunch &a, int sms, cudaStream_t st) {
   static SmemOptIn opt;
@@ -809,26 +1262,26 @@ static cudaError_t launch_v(const LdpcLaunch &a, int sms, cudaStream_t st) {
 
 static cudaError_t launch_variant(int code, int v, const LdpcLaunch &a, int sms, cudaStream_t st) {
   switch (code * kMaxVariants + v) {
-    case 0: return launch_v<0, 2, true, true>(a, sms, st);
-    case 1: return launch_v<0, 1, true, false>(a, sms, st);
-    case 2: return launch_v<0, 2, false, false>(a, sms, st);
+    case 0: return launch_dual<0>(a, sms, st);
+    case 1: return launch_v<0, 2, true, true>(a, sms, st);
+    case 2: return launch_v<0, 1, true, false>(a, sms, st);
     case 3: return launch_v<0, 2, true, false>(a, sms, st);
     case 4: return launch_v<0, 2, false, true>(a, sms, st);
     case 5: return launch_v<0, 1, true, true>(a, sms, st);
-    case 8: return launch_v<1, 2, false, false>(a, sms, st);
-    case 9: return launch_v<1, 1, true, false>(a, sms, st);
+    case 8: return launch_dual<1>(a, sms, st);
+    case 9: return launch_v<1, 2, false, false>(a, sms, st);
     case 10: return launch_v<1, 4, false, false>(a, sms, st);
     case 11: return launch_v<1, 2, true, false>(a, sms, st);
     case 12: return launch_v<1, 2, false, true>(a, sms, st);
     case 13: return launch_v<1, 1, false, true>(a, sms, st);
-    case 16: return launch_v<2, 2, false, false>(a, sms, st);
-    case 17: return launch_v<2, 1, true, false>(a, sms, st);
+    case 16: return launch_dual<2>(a, sms, st);
+    case 17: return launch_v<2, 2, false, false>(a, sms, st);
     case 18: return launch_v<2, 4, false, false>(a, sms, st);
     case 19: return launch_v<2, 2, false, true>(a, sms, st);
     case 20: return launch_v<2, 1, false, true>(a, sms, st);
-    case 24: return launch_v<3, 4, false, false>(a, sms, st);
-    case 25: return launch_v<3, 2, false, false>(a, sms, st);
-    case 26: return launch_v<3, 1, false, false>(a, sms, st);
+    case 24: return launch_dual<3>(a, sms, st);
+    case 25: return launch_v<3, 4, false, false>(a, sms, st);
+    case 26: return launch_v<3, 2, false, false>(a, sms, st);
     case 27: return launch_v<3, 2, false, true>(a, sms, st);
     case 28: return launch_v<3, 1, false, true>(a, sms, st);
   }
@@ -879,7 +1332,7 @@ int lizg_ldpc_variant(int rate, int32_t *wpc, int32_t *loop_form) {
   if (int rc = lizg::device_ready(&sms)) return rc;
   const int v = lizg::choice_of(c);
   if (wpc) *wpc = lizg::kVariants[c][v].wpc;
-  if (loop_form) *loop_form = (lizg::kVariants[c][v].loop ? 1 : 0) | (lizg::kVariants[c][v].pair ? 2 : 0);
+  if (loop_form) *loop_form = (lizg::kVariants[c][v].loop ? 1 : 0) | (lizg::kVariants[c][v].pair ? 2 : 0) | (lizg::kVariants[c][v].dual ? 4 : 0);
   return v;
 }
 

@@ -241,3 +241,16 @@ def test_autotune_keeps_a_variant_and_decodes_alike():
     finally:
         for r in (6, 4, 3, 2):
             lz.ldpc_set_variant(r, 0)
+
+
+@pytest.mark.parametrize("rate", [6, 4, 3, 2])
+@pytest.mark.parametrize("count,mi,si", [(1, 20, 9), (2, 1, 0), (3, 2, 2), (153, 20, 9), (305, 3, 0), (1221, 20, 9), (1300, 7, 3)])
+def test_two_codeword_form_at_its_edges(rate, count, mi, si):
+    """The default form's edges: one codeword, odd counts, counts about the grid's one and two a CTA and past them (items
+    from the counter), odd iteration limits (halves of a CTA that stop apart), the whole int8 range of soft values."""
+    b = synth.ldpc_batch(count, seed=900 + count, rates=np.full(count, rate, np.int32))
+    llr = b["llr"].copy()
+    n = lz.CODE_N[rate]
+    wild = np.random.default_rng(count).integers(-128, 128, n, dtype=np.int64).astype(np.int8)
+    llr[(count // 2) * n:(count // 2 + 1) * n] = wild
+    check_against_oracle({**b, "llr": llr}, mi, si, 0.95)
