@@ -233,12 +233,6 @@ __device__ __forceinline__ bool in_square(const FftDev &xd, int t) {
   return in;
 }
 
-// The shading basis 1, c(x), q(x), c(y), q(y), c(x) c(y) at sample (x, y) (liblizard/src/lizard_phy.c:336-340).
-__device__ __forceinline__ void hole_basis(const FftDev &xd, int x, int y, double b[6]) {
-  const double cx = xd.cx[x], cy = xd.cx[y];
-  b[0] = 1; b[1] = cx; b[2] = xd.qx[x]; b[3] = cy; b[4] = xd.qx[y]; b[5] = cx * cy;
-}
-
 // The shading fit's right-hand side (liblizard/src/lizard_phy.c:1609-1623) over kHoleBand of the frame's
 // every-eighth rows: hole[f][band][0..5]. A warp takes a row: its samples outside the squares summed in float as
 // z, z c(x), z q(x) (the basis is separable: 1, c(x), q(x), c(y), q(y), c(x) c(y)), then the row's six terms added
@@ -329,14 +323,6 @@ struct FftRowsMix {
 };
 static_assert(sizeof(FftColsMix) <= 32000 && sizeof(FftRowsMix) <= 32000, "the mixed grids' arguments fit a launch");
 
-// The surface's value at (x, y) inside an anchor's square (liblizard/src/lizard_phy.c:341-346).
-__device__ __forceinline__ float hole_value(const FftDev &xd, const double *beta, int x, int y) {
-  double bb[6], h = 0;
-  hole_basis(xd, x, y, bb);
-  for (int r = 0; r < 6; r++) h += beta[r] * bb[r];
-  return (float)h;
-}
-
 // The sampler's per-row quantities of a batch, worked out once a frame before the column pass reads them, with the
 // same functions and inputs as the per-sample walk (the cell's 1 / width as the column table computes it), so the
 // column pass reads the walk's own values. A thread an entry, entries in table order. The exact walk: for picture row
@@ -377,11 +363,11 @@ __global__ void __launch_bounds__(256) cell_table_kernel(SrcDev src, int per_fra
 // the imaginary part) at rows y = t / L, t / L + kThreads / L, ...; the anchors' squares erased to the shading
 // surface as they are read. Each row's two samples are summed into the five detrend projections' raw sums, z c(x),
 // z c(y), z c(x) c(y), z q(x), z q(y) (liblizard/src/lizard_phy.c:1584-1591, 1657-1667), in p. SRC: kSrcGrid reads a
-// supplied grid; kSrcExact and kSrcDecode sample the captured frame by the exact walk or the decode's read.
+// supplied grid; kSrcExact and kSrcDecode sample the captured frame by the exact walk or the decode's read. The squares'
+// values are in the lines already (erase_tile).
 constexpr int kSrcGrid = 0, kSrcExact = 1, kSrcDecode = 2;
 template <int N, int SRC>
-__device__ __forceinline__ void load_tile(const FftDev &xd, const SrcDev &src, const float4 *ctab, int f, int x0, const double *beta,
-                                          float2 *line, float p[5]) {
+__device__ __forceinline__ void load_tile(const FftDev &xd, const SrcDev &src, const float4 *ctab, int f, int x0, float2 *line, float p[5]) {
   constexpr int L = plan_of(N).lines, ystep = kThreads / L;
   const int l = threadIdx.x % L, xa = x0 + l, xb = x0 + L + l;
   const bool ina = in_square(xd, xa), inb = in_square(xd, xb);
@@ -431,8 +417,11 @@ __device__ __forceinline__ void load_tile(const FftDev &xd, const SrcDev &src, c
       lin_steps(lc, s, L / 4);
       vb = lin_point(px, src.w, src.h, src.pitch, s, tb, rw.z);
     }
-    if (ina && ysq) va = hole_value(xd, beta, xa, y);
-    if (inb && ysq) vb = hole_value(xd, beta, xb, y);
+    if (ysq) {
+      const float2 erased = line[pad(y)];
+      if (ina) va = erased.x;
+      if (inb) vb = erased.y;
+    }
     const float cy = __ldg(xd.cx + y), qy = __ldg(xd.qx + y);
     const float t0 = va + vb, t1 = cxa * va + cxb * vb, t2 = qxa * va + qxb * vb;
     p[0] += t1; p[1] += cy * t0; p[2] += cy * t1; p[3] += t2; p[4] += qy * t0;
@@ -443,8 +432,53 @@ __device__ __forceinline__ void load_tile(const FftDev &xd, const SrcDev &src, c
 // The column pass's per-CTA scalars in shared memory.
 struct ColsShared {
   double rhs[6], beta[6];
+  double h2[32], cx[32];   // a column's part of the surface and its c(x), the tile's columns inside a square
   float part[kThreads / 32][5];
 };
+
+// The anchors' squares of one tile laid into its lines before the samples are read: at (x, y) the shading surface
+// beta . (1, c(x), q(x), c(y), q(y), c(x) c(y)) in double, rounded to float (liblizard/src/lizard_phy.c:336-346). A tile
+// meets at most one square's columns (a tile is at most 32 wide, the squares' gaps are wider); a thread takes a row
+// inside a square over those columns, the columns' terms (the first three, the same for every row) worked out once.
+// The double pipe is the reason: worked out where each sample is read, in warps with a few lanes inside a square, it was
+// 86% busy and most of the pass on grids (the transform of 64 grids of n = 768: 572 us, 253 with the values laid in
+// first; 32 captured frames of n = 1536 decoded: 1093 us, 1071).
+template <int N>
+__device__ __forceinline__ void erase_tile(const FftDev &xd, int x0, float2 *buf, ColsShared &s) {
+  constexpr int L = plan_of(N).lines, LSTR = lstride_of(N);
+  static_assert(2 * L <= 32, "a tile's columns");
+  int lo = 0, cols = 0, rows = 0;
+#pragma unroll
+  for (int i = 0; i < 7; i++) {
+    const int a = max(xd.elo[i], x0), b = min(xd.ehi[i], x0 + 2 * L - 1);
+    if (a <= b) { lo = a; cols = b - a + 1; }
+    rows += xd.ehi[i] - xd.elo[i] + 1;
+  }
+  if (cols == 0) return;
+  const int tid = threadIdx.x;
+  if (tid < cols) {
+    const double cx = xd.cx[lo + tid], qx = xd.qx[lo + tid];
+    s.h2[tid] = fma(s.beta[2], qx, fma(s.beta[1], cx, s.beta[0]));
+    s.cx[tid] = cx;
+  }
+  __syncthreads();
+  for (int k = tid; k < rows; k += kThreads) {
+    int y = k;   // the k-th row inside a square
+#pragma unroll
+    for (int i = 0; i < 7; i++) {
+      const int w = xd.ehi[i] - xd.elo[i] + 1;
+      if (y < w) { y += xd.elo[i]; break; }
+      y -= w;
+    }
+    const double cy = xd.cx[y], qy = xd.qx[y];
+    for (int c = 0; c < cols; c++) {
+      const double h = fma(s.beta[5], s.cx[c] * cy, fma(s.beta[4], qy, fma(s.beta[3], cy, s.h2[c])));
+      const int q = lo - x0 + c;
+      reinterpret_cast<float *>(buf + (q % L) * LSTR + pad(y))[q / L] = (float)h;
+    }
+  }
+  __syncthreads();
+}
 
 // The column pass on one tile (frame f, columns x0 = 2 L tile .. x0 + 2L - 1): the shading surface beta from the
 // frame's bands, the tile's samples (erased, projections summed: part[f][tile][0..4]), the L lines' transforms along
@@ -464,20 +498,18 @@ __device__ __forceinline__ void cols_tile(const FftDev &xd, const SrcDev &src, c
     s.rhs[tid] = acc;
   }
   __syncthreads();
-  if (tid == 0) {
+  if (tid < 6) {
+    double acc = 0;
 #pragma unroll
-    for (int r = 0; r < 6; r++) {
-      double acc = 0;
-#pragma unroll
-      for (int k = 0; k < 6; k++) acc += xd.hole_inv[r * 6 + k] * s.rhs[k];
-      s.beta[r] = acc;
-    }
+    for (int k = 0; k < 6; k++) acc += xd.hole_inv[tid * 6 + k] * s.rhs[k];
+    s.beta[tid] = acc;
   }
   __syncthreads();
+  erase_tile<N>(xd, x0, sm.buf, s);
   float p[5] = {0, 0, 0, 0, 0};
-  if (src.grid) load_tile<N, kSrcGrid>(xd, src, ctab, f, x0, s.beta, line, p);
-  else if (src.sd.read == LIZG_READ_DECODE) load_tile<N, kSrcDecode>(xd, src, ctab, f, x0, s.beta, line, p);
-  else load_tile<N, kSrcExact>(xd, src, ctab, f, x0, s.beta, line, p);
+  if (src.grid) load_tile<N, kSrcGrid>(xd, src, ctab, f, x0, line, p);
+  else if (src.sd.read == LIZG_READ_DECODE) load_tile<N, kSrcDecode>(xd, src, ctab, f, x0, line, p);
+  else load_tile<N, kSrcExact>(xd, src, ctab, f, x0, line, p);
 #pragma unroll
   for (int q = 0; q < 5; q++)
     for (int o = 16; o > 0; o >>= 1) p[q] += __shfl_xor_sync(0xffffffffu, p[q], o);
