@@ -24,87 +24,194 @@ __device__ __forceinline__ float2 turned(const FmtDev &fd, const float2 *spec, i
   return make_float2(z.x * cs.x + z.y * cs.y, z.y * cs.x - z.x * cs.y);
 }
 
-// A cluster of kPilotCtas CTAs a frame: CTA r works out the six products of pilots [r chunk, (r + 1) chunk) into its
-// shared memory; then six threads of CTA 0 add one sum each in pilot order, reading the cluster's shared memory, so
-// the double sums are the reference's (liblizard/src/lizard_phy.c:283-317), and CTA 0's thread 0 solves for the
-// shift and hands it to every CTA for the second fit. Writes align[3 f ..] = dx, dy, and 1 where the shift is turned
-// back. (The products are spread over the cluster's SMs because double arithmetic is slow on one SM.)
-constexpr int kPilotCtas = 8;
+// The pilots' fit, a cluster of kPilotCtas CTAs a frame. The reference adds its six double sums in pilot order
+// (liblizard/src/lizard_phy.c:283-317), a chain of as many dependent additions as there are pilots. Only three things of
+// the fit are seen: the shift rounded to float after the first pass (the second pass turns the pilots by it), whether
+// the shift is worth turning back, and, where it is, the shift rounded to float. So the sums are first added as a
+// tree, each quantity's distance from the ordered sums' is bounded (pilot_bound), and where every one of the three
+// comes out the same over the whole bound it is the reference's, whatever the order; else the frame is done again
+// with the sums in pilot order. A rounding edge falls inside the bound (about 1e-12 of the shift) for about one frame
+// in ten thousand; an empty or overflowing spectrum always takes the second way.
+// Bound: the double pipe's latency (about 70 cycles an operation). One frame of n = 1536 (984 pilots) decoded: 277 us with
+// the ordered sums (95 of them here), 200 with the tree.
+constexpr int kPilotCtas = 8, kPilotThreads = 128, kPilotWarps = kPilotThreads / 32;
+static_assert(kPilotCtas * kPilotWarps == 32, "a lane of one warp a warp of the cluster");
+enum { kPilotOn = 0, kPilotGiveUp = 1, kPilotAgain = 2 };
+
+// v[0..5] summed over the warp: value k ends in lane 16 (k >> 2 & 1) + 8 (k >> 1 & 1) + 4 (k & 1) and its three
+// neighbours. Each step sends the half of the values that the partner keeps: nine additions in place of thirty.
+__device__ __forceinline__ double warp_sum6(double v[8], int lane) {
+  v[6] = v[7] = 0;
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const double keep = (lane & 16) ? v[j + 4] : v[j], send = (lane & 16) ? v[j] : v[j + 4];
+    v[j] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+  }
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    const double keep = (lane & 8) ? v[j + 2] : v[j], send = (lane & 8) ? v[j] : v[j + 2];
+    v[j] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+  }
+  const double keep = (lane & 4) ? v[1] : v[0], send = (lane & 4) ? v[0] : v[1];
+  double s = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  return s;
+}
+
+// How far the tree's sums (a = S cu cu, b = S cu cv, c = S cv cv, p = S cu zi, q = S cv zi, y = S zi zi over `used` terms)
+// and what is worked out from them may be from the ordered sums': a sum in any order is within used u of the sum of its
+// terms' magnitudes (u = 2^-53), itself the sum or, by Cauchy and Schwarz, the root of two. Every figure in float and
+// taken generously; an infinity or a NaN fails the comparisons it is used in.
+struct PilotBound {
+  float ea, eb, ec, ep, eq, ey, det;   // the sums' and a c - b b's
+};
+constexpr float kU = 1.2e-16f;   // over 2^-53
+__device__ __forceinline__ PilotBound pilot_bound(float a, float b, float c, float y, int used) {
+  PilotBound e;
+  const float E = (float)(used + 64) * 2.0f * kU;
+  e.ea = E * a; e.ec = E * c; e.ey = E * y;
+  e.eb = E * sqrtf(a) * sqrtf(c); e.ep = E * sqrtf(a) * sqrtf(y); e.eq = E * sqrtf(c) * sqrtf(y);
+  e.det = 2.0f * (e.ea * c + a * e.ec + 2.0f * fabsf(b) * e.eb) + 8.0f * kU * (a * c + b * b);
+  return e;
+}
 
 // Frame f's fit by the calling cluster. tm: this CTA's dynamic shared memory (chunk x 6 doubles at least).
 __device__ __forceinline__ void pilot_align_frame(const FmtDev &fd, const float2 *spec, int64_t spec_stride, float *align, int f, double *tm) {
-  __shared__ double sums[6], dxy[2];
-  __shared__ int give_up;
+  __shared__ double part[kPilotWarps][6], sums[6], dxy[2];
+  __shared__ int status;
   cg::cluster_group cl = cg::this_cluster();
-  const int rank = (int)cl.block_rank(), used = fd.npilot;
+  const int rank = (int)cl.block_rank(), used = fd.npilot, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int chunk = (used + kPilotCtas - 1) / kPilotCtas, p0 = rank * chunk, p1 = min(used, p0 + chunk);
   const float2 *sp = spec + f * spec_stride;
   const double k = 2.0 * 3.14159265358979323846 / fd.n;
-  if (threadIdx.x == 0) { dxy[0] = dxy[1] = 0; give_up = 0; }
-  cl.sync();
-  for (int it = 0; it < 2; it++) {
-    const double dx = dxy[0], dy = dxy[1];
-    for (int pi = p0 + (int)threadIdx.x; pi < p1; pi += blockDim.x) {
-      const int i = fd.pilot_coef[pi], w = fd.pilot_white[pi];
-      const float2 y = turned(fd, sp, i, (float)dx, (float)dy);
-      const double xr = (w & 1) ? -1.0 : 1.0, xi = (w & 2) ? -1.0 : 1.0;
-      const double zr = (double)y.x * xr + (double)y.y * xi, zi = (double)y.y * xr - (double)y.x * xi;
-      const double cu = k * zr * fd.uv[2 * i], cv = k * zr * fd.uv[2 * i + 1];
-      double *t = tm + 6 * (pi - p0);
-      t[0] = cu * cu; t[1] = cu * cv; t[2] = cv * cv; t[3] = cu * zi; t[4] = cv * zi; t[5] = zi * zi;
-    }
+  for (int ordered = 0;; ordered = 1) {
+    if (tid == 0) { dxy[0] = dxy[1] = 0; status = used < 8 ? kPilotGiveUp : kPilotOn; }
     cl.sync();
-    if (rank == 0) {
-      if (threadIdx.x < 6) {
-        // in pilot order, CTA by CTA; the loads of eight terms issued ahead of their adds
-        double acc = 0;
-        for (int r = 0; r < kPilotCtas; r++) {
-          const double *rt = cl.map_shared_rank(tm, r) + threadIdx.x;
-          const int cnt = max(0, min(used, (r + 1) * chunk) - r * chunk);
-          int q = 0;
-          for (; q + 8 <= cnt; q += 8) {
-            double v[8];
+    if (status) break;
+    float e_prev = 0;   // rank 0's lanes 0 and 1: the bound on dx's, dy's distance from the ordered one
+    for (int it = 0; it < 2; it++) {
+      const float dx = (float)dxy[0], dy = (float)dxy[1];
+      double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      for (int pi = p0 + tid; pi < p1; pi += kPilotThreads) {
+        const int i = fd.pilot_coef[pi], w = fd.pilot_white[pi];
+        const float2 y = turned(fd, sp, i, dx, dy);
+        const double xr = (w & 1) ? -1.0 : 1.0, xi = (w & 2) ? -1.0 : 1.0;
+        const double zr = (double)y.x * xr + (double)y.y * xi, zi = (double)y.y * xr - (double)y.x * xi;
+        const double cu = k * zr * fd.uv[2 * i], cv = k * zr * fd.uv[2 * i + 1];
+        const double t[6] = {cu * cu, cu * cv, cv * cv, cu * zi, cv * zi, zi * zi};
 #pragma unroll
-            for (int e = 0; e < 8; e++) v[e] = rt[6 * (q + e)];
+        for (int q = 0; q < 6; q++) {
+          if (ordered) tm[6 * (pi - p0) + q] = t[q];
+          else v[q] += t[q];
+        }
+      }
+      if (!ordered) {
+        const double s = warp_sum6(v, lane);
+        const int q = 4 * (lane >> 4) + 2 * (lane >> 3 & 1) + (lane >> 2 & 1);
+        if ((lane & 3) == 0 && q < 6) part[warp][q] = s;
+      }
+      cl.sync();
+      if (rank == 0 && ordered) {
+        if (tid < 6) {
+          // in pilot order, CTA by CTA; the loads of eight terms issued ahead of their adds
+          double acc = 0;
+          for (int r = 0; r < kPilotCtas; r++) {
+            const double *rt = cl.map_shared_rank(tm, r) + tid;
+            const int cnt = max(0, min(used, (r + 1) * chunk) - r * chunk);
+            int q = 0;
+            for (; q + 8 <= cnt; q += 8) {
+              double x[8];
 #pragma unroll
-            for (int e = 0; e < 8; e++) acc += v[e];
+              for (int e = 0; e < 8; e++) x[e] = rt[6 * (q + e)];
+#pragma unroll
+              for (int e = 0; e < 8; e++) acc += x[e];
+            }
+            for (; q < cnt; q++) acc += rt[6 * q];
           }
-          for (; q < cnt; q++) acc += rt[6 * q];
+          sums[tid] = acc;
         }
-        sums[threadIdx.x] = acc;
+        __syncthreads();
       }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        const double a = sums[0], b = sums[1], c = sums[2], p = sums[3], q = sums[4];
-        const double det = a * c - b * b;
-        int gu = 0;
-        double nx = dx, ny = dy;
-        if (used < 8 || !(det > 0)) gu = 1;
-        else { nx = dx + (p * c - q * b) / det; ny = dy + (a * q - b * p) / det; }
-        for (int r = 0; r < kPilotCtas; r++) {
-          double *rd = cl.map_shared_rank(dxy, r);
+      if (rank == 0 && warp == 0) {
+        double a, b, c, p, q, yy;
+        if (ordered) {
+          a = sums[0]; b = sums[1]; c = sums[2]; p = sums[3]; q = sums[4]; yy = sums[5];
+        } else {
+          const double *rp = cl.map_shared_rank(&part[0][0], lane / kPilotWarps) + 6 * (lane % kPilotWarps);
+#pragma unroll
+          for (int j = 0; j < 6; j++) v[j] = rp[j];
+          const double s = warp_sum6(v, lane);
+          a = __shfl_sync(0xffffffffu, s, 0); b = __shfl_sync(0xffffffffu, s, 4); c = __shfl_sync(0xffffffffu, s, 8);
+          p = __shfl_sync(0xffffffffu, s, 12); q = __shfl_sync(0xffffffffu, s, 16); yy = __shfl_sync(0xffffffffu, s, 20);
+        }
+        // lane 0 takes x, lane 1 y (the others repeat them): the shift's step (p c - q b) / det, (a q - b p) / det
+        const bool ly = lane & 1;
+        const double det = a * c - b * b, num = ly ? a * q - b * p : p * c - q * b;
+        const double step = num / det, was = ly ? dxy[1] : dxy[0], now = was + step;
+        int st = kPilotOn;
+        float e_step = 0, e_now = 0;
+        const PilotBound e = pilot_bound((float)a, (float)b, (float)c, (float)yy, used);
+        if (ordered) {
+          if (!(det > 0)) st = kPilotGiveUp;
+        } else {
+          const float fa = (float)a, fb = fabsf((float)b), fc = (float)c, fp = fabsf((float)p), fq = fabsf((float)q), fdet = (float)det;
+          const float m = ly ? fa : fc, em = ly ? e.ea : e.ec, f1 = ly ? fq : fp, e1 = ly ? e.eq : e.ep, f2 = ly ? fp : fq, e2 = ly ? e.ep : e.eq;
+          const float e_num = 2.0f * (e1 * m + f1 * em + e2 * fb + f2 * e.eb) + 8.0f * kU * (f1 * m + f2 * fb);
+          const float fs = fabsf((float)step);
+          e_step = 2.0f * (e_num + fs * e.det) / fdet + 8.0f * kU * fs;
+          e_now = e_prev + e_step + 8.0f * kU * fabsf((float)now);
+          // the determinant's sign is not sure, or figures so small that the bound itself could vanish
+          if (!(fdet > 4.0f * e.det && fdet > 1e-20f && (yy == 0 || (float)yy > 1e-15f))) st = kPilotAgain;
+          // the first pass's shift has to round alike over the bound: the second turns by it
+          if (it == 0 && !((float)(now - e_now) == (float)(now + e_now))) st = kPilotAgain;
+        }
+        st = (int)__reduce_max_sync(0xffffffffu, (unsigned)st);
+        if (it == 1 && st == kPilotOn) {
+          // worth turning back: chi^2 of the shift over the residual's variance past 13.8
+          const double nx = __shfl_sync(0xffffffffu, now, 0), ny = __shfl_sync(0xffffffffu, now, 1);
+          const double ex = __shfl_sync(0xffffffffu, step, 0), ey = __shfl_sync(0xffffffffu, step, 1);
+          const double s2 = (yy - ex * p - ey * q) / (used - 2);
+          const double chi = s2 > 0 ? (nx * nx * a + 2 * nx * ny * b + ny * ny * c) / s2 : 0;
+          bool back = chi > 13.8 && nx == nx && ny == ny;
+          if (!ordered) {
+            const float dsx = __shfl_sync(0xffffffffu, e_step, 0), dsy = __shfl_sync(0xffffffffu, e_step, 1);
+            const float dnx = __shfl_sync(0xffffffffu, e_now, 0), dny = __shfl_sync(0xffffffffu, e_now, 1);
+            const float fa = (float)a, fb = fabsf((float)b), fc = (float)c, fp = fabsf((float)p), fq = fabsf((float)q), fy = (float)yy;
+            const float fx = fabsf((float)ex), fey = fabsf((float)ey), x = fabsf((float)nx), y = fabsf((float)ny), fs2 = (float)s2, fchi = (float)chi;
+            const float e_s2 = 2.0f * (e.ey + fx * e.ep + fp * dsx + fey * e.eq + fq * dsy + 8.0f * kU * (fy + fx * fp + fey * fq)) / (float)(used - 2);
+            const float e_n = 2.0f * (2.0f * x * dnx * fa + x * x * e.ea + 2.0f * (dnx * y * fb + x * dny * fb + x * y * e.eb) + 2.0f * y * dny * fc +
+                                      y * y * e.ec) + 16.0f * kU * (x * x * fa + 2.0f * x * y * fb + y * y * fc);
+            const float e_chi = 2.0f * (e_n + fchi * e_s2) / fs2 + 8.0f * kU * fchi;
+            bool sure = fs2 > 4.0f * e_s2 && fabs(chi - 13.8) > 4.0 * e_chi;
+            if (back && !((float)(nx - dnx) == (float)(nx + dnx) && (float)(ny - dny) == (float)(ny + dny))) sure = false;
+            if (!sure) st = kPilotAgain;
+          }
+          if (lane == 0 && st == kPilotOn) {
+            const float d0 = back ? (float)nx : 0.0f, d1 = back ? (float)ny : 0.0f;
+            align[3 * f] = d0; align[3 * f + 1] = d1;
+            align[3 * f + 2] = d0 != 0 || d1 != 0 ? 1.0f : 0.0f;
+          }
+        }
+        e_prev = e_now;
+        // the shift and what to do next, to every CTA of the cluster
+        const double nx = __shfl_sync(0xffffffffu, now, 0), ny = __shfl_sync(0xffffffffu, now, 1);
+        if (lane < kPilotCtas) {
+          double *rd = cl.map_shared_rank(dxy, lane);
           rd[0] = nx; rd[1] = ny;
-          *cl.map_shared_rank(&give_up, r) = gu;
+          *cl.map_shared_rank(&status, lane) = st;
         }
       }
+      cl.sync();
+      if (status) break;
     }
-    cl.sync();
-    if (give_up) break;
+    if (status != kPilotAgain) break;
+    cl.sync();   // every CTA has read the status before it is set anew
   }
-  if (rank != 0 || threadIdx.x != 0) return;
-  float d0 = 0, d1 = 0;
-  if (!give_up) {
-    const double a = sums[0], b = sums[1], c = sums[2], p = sums[3], q = sums[4], yy = sums[5], dx = dxy[0], dy = dxy[1];
-    const double det = a * c - b * b, ex = (p * c - q * b) / det, ey = (a * q - b * p) / det;
-    const double s2 = (yy - ex * p - ey * q) / (used - 2);
-    const double chi = s2 > 0 ? (dx * dx * a + 2 * dx * dy * b + dy * dy * c) / s2 : 0;
-    if (chi > 13.8 && dx == dx && dy == dy) { d0 = (float)dx; d1 = (float)dy; }
-  }
-  align[3 * f] = d0; align[3 * f + 1] = d1;
-  align[3 * f + 2] = (used > 0 && (d0 != 0 || d1 != 0)) ? 1.0f : 0.0f;
+  if (rank == 0 && tid == 0 && status == kPilotGiveUp) align[3 * f] = align[3 * f + 1] = align[3 * f + 2] = 0;
 }
 
-__global__ void __cluster_dims__(kPilotCtas, 1, 1) __launch_bounds__(128) pilot_align_kernel(FmtDev fd, const float2 *spec, int64_t spec_stride,
+__global__ void __cluster_dims__(kPilotCtas, 1, 1) __launch_bounds__(kPilotThreads) pilot_align_kernel(FmtDev fd, const float2 *spec, int64_t spec_stride,
                                                                                            float *align) {
   extern __shared__ double tm[];              // chunk x 6: this CTA's pilots' products
   pilot_align_frame(fd, spec, spec_stride, align, blockIdx.x / kPilotCtas, tm);
@@ -258,7 +365,7 @@ __device__ __forceinline__ int seg_at(const int *first, int nseg, int b) {
   return k;
 }
 
-__global__ void __cluster_dims__(kPilotCtas, 1, 1) __launch_bounds__(128) pilot_align_mixed_kernel(const __grid_constant__ DemapMix m) {
+__global__ void __cluster_dims__(kPilotCtas, 1, 1) __launch_bounds__(kPilotThreads) pilot_align_mixed_kernel(const __grid_constant__ DemapMix m) {
   extern __shared__ double tm[];
   const int c = blockIdx.x / kPilotCtas, k = seg_at(m.pf, m.nseg, c);
   const DemapSeg &g = m.seg[k];
@@ -292,7 +399,7 @@ cudaError_t demap_mixed_launch(const DemapSeg *a, int count, cudaStream_t st) {
     m.bf[k + 1] = m.bf[k] + (fd.frames * fd.blocks + kBlocksThreads - 1) / kBlocksThreads;
   }
   if (psm > 48 * 1024) return cudaErrorInvalidValue;
-  pilot_align_mixed_kernel<<<m.pf[count] * kPilotCtas, 128, psm, st>>>(m);
+  pilot_align_mixed_kernel<<<m.pf[count] * kPilotCtas, kPilotThreads, psm, st>>>(m);
   demap_mixed_kernel<<<m.df[count], 256, 0, st>>>(m);
   blocks_mixed_kernel<<<m.bf[count], kBlocksThreads, 0, st>>>(m);
   return cudaGetLastError();
@@ -303,7 +410,7 @@ cudaError_t demap_launch(const FmtDev &fd, const float2 *spec, int64_t spec_stri
   const int chunk = (fd.npilot + kPilotCtas - 1) / kPilotCtas;
   const int psm = 6 * (chunk > 0 ? chunk : 1) * (int)sizeof(double);
   if (psm > 48 * 1024) return cudaErrorInvalidValue;
-  pilot_align_kernel<<<fd.frames * kPilotCtas, 128, psm, st>>>(fd, spec, spec_stride, align);
+  pilot_align_kernel<<<fd.frames * kPilotCtas, kPilotThreads, psm, st>>>(fd, spec, spec_stride, align);
   const int groups = fd.frames * fd.subch;
   demap_kernel<<<(groups + 63) / 64, 256, 0, st>>>(fd, spec, spec_stride, align, llrf, sub_est, sub_rms);
   const int nbk = fd.frames * fd.blocks;

@@ -107,3 +107,29 @@ def test_receiver_refuses_bad_calls():
     # still usable: the clean frame decodes every block
     out = rx.finish_luma(luma[None], reg[None], grid=False)
     assert out["ok"].all()
+
+
+@pytest.mark.parametrize("n,subch", [(384, 64), (768, 320), (1536, 1024)])
+def test_pilot_fit_is_the_ordered_sums(n, subch):
+    """The pilots' shift, its worth and its rounding as the reference's ordered double sums give them, over shifts about
+    the threshold of turning back, and where the sums say little (no noise, an empty spectrum, scales at float's ends)."""
+    fmt = lz.Format(n, subch, 128)
+    o = oracle.Fmt(n, subch, 128)
+    rng = np.random.default_rng(n)
+    u, v = fmt.uv[0::2].astype(np.float64), fmt.uv[1::2].astype(np.float64)
+    sym = (1.0 - 2.0 * fmt.white[0::2]) + 1j * (1.0 - 2.0 * fmt.white[1::2])
+    cases = [(rng.normal(0, s, 2), noise, scale) for s in (0.0, 3e-4, 1e-3, 3e-3, 1e-2, 0.1) for noise in (0.0, 0.1, 0.7) for scale in (1.0, 400.0)]
+    cases += [((0.01, -0.02), 0.3, 0.0), ((0.01, -0.02), 0.3, 1e-18), ((0.01, -0.02), 0.3, 1e14), ((0.3, 0.2), 0.0, 1e-9)]
+    coef = np.empty((len(cases), u.size), np.complex64)
+    for i, (d, noise, scale) in enumerate(cases):
+        z = sym * np.exp(-2j * np.pi * (u * d[0] + v * d[1]) / n)
+        coef[i] = scale * (z + noise * (rng.standard_normal(u.size) + 1j * rng.standard_normal(u.size)))
+    rx = lz.Receiver(n, subch, 128, max_frames=len(cases))
+    got = rx.finish_coef(coef)["align"]
+    turned = 0
+    for i in range(len(cases)):
+        want, _ = o.pilot_align(coef[i].view(np.float32))
+        assert np.array_equal(got[i, :2], want), (i, cases[i], got[i], want)
+        assert got[i, 2] == float(np.any(want != 0))
+        turned += int(np.any(want != 0))
+    assert 0 < turned < len(cases)
