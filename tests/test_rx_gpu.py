@@ -133,3 +133,29 @@ def test_pilot_fit_is_the_ordered_sums(n, subch):
         assert got[i, 2] == float(np.any(want != 0))
         turned += int(np.any(want != 0))
     assert 0 < turned < len(cases)
+
+
+@pytest.mark.parametrize("turn", [False, True])
+def test_finish_coef_from_and_to_unaligned_buffers(turn):
+    """Spectra 8 bytes past a 16-byte boundary, soft values and blocks at odd addresses: the values of the aligned call."""
+    import ctypes
+    import torch
+    fmt = lz.Format(512, 128, 128)
+    _, _, res = oracle_frames(fmt, 2, seed=11, shift=(0.2, 0.1) if turn else None)
+    rx = lz.Receiver(512, 128, 128, max_frames=2)
+    coef = np.ascontiguousarray(np.stack([r["coef"] for r in res]), np.float32).reshape(2, -1)
+    want = rx.finish_coef(coef)
+    assert bool(want["align"][:, 2].all()) == turn
+    o, s = lz.rx_outputs(fmt, 2, keep=True)
+    d = torch.zeros(coef.size + 8, dtype=torch.float32, device="cuda")
+    d[2:2 + coef.size] = torch.from_numpy(coef.ravel()).cuda()
+    soft = torch.zeros(o["llrf"].numel() + 16, dtype=torch.int8, device="cuda")
+    blocks = torch.zeros(o["blocks"].numel() + 16, dtype=torch.uint8, device="cuda")
+    s.llrf, s.blocks = soft.data_ptr() + 2, blocks.data_ptr() + 1
+    lz._check(lz.lib().lizg_rx_finish_coef_dev(rx._h, ctypes.c_void_p(d.data_ptr() + 8), 2, ctypes.byref(s),
+                                               ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), "finish_coef")
+    torch.cuda.synchronize()
+    assert np.array_equal(soft[2:2 + o["llrf"].numel()].cpu().numpy(), want["llrf"].ravel())
+    assert np.array_equal(blocks[1:1 + o["blocks"].numel()].cpu().numpy(), want["blocks"].ravel())
+    for k in ("its", "ok", "est", "pilot", "sub_est", "sub_rms"):
+        assert np.array_equal(o[k].cpu().numpy(), want[k], equal_nan=k == "pilot"), k
