@@ -3,14 +3,14 @@
 //
 // Four kernels a batch (five when the samples come straight from captured frames):
 //   hole_rhs_kernel   a CTA takes a band of the frame's every-eighth-sample rows: the shading fit's right-hand side
-//                     over the samples outside the anchors' squares, one partial sum a band (6 doubles);
+//                     over the samples outside the anchors' squares, one partial sum a band (6 doubles); the frame's
+//                     last CTA to finish adds the bands and solves for the shading surface beta;
 //   cell_table_kernel (captured frames only) each picture row's homography terms and the mesh displacement line of
 //                     each mesh cell along it, so the column pass reads them instead of walking the mesh per sample;
 //   fft_cols_kernel   a CTA takes 2L picture columns of a frame (L complex lines: column x0 + l real, x0 + L + l
-//                     imaginary), forms the shading surface beta from the bands' partials, erases the anchors' squares
-//                     as it loads them, sums each column's detrend moments, transforms the L lines along y in shared
+//                     imaginary), erases the anchors' squares to the shading surface, loads the rest, sums each column's detrend moments, transforms the L lines along y in shared
 //                     memory and separates the two real columns of each, writing Y[v][x] for the kept rows v;
-//   fac_kernel        one CTA a frame: the five projections from the columns' moments, then the surface spectrum's
+//   fac_kernel        kFacCtas CTAs a frame: the five projections from the columns' moments, then the surface spectrum's
 //                     per-column and per-row factors (the double products the reference rounds to float);
 //   fft_rows_kernel   a CTA takes L kept rows v of a frame, transforms along x and subtracts the surface's spectrum
 //                     (the xy term everywhere, the x terms on v = 0, the y terms on u = 0), writing the used
@@ -209,21 +209,12 @@ __device__ __forceinline__ void fft_lines(float2 *buf, const float2 *tw, int Lr)
   pass<N, P.r2, P.r0 * P.r1, P.lines>(buf, tw, Lr);
 }
 
-// A frame's shading-fit sample (x, y) = (8 kx, 8 ky): from the captured frame through its registration when the
-// frame is given (the decode's read as the reference's finish takes these samples, one call over every eighth row and
-// column, liblizard/src/lizard_phy.c:1611; or the exact walk), else from a supplied grid.
-__device__ __forceinline__ float shade_at(const SrcDev &s, int f, int kx, int ky) {
-  const int x = 8 * kx, y = 8 * ky;
+// A frame's shading-fit sample (x, y) = (8 kx, 8 ky) from a supplied grid or by the exact walk of the captured frame
+// (the decode's read walks the row: hole_rhs_band).
+__device__ __forceinline__ float shade_at(const SrcDev &s, int f, int x, int y) {
   if (!s.luma) return s.grid[f * s.gstride + (int64_t)y * s.sd.n + x];
   const float *H = s.reg + (int64_t)f * s.regstride;
-  const uint8_t *px = s.luma + f * s.fstride;
-  const float4 ct = s.sd.colt[x], rt = s.sd.rowt[y];
-  if (s.sd.read != LIZG_READ_DECODE) return sample_xy_exact(s.sd, px, s.w, s.h, s.pitch, H, H + 9, ct, rt);
-  const RowTerms r = row_terms(H, rt);
-  const LinCol c = lin_col_shade(s.sd, H, kx);
-  LinNum n = lin_start(c, r.kw, r.ku, r.kv);
-  lin_steps(c, n, c.g);
-  return lin_point(px, s.w, s.h, s.pitch, n, lin_cell(s.sd, H + 9, ct, r.j), r.v);
+  return sample_xy_exact(s.sd, s.luma + f * s.fstride, s.w, s.h, s.pitch, H, H + 9, s.sd.colt[x], s.sd.rowt[y]);
 }
 
 __device__ __forceinline__ bool in_square(const FftDev &xd, int t) {
@@ -233,44 +224,104 @@ __device__ __forceinline__ bool in_square(const FftDev &xd, int t) {
   return in;
 }
 
-// The shading fit's right-hand side (liblizard/src/lizard_phy.c:1609-1623) over kHoleBand of the frame's
-// every-eighth rows: hole[f][band][0..5]. A warp takes a row: its samples outside the squares summed in float as
-// z, z c(x), z q(x) (the basis is separable: 1, c(x), q(x), c(y), q(y), c(x) c(y)), then the row's six terms added
-// in double; the warps' sums added in warp order.
-__device__ __forceinline__ void hole_rhs_band(const FftDev &xd, const SrcDev &src, int bands, double *hole, int f, int band) {
-  const int n = xd.n, c = n / 8;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ky1 = min(c, (band + 1) * kHoleBand);
-  double rhs[6] = {0, 0, 0, 0, 0, 0};
-  for (int ky = band * kHoleBand + warp; ky < ky1; ky += 8) {
-    const int y = 8 * ky;
+// The shading fit's right-hand side (liblizard/src/lizard_phy.c:1609-1623) over kHoleBand of the frame's every-eighth
+// rows, hole[f][band][0..5], then, by the frame's last CTA to finish (its ticket), the surface beta[f][0..5] from the bands
+// in order. A warp takes a row: its samples outside the squares summed in float as z, z c(x), z q(x) (the basis is
+// separable: 1, c(x), q(x), c(y), q(y), c(x) c(y)), then the row's six terms added in double, rows w and w + 8, then w in
+// order. The decode's read is the reference's one call over every eighth column (liblizard/src/lizard_phy.c:1611): lane l
+// takes columns l, l + 32, ..., so its homography lane is walked on eight steps from one to the next, and the at most
+// six samples' loads are in flight together. Bound: latency. A frame of n = 1536: 26 us with two rows a warp, each sample
+// walked from the first column, 15 so; and the column pass no longer adds the bands in every CTA (39 us, 35).
+constexpr int kHoleThreads = 32 * kHoleBand, kHoleCols = 6;
+static_assert(kHoleBand == 16, "rows w and w + 8 of a band share a sum");
+__device__ __forceinline__ void hole_rhs_band(const FftDev &xd, const SrcDev &src, int bands, double *hole, double *beta, int *ticket, int f,
+                                              int band) {
+  __shared__ float s_row[kHoleBand][3];
+  __shared__ double s_red[8][6], s_rhs[6];
+  __shared__ bool s_last;
+  const int n = xd.n, c = n / 8, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ky = band * kHoleBand + warp, y = 8 * ky;
+  if (ky < c) {
     const bool ysq = in_square(xd, y);
+    float v[kHoleCols];
+    if (src.luma && src.sd.read == LIZG_READ_DECODE) {
+      const float *H = src.reg + (int64_t)f * src.regstride;
+      const uint8_t *px = src.luma + f * src.fstride;
+      const RowTerms r = row_terms(H, src.sd.rowt[y]);
+      const LinCol lc = lin_col_shade(src.sd, H, lane);
+      LinNum s = lin_start(lc, r.kw, r.ku, r.kv);
+      lin_steps(lc, s, lc.g);
+#pragma unroll
+      for (int m = 0; m < kHoleCols; m++) {
+        const int x = 8 * min(lane + 32 * m, c - 1);
+        v[m] = lin_point(px, src.w, src.h, src.pitch, s, lin_cell(src.sd, H + 9, src.sd.colt[x], r.j), r.v);
+#pragma unroll
+        for (int q = 0; q < 8; q++) lin_steps(lc, s, 1);
+      }
+    } else {
+#pragma unroll
+      for (int m = 0; m < kHoleCols; m++) v[m] = shade_at(src, f, 8 * min(lane + 32 * m, c - 1), y);
+    }
     float s0 = 0, s1 = 0, s2 = 0;
-    for (int kx = lane; kx < c; kx += 32) {
-      const int x = 8 * kx;
-      if (ysq && in_square(xd, x)) continue;
-      const float v = shade_at(src, f, kx, ky);
-      s0 += v; s1 += __ldg(xd.cx + x) * v; s2 += __ldg(xd.qx + x) * v;
+#pragma unroll
+    for (int m = 0; m < kHoleCols; m++) {
+      const int kx = lane + 32 * m, x = 8 * kx;
+      if (kx < c && !(ysq && in_square(xd, x))) { s0 += v[m]; s1 += __ldg(xd.cx + x) * v[m]; s2 += __ldg(xd.qx + x) * v[m]; }
     }
     for (int o = 16; o > 0; o >>= 1) {
       s0 += __shfl_xor_sync(0xffffffffu, s0, o);
       s1 += __shfl_xor_sync(0xffffffffu, s1, o);
       s2 += __shfl_xor_sync(0xffffffffu, s2, o);
     }
-    const double cy = xd.cx[y], qy = xd.qx[y];
-    rhs[0] += s0; rhs[1] += s1; rhs[2] += s2; rhs[3] += cy * s0; rhs[4] += qy * s0; rhs[5] += cy * s1;
+    if (lane == 0) { s_row[warp][0] = s0; s_row[warp][1] = s1; s_row[warp][2] = s2; }
   }
-  __shared__ double red[8][6];
-  if (lane == 0)
-    for (int r = 0; r < 6; r++) red[warp][r] = rhs[r];
   __syncthreads();
-  if (threadIdx.x < 6) {
+  if (tid < 48) {
+    const int w = tid / 6, r = tid % 6, k = r < 3 ? r : r == 5 ? 1 : 0;   // terms s0, s1, s2, c(y) s0, q(y) s0, c(y) s1
     double acc = 0;
-    for (int w = 0; w < 8; w++) acc += red[w][threadIdx.x];
-    hole[((int64_t)f * bands + band) * 6 + threadIdx.x] = acc;
+    for (int row = w; row < kHoleBand; row += 8) {
+      const int kr = band * kHoleBand + row;
+      if (kr >= c) break;
+      const double sv = s_row[row][k], b = r < 3 ? 1.0 : r == 4 ? xd.qx[8 * kr] : xd.cx[8 * kr];
+      acc = fma(b, sv, acc);
+    }
+    s_red[w][r] = acc;
   }
+  __syncthreads();
+  if (tid < 6) {
+    double acc = 0;
+    for (int w = 0; w < 8; w++) acc += s_red[w][tid];
+    __stcg(hole + ((int64_t)f * bands + band) * 6 + tid, acc);
+    __threadfence();
+  }
+  __syncthreads();
+  if (tid == 0) {
+    s_last = atomicAdd(ticket + f, 1) == bands - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!s_last || tid >= 32) return;
+  if (tid < 6) {
+    double acc = 0;
+    for (int b0 = 0; b0 < bands; b0 += 12) {   // the bands' loads in flight, then added in order
+      double v[12];
+#pragma unroll
+      for (int k = 0; k < 12; k++) v[k] = b0 + k < bands ? __ldcg(hole + ((int64_t)f * bands + b0 + k) * 6 + tid) : 0.0;
+#pragma unroll
+      for (int k = 0; k < 12; k++) if (b0 + k < bands) acc += v[k];
+    }
+    s_rhs[tid] = acc;
+  }
+  __syncwarp();
+  if (tid < 6) {
+    double acc = 0;
+#pragma unroll
+    for (int k = 0; k < 6; k++) acc += xd.hole_inv[tid * 6 + k] * s_rhs[k];
+    beta[6 * f + tid] = acc;
+  }
+  if (tid == 0) ticket[f] = 0;   // as the next call finds it
 }
-__global__ void __launch_bounds__(256) hole_rhs_kernel(FftDev xd, SrcDev src, int bands, double *hole) {
-  hole_rhs_band(xd, src, bands, hole, blockIdx.x / bands, blockIdx.x % bands);
+__global__ void __launch_bounds__(kHoleThreads) hole_rhs_kernel(FftDev xd, SrcDev src, int bands, double *hole, double *beta, int *ticket) {
+  hole_rhs_band(xd, src, bands, hole, beta, ticket, blockIdx.x / bands, blockIdx.x % bands);
 }
 
 // The transform CTA's shared memory: the lines, the twiddles, the moments' reduction.
@@ -297,10 +348,9 @@ struct FftColsSeg {
   FftDev xd;
   SrcDev src;
   const float4 *ctab;
-  const double *hole;
+  const double *beta;
   double *part;
   float2 *Y;
-  int bands;
 };
 struct FftColsMix {
   FftColsSeg seg[kFftMixSegs];
@@ -431,7 +481,7 @@ __device__ __forceinline__ void load_tile(const FftDev &xd, const SrcDev &src, c
 
 // The column pass's per-CTA scalars in shared memory.
 struct ColsShared {
-  double rhs[6], beta[6];
+  double beta[6];
   double h2[32], cx[32];   // a column's part of the surface and its c(x), the tile's columns inside a square
   float part[kThreads / 32][5];
 };
@@ -480,30 +530,18 @@ __device__ __forceinline__ void erase_tile(const FftDev &xd, int x0, float2 *buf
   __syncthreads();
 }
 
-// The column pass on one tile (frame f, columns x0 = 2 L tile .. x0 + 2L - 1): the shading surface beta from the
-// frame's bands, the tile's samples (erased, projections summed: part[f][tile][0..4]), the L lines' transforms along
+// The column pass on one tile (frame f, columns x0 = 2 L tile .. x0 + 2L - 1): the tile's samples (erased, projections summed: part[f][tile][0..4]), the L lines' transforms along
 // y, and the two real columns of each line separated: A(v) = (Z(v) + conj Z(n - v)) / 2, B(v) = -i (Z(v) - conj
 // Z(n - v)) / 2, written to Y[f][v][x] for the kept rows v. Every thread of the CTA takes part.
 template <int N>
-__device__ __forceinline__ void cols_tile(const FftDev &xd, const SrcDev &src, const float4 *ctab, int bands, const double *hole,
+__device__ __forceinline__ void cols_tile(const FftDev &xd, const SrcDev &src, const float4 *ctab, const double *beta,
                                           double *part, float2 *Y, int f, int tile, unsigned char *smraw, ColsShared &s) {
   constexpr int n = N, L = plan_of(N).lines, LSTR = lstride_of(N), tiles = n / (2 * L), ystep = kThreads / L;
   const SmemMap sm = smem_map<N>(smraw);
   const int tid = threadIdx.x, l = tid % L, warp = tid >> 5, lane = tid & 31, x0 = tile * 2 * L;
   for (int i = tid; i < n; i += kThreads) sm.tw[i] = xd.tws[i];
   float2 *line = sm.buf + l * LSTR;
-  if (tid < 6) {
-    double acc = 0;
-    for (int b = 0; b < bands; b++) acc += hole[((int64_t)f * bands + b) * 6 + tid];
-    s.rhs[tid] = acc;
-  }
-  __syncthreads();
-  if (tid < 6) {
-    double acc = 0;
-#pragma unroll
-    for (int k = 0; k < 6; k++) acc += xd.hole_inv[tid * 6 + k] * s.rhs[k];
-    s.beta[tid] = acc;
-  }
+  if (tid < 6) s.beta[tid] = beta[6 * f + tid];
   __syncthreads();
   erase_tile<N>(xd, x0, sm.buf, s);
   float p[5] = {0, 0, 0, 0, 0};
@@ -533,12 +571,12 @@ __device__ __forceinline__ void cols_tile(const FftDev &xd, const SrcDev &src, c
 
 // The column pass of one picture size: CTA b takes tile b mod tiles of frame b / tiles.
 template <int N>
-__global__ void __launch_bounds__(kThreads, 3) fft_cols_kernel(FftDev xd, SrcDev src, const float4 *ctab, int bands, const double *hole, double *part,
+__global__ void __launch_bounds__(kThreads, 3) fft_cols_kernel(FftDev xd, SrcDev src, const float4 *ctab, const double *beta, double *part,
                                                                 float2 *Y) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ ColsShared s;
   constexpr int tiles = N / (2 * plan_of(N).lines);
-  cols_tile<N>(xd, src, ctab, bands, hole, part, Y, blockIdx.x / tiles, blockIdx.x % tiles, smraw, s);
+  cols_tile<N>(xd, src, ctab, beta, part, Y, blockIdx.x / tiles, blockIdx.x % tiles, smraw, s);
 }
 
 // The column pass over several picture sizes in one grid: a queue of (format, frame, tile) items, format k's at CTAs
@@ -552,44 +590,50 @@ __global__ void __launch_bounds__(kThreads, 3) fft_cols_mixed_kernel(const __gri
   const FftColsSeg &g = m.seg[k];
   const int b = (int)blockIdx.x - m.first[k], tiles = g.xd.n / (2 * plan_of(g.xd.n).lines), f = b / tiles, tile = b - f * tiles;
   switch (g.xd.n) {
-    case 384: cols_tile<384>(g.xd, g.src, g.ctab, g.bands, g.hole, g.part, g.Y, f, tile, smraw, s); break;
-    case 512: cols_tile<512>(g.xd, g.src, g.ctab, g.bands, g.hole, g.part, g.Y, f, tile, smraw, s); break;
-    case 768: cols_tile<768>(g.xd, g.src, g.ctab, g.bands, g.hole, g.part, g.Y, f, tile, smraw, s); break;
-    case 1024: cols_tile<1024>(g.xd, g.src, g.ctab, g.bands, g.hole, g.part, g.Y, f, tile, smraw, s); break;
-    case 1152: cols_tile<1152>(g.xd, g.src, g.ctab, g.bands, g.hole, g.part, g.Y, f, tile, smraw, s); break;
-    case 1280: cols_tile<1280>(g.xd, g.src, g.ctab, g.bands, g.hole, g.part, g.Y, f, tile, smraw, s); break;
-    default: cols_tile<1536>(g.xd, g.src, g.ctab, g.bands, g.hole, g.part, g.Y, f, tile, smraw, s); break;
+    case 384: cols_tile<384>(g.xd, g.src, g.ctab, g.beta, g.part, g.Y, f, tile, smraw, s); break;
+    case 512: cols_tile<512>(g.xd, g.src, g.ctab, g.beta, g.part, g.Y, f, tile, smraw, s); break;
+    case 768: cols_tile<768>(g.xd, g.src, g.ctab, g.beta, g.part, g.Y, f, tile, smraw, s); break;
+    case 1024: cols_tile<1024>(g.xd, g.src, g.ctab, g.beta, g.part, g.Y, f, tile, smraw, s); break;
+    case 1152: cols_tile<1152>(g.xd, g.src, g.ctab, g.beta, g.part, g.Y, f, tile, smraw, s); break;
+    case 1280: cols_tile<1280>(g.xd, g.src, g.ctab, g.beta, g.part, g.Y, f, tile, smraw, s); break;
+    default: cols_tile<1536>(g.xd, g.src, g.ctab, g.beta, g.part, g.Y, f, tile, smraw, s); break;
   }
 }
 
-// The five projections of each frame from its column tiles' sums, in tile order, normalised
-// (liblizard/src/lizard_phy.c:1697), then the surface spectrum's factors (liblizard/src/lizard_phy.c:1702-1716),
-// rounded to float as there: fac[f] = xy[u] (pxy X1[u]) for u < n, x0[u] (n (px X1[u] + pxx X2[u])) for u < n,
-// y0[v] (n (py X1[v] + pyy X2[v])) for v < vrows.
-__device__ __forceinline__ void fac_frame(const FftDev &xd, int tiles, const double *part, float2 *fac, int f) {
-  const int n = xd.n;
+// The five projections of each frame from its column tiles' sums, normalised (liblizard/src/lizard_phy.c:1697), then the
+// surface spectrum's factors (liblizard/src/lizard_phy.c:1702-1716), rounded to float as there: fac[f] = xy[u] (pxy
+// X1[u]) for u < n, x0[u] (n (px X1[u] + pxx X2[u])) for u < n, y0[v] (n (py X1[v] + pyy X2[v])) for v < vrows. Each of a
+// frame's kFacCtas CTAs adds the tiles itself (a warp a projection, as a tree) and takes its share of the factors: one CTA
+// a frame adding the tiles in a chain held one SM's double pipe 27 us at n = 1536; 6 so (9 for 32 frames).
+constexpr int kFacCtas = 8;
+__device__ __forceinline__ void fac_frame(const FftDev &xd, int tiles, const double *part, float2 *fac, int f, int piece) {
+  const int n = xd.n, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   __shared__ double s_p[5];
-  if (threadIdx.x < 5) {
+  if (warp < 5) {
     double acc = 0;
-    for (int t = 0; t < tiles; t++) acc += part[((int64_t)f * tiles + t) * 5 + threadIdx.x];
-    s_p[threadIdx.x] = acc;
+#pragma unroll 6
+    for (int t = lane; t < tiles; t += 32) acc += part[((int64_t)f * tiles + t) * 5 + warp];
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    // z c(x), z c(y): n sx2; z c(x) c(y): sx2 sx2; z q(x), z q(y): n sq2
+    if (lane == 0) s_p[warp] = acc / (warp < 2 ? n * xd.sx2 : warp == 2 ? xd.sx2 * xd.sx2 : n * xd.sq2);
   }
   __syncthreads();
-  const double px = s_p[0] / (n * xd.sx2), py = s_p[1] / (n * xd.sx2), pxy = s_p[2] / (xd.sx2 * xd.sx2);
-  const double pxx = s_p[3] / (n * xd.sq2), pyy = s_p[4] / (n * xd.sq2);
+  const double px = s_p[0], py = s_p[1], pxy = s_p[2], pxx = s_p[3], pyy = s_p[4];
   float2 *o = fac + (int64_t)f * (2 * n + xd.vrows);
-  for (int u = threadIdx.x; u < n; u += blockDim.x) {
-    const float2 x1 = xd.x1[u], x2 = xd.x2[u];
-    o[u] = make_float2((float)(pxy * x1.x), (float)(pxy * x1.y));
-    o[n + u] = make_float2((float)(n * (px * x1.x + pxx * x2.x)), (float)(n * (px * x1.y + pxx * x2.y)));
-  }
-  for (int v = threadIdx.x; v < xd.vrows; v += blockDim.x) {
-    const float2 x1 = xd.x1[v], x2 = xd.x2[v];
-    o[2 * n + v] = make_float2((float)(n * (py * x1.x + pyy * x2.x)), (float)(n * (py * x1.y + pyy * x2.y)));
+  for (int i = piece * blockDim.x + threadIdx.x; i < 2 * n + xd.vrows; i += kFacCtas * blockDim.x) {
+    const int k = i < n ? i : i < 2 * n ? i - n : i - 2 * n;
+    const float2 x1 = xd.x1[k];
+    if (i < n) {
+      o[i] = make_float2((float)(pxy * x1.x), (float)(pxy * x1.y));
+    } else {
+      const float2 x2 = xd.x2[k];
+      const double a = i < 2 * n ? px : py, b = i < 2 * n ? pxx : pyy;
+      o[i] = make_float2((float)(n * (a * x1.x + b * x2.x)), (float)(n * (a * x1.y + b * x2.y)));
+    }
   }
 }
 __global__ void __launch_bounds__(256) fac_kernel(FftDev xd, int tiles, const double *part, float2 *fac) {
-  fac_frame(xd, tiles, part, fac, blockIdx.x);
+  fac_frame(xd, tiles, part, fac, blockIdx.x / kFacCtas, blockIdx.x % kFacCtas);
 }
 
 // The shading sums, the sampler's tables and the surface factors over several formats' batches, one launch a stage:
@@ -598,7 +642,8 @@ __global__ void __launch_bounds__(256) fac_kernel(FftDev xd, int tiles, const do
 struct FftLightSeg {
   FftDev xd;
   SrcDev src;
-  double *hole, *part;
+  double *hole, *beta, *part;
+  int *ticket;
   float4 *ctab;
   float2 *fac;
   int bands, per_frame, tblocks, tiles;
@@ -614,24 +659,25 @@ __device__ __forceinline__ int seg_at(const int *first, int nseg, int b) {
   while (k < nseg - 1 && b >= first[k + 1]) k++;
   return k;
 }
-__global__ void __launch_bounds__(256) fft_pre_mixed_kernel(const __grid_constant__ FftLightMix m) {
+__global__ void __launch_bounds__(kHoleThreads) fft_pre_mixed_kernel(const __grid_constant__ FftLightMix m) {
   const int b = blockIdx.x;
   if (b < m.hf[m.nseg]) {
     const int k = seg_at(m.hf, m.nseg, b);
     const FftLightSeg &g = m.seg[k];
     const int lb = b - m.hf[k];
-    hole_rhs_band(g.xd, g.src, g.bands, g.hole, lb / g.bands, lb % g.bands);
+    hole_rhs_band(g.xd, g.src, g.bands, g.hole, g.beta, g.ticket, lb / g.bands, lb % g.bands);
   } else {
     const int k = seg_at(m.tf, m.nseg, b);
     const FftLightSeg &g = m.seg[k];
     const int lb = b - m.tf[k], f = lb / g.tblocks;
-    cell_table_entry(g.src, g.per_frame, g.ctab, f, (lb - f * g.tblocks) * 256 + threadIdx.x);
+    cell_table_entry(g.src, g.per_frame, g.ctab, f, (lb - f * g.tblocks) * kHoleThreads + threadIdx.x);
   }
 }
 __global__ void __launch_bounds__(256) fac_mixed_kernel(const __grid_constant__ FftLightMix m) {
   const int k = seg_at(m.ff, m.nseg, blockIdx.x);
   const FftLightSeg &g = m.seg[k];
-  fac_frame(g.xd, g.tiles, g.part, g.fac, blockIdx.x - m.ff[k]);
+  const int b = blockIdx.x - m.ff[k];
+  fac_frame(g.xd, g.tiles, g.part, g.fac, b / kFacCtas, b % kFacCtas);
 }
 
 // A bounded wait on an mbarrier's phase (try_wait blocks a while in hardware before it answers): false when the
@@ -783,7 +829,7 @@ int fft_y_map(CUtensorMap *map, float2 *Y, int n, int64_t rows) {
 // The shading fit's partial sums, then (captured frames only) the sampler's row and cell table.
 cudaError_t fft_pre_launch(const FftSegArgs &a, cudaStream_t st) {
   const int bands = fft_hole_bands(a.xd.n);
-  hole_rhs_kernel<<<a.frames * bands, 256, 0, st>>>(a.xd, a.src, bands, a.b.hole);
+  hole_rhs_kernel<<<a.frames * bands, kHoleThreads, 0, st>>>(a.xd, a.src, bands, a.b.hole, a.b.beta, a.b.ticket);
   if (!a.src.grid) {
     if (!a.b.ctab || a.src.sd.nx != a.src.sd.ny) return cudaErrorInvalidValue;
     const int per_frame = a.xd.n * a.src.sd.nx;
@@ -793,7 +839,7 @@ cudaError_t fft_pre_launch(const FftSegArgs &a, cudaStream_t st) {
 }
 
 cudaError_t fft_fac_launch(const FftSegArgs &a, cudaStream_t st) {
-  fac_kernel<<<a.frames, 256, 0, st>>>(a.xd, a.xd.n / (2 * plan_of(a.xd.n).lines), a.b.part, a.b.fac);
+  fac_kernel<<<a.frames * kFacCtas, 256, 0, st>>>(a.xd, a.xd.n / (2 * plan_of(a.xd.n).lines), a.b.part, a.b.fac);
   return cudaGetLastError();
 }
 
@@ -810,7 +856,7 @@ static cudaError_t fft_launch_n(const FftDev &xd, int frames, const SrcDev &src,
   (void)sms;
   const FftSegArgs a{xd, src, b, frames};
   if ((e = fft_pre_launch(a, st)) != cudaSuccess) return e;
-  fft_cols_kernel<N><<<frames * tiles, kThreads, smem, st>>>(xd, src, b.ctab, fft_hole_bands(N), b.hole, b.part, b.Y);
+  fft_cols_kernel<N><<<frames * tiles, kThreads, smem, st>>>(xd, src, b.ctab, b.beta, b.part, b.Y);
   if ((e = fft_fac_launch(a, st)) != cudaSuccess) return e;
   if (!b.ymap || !b.err) return cudaErrorInvalidValue;
   fft_rows_kernel<N><<<frames * ((xd.vrows + L - 1) / L), kThreads, smem, st>>>(xd, b.fac, *b.ymap, b.tpos, b.need, b.C, b.err);
@@ -832,11 +878,11 @@ static cudaError_t light_mix(const FftSegArgs *a, int count, FftLightMix &m) {
     const FftSegArgs &s = a[k];
     if (!ladder_size(s.xd.n) || s.frames < 1 || s.src.grid || !s.b.ctab || s.src.sd.nx != s.src.sd.ny) return cudaErrorInvalidValue;
     FftLightSeg &g = m.seg[k];
-    g.xd = s.xd; g.src = s.src; g.hole = s.b.hole; g.part = s.b.part; g.ctab = s.b.ctab; g.fac = s.b.fac;
-    g.bands = fft_hole_bands(s.xd.n); g.per_frame = s.xd.n * s.src.sd.nx; g.tblocks = (g.per_frame + 255) / 256;
+    g.xd = s.xd; g.src = s.src; g.hole = s.b.hole; g.beta = s.b.beta; g.ticket = s.b.ticket; g.part = s.b.part; g.ctab = s.b.ctab; g.fac = s.b.fac;
+    g.bands = fft_hole_bands(s.xd.n); g.per_frame = s.xd.n * s.src.sd.nx; g.tblocks = (g.per_frame + kHoleThreads - 1) / kHoleThreads;
     g.tiles = s.xd.n / (2 * plan_of(s.xd.n).lines);
     m.hf[k + 1] = m.hf[k] + s.frames * g.bands;
-    m.ff[k + 1] = m.ff[k] + s.frames;
+    m.ff[k + 1] = m.ff[k] + s.frames * kFacCtas;
   }
   m.tf[0] = m.hf[count];
   for (int k = 0; k < count; k++) m.tf[k + 1] = m.tf[k] + a[k].frames * m.seg[k].tblocks;
@@ -846,7 +892,7 @@ static cudaError_t light_mix(const FftSegArgs *a, int count, FftLightMix &m) {
 cudaError_t fft_pre_mixed_launch(const FftSegArgs *a, int count, cudaStream_t st) {
   FftLightMix m;
   if (cudaError_t e = light_mix(a, count, m)) return e;
-  fft_pre_mixed_kernel<<<m.tf[count], 256, 0, st>>>(m);
+  fft_pre_mixed_kernel<<<m.tf[count], kHoleThreads, 0, st>>>(m);
   return cudaGetLastError();
 }
 
@@ -869,7 +915,7 @@ cudaError_t fft_cols_mixed_launch(const FftSegArgs *a, int count, cudaStream_t s
     const FftSegArgs &s = a[k];
     if (!ladder_size(s.xd.n) || s.frames < 1) return cudaErrorInvalidValue;
     FftColsSeg &g = m.seg[k];
-    g.xd = s.xd; g.src = s.src; g.ctab = s.b.ctab; g.hole = s.b.hole; g.part = s.b.part; g.Y = s.b.Y; g.bands = fft_hole_bands(s.xd.n);
+    g.xd = s.xd; g.src = s.src; g.ctab = s.b.ctab; g.beta = s.b.beta; g.part = s.b.part; g.Y = s.b.Y;
     m.first[k + 1] = m.first[k] + s.frames * (s.xd.n / (2 * plan_of(s.xd.n).lines));
     smem = cmax_i(smem, smem_bytes_of(s.xd.n));
   }

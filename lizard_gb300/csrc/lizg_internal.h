@@ -73,6 +73,8 @@ struct FftBufs {
   // pass's bulk tensor loads, and a device word the passes set when a bounded wait gave up
   const CUtensorMap *ymap;
   int *err;
+  double *beta;                      // frames x 6: the shading surface
+  int *ticket;                       // frames: the shading fit's CTAs done, 0 between calls
 };
 // Encodes the tensor map of a Y buffer of `rows` rows of n complex points (the row pass's loads). 0, or a CUresult.
 int fft_y_map(CUtensorMap *map, float2 *Y, int n, int64_t rows);

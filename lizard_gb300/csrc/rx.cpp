@@ -29,7 +29,8 @@ struct lizg_rx {
   float *sub_rms = nullptr, *est = nullptr, *pilot = nullptr, *align = nullptr;
   uint8_t *decl = nullptr;
   int *counters = nullptr;
-  double *hole = nullptr, *part = nullptr;
+  double *hole = nullptr, *beta = nullptr, *part = nullptr;
+  int *ticket = nullptr;
   float2 *fac = nullptr;
   lizg::SampleDev sd{};
   float *node_xy = nullptr;
@@ -174,6 +175,9 @@ lizg_rx *lizg_rx_new(int n, int subch, int span, int max_frames) {
   }
   const size_t F = (size_t)max_frames;
   ok(dev_alloc(r, &r->hole, F * lizg::fft_hole_bands(n) * 6));
+  ok(dev_alloc(r, &r->beta, F * 6));
+  ok(dev_alloc(r, &r->ticket, F));
+  if (e == cudaSuccess) e = cudaMemset(r->ticket, 0, F * sizeof(int));
   ok(dev_alloc(r, &r->fac, F * (2 * (size_t)n + r->xd.vrows)));
   ok(dev_alloc(r, &r->part, F * (size_t)(n / 2) * 5));   // column tiles (at most n / 2) x 5
   ok(dev_alloc(r, &r->Y, F * (size_t)r->xd.vrows * n));
@@ -378,7 +382,7 @@ int lizg_rx_finish_coef_dev(lizg_rx *r, const float *d_coef, int frames, const l
 static int finish_src(lizg_rx *r, const lizg::SrcDev &src, int frames, const lizg_rx_out *out, float *d_coef, cudaStream_t st, int sms) {
   const int need = r->f.subch * lizg::kSub;
   float2 *C = d_coef ? reinterpret_cast<float2 *>(d_coef) : r->C;   // the caller's spectrum buffer when given
-  const lizg::FftBufs b{r->hole, r->part, r->fac, r->Y, r->tpos, need, C, r->ctab, &r->ymap, r->dev_err};
+  const lizg::FftBufs b{r->hole, r->part, r->fac, r->Y, r->tpos, need, C, r->ctab, &r->ymap, r->dev_err, r->beta, r->ticket};
   cudaError_t e = lizg::fft_launch(r->xd, frames, src, b, sms, st);
   if (e != cudaSuccess) return lizg::record_error(LIZG_E_CUDA, (std::string("transform: ") + cudaGetErrorString(e)).c_str());
   r->launches += src.grid ? 4 : 5;   // sampling in the column pass adds the sampler's row and cell table
@@ -404,7 +408,7 @@ int lizg_rx_spectrum_grid_dev(lizg_rx *r, const float *d_grid, int frames, float
   lizg::SrcDev src{};
   src.grid = d_grid; src.gstride = (int64_t)r->f.n * r->f.n; src.sd = r->sd;
   const int need = r->f.subch * lizg::kSub;
-  const lizg::FftBufs b{r->hole, r->part, r->fac, r->Y, r->tpos, need, reinterpret_cast<float2 *>(d_coef), r->ctab, &r->ymap, r->dev_err};
+  const lizg::FftBufs b{r->hole, r->part, r->fac, r->Y, r->tpos, need, reinterpret_cast<float2 *>(d_coef), r->ctab, &r->ymap, r->dev_err, r->beta, r->ticket};
   cudaError_t e = lizg::fft_launch(r->xd, frames, src, b, sms, static_cast<cudaStream_t>(stream));
   r->launches = 4;
   return e == cudaSuccess ? 0 : lizg::record_error(LIZG_E_CUDA, (std::string("lizg_rx_spectrum_grid_dev: ") + cudaGetErrorString(e)).c_str());
@@ -447,7 +451,7 @@ int lizg::rx_spectrum_luma(lizg_rx *r, const uint8_t *d_luma, int w, int h, int 
   src.sd = r->sd;
   src.luma = d_luma; src.w = w; src.h = h; src.pitch = pitch; src.fstride = frame_stride; src.reg = d_reg;
   src.regstride = 9 + 2 * r->sd.nx * r->sd.ny;
-  const lizg::FftBufs b{r->hole, r->part, r->fac, r->Y, r->tpos, r->f.subch * lizg::kSub, reinterpret_cast<float2 *>(d_coef), r->ctab, &r->ymap, r->dev_err};
+  const lizg::FftBufs b{r->hole, r->part, r->fac, r->Y, r->tpos, r->f.subch * lizg::kSub, reinterpret_cast<float2 *>(d_coef), r->ctab, &r->ymap, r->dev_err, r->beta, r->ticket};
   const cudaError_t e = lizg::fft_launch(r->xd, frames, src, b, sms, st);
   return e == cudaSuccess ? 0 : lizg::record_error(LIZG_E_CUDA, (std::string("spectrum from frames: ") + cudaGetErrorString(e)).c_str());
 }
@@ -466,7 +470,7 @@ int lizg::rx_call(lizg_rx *r, const uint8_t *d_luma, int w, int h, int pitch, in
   src.sd = r->sd;
   src.luma = d_luma; src.w = w; src.h = h; src.pitch = pitch; src.fstride = frame_stride; src.reg = d_reg;
   src.regstride = 9 + 2 * r->sd.nx * r->sd.ny;
-  c.fft.b = FftBufs{r->hole, r->part, r->fac, r->Y, r->tpos, r->f.subch * lizg::kSub, r->C, r->ctab, &r->ymap, r->dev_err};
+  c.fft.b = FftBufs{r->hole, r->part, r->fac, r->Y, r->tpos, r->f.subch * lizg::kSub, r->C, r->ctab, &r->ymap, r->dev_err, r->beta, r->ticket};
   c.fd = fmt_dev(r, frames);
   c.tiers = r->f.tiers;
   c.out = out;
