@@ -5,8 +5,10 @@
 //   hole_rhs_kernel   a CTA takes a band of the frame's every-eighth-sample rows: the shading fit's right-hand side
 //                     over the samples outside the anchors' squares, one partial sum a band (6 doubles); the frame's
 //                     last CTA to finish adds the bands and solves for the shading surface beta;
-//   cell_table_kernel (captured frames only) each picture row's homography terms and the mesh displacement line of
-//                     each mesh cell along it, so the column pass reads them instead of walking the mesh per sample;
+//   sample16_kernel   (captured frames by the decode's read) the samples, 16 bits each;
+//   cell_table_kernel (captured frames by the exact walk) each picture row's homography terms and the mesh displacement
+//                     line of each mesh cell along it, so the column pass reads them instead of walking the mesh per
+//                     sample;
 //   fft_cols_kernel   a CTA takes 2L picture columns of a frame (L complex lines: column x0 + l real, x0 + L + l
 //                     imaginary), erases the anchors' squares to the shading surface, loads the rest, sums each column's detrend moments, transforms the L lines along y in shared
 //                     memory and separates the two real columns of each, writing Y[v][x] for the kept rows v;
@@ -27,6 +29,7 @@
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <type_traits>
 #include "lizg_internal.h"
 #include "sample_dev.cuh"
 
@@ -202,11 +205,16 @@ __device__ __forceinline__ void pass(float2 *buf, const float2 *tw, int Lr) {
 // place by the size's three passes. tw: the passes' twiddles, pass s's at NS (a multiple of 16 past the first pass,
 // so a half-warp's 16 twiddles are one aligned 128-byte row). Every thread of the CTA takes part.
 template <int N>
+__device__ __forceinline__ void later_passes(float2 *buf, const float2 *tw, int Lr) {
+  constexpr Plan P = plan_of(N);
+  pass<N, P.r1, P.r0, P.lines>(buf, tw, Lr);
+  pass<N, P.r2, P.r0 * P.r1, P.lines>(buf, tw, Lr);
+}
+template <int N>
 __device__ __forceinline__ void fft_lines(float2 *buf, const float2 *tw, int Lr) {
   constexpr Plan P = plan_of(N);
   pass<N, P.r0, 1, P.lines>(buf, tw, Lr);
-  pass<N, P.r1, P.r0, P.lines>(buf, tw, Lr);
-  pass<N, P.r2, P.r0 * P.r1, P.lines>(buf, tw, Lr);
+  later_passes<N>(buf, tw, Lr);
 }
 
 // A frame's shading-fit sample (x, y) = (8 kx, 8 ky) from a supplied grid or by the exact walk of the captured frame
@@ -348,6 +356,7 @@ struct FftColsSeg {
   FftDev xd;
   SrcDev src;
   const float4 *ctab;
+  const int16_t *g16;
   const double *beta;
   double *part;
   float2 *Y;
@@ -373,110 +382,237 @@ struct FftRowsMix {
 };
 static_assert(sizeof(FftColsMix) <= 32000 && sizeof(FftRowsMix) <= 32000, "the mixed grids' arguments fit a launch");
 
-// The sampler's per-row quantities of a batch, worked out once a frame before the column pass reads them, with the
+// The exact walk's per-row quantities of a batch, worked out once a frame before the column pass reads them, with the
 // same functions and inputs as the per-sample walk (the cell's 1 / width as the column table computes it), so the
-// column pass reads the walk's own values. A thread an entry, entries in table order. The exact walk: for picture row
-// y and mesh cell i < nx - 1 the displacement line cell_terms gives, and at i = nx - 1 the homography's row terms
-// (kw, ku, kv). The decode's read: the row terms of row y at y < n, then each column x's displacement terms at mesh
-// row j (lin_cell) at n + j n + x.
+// column pass reads the walk's own values. A thread an entry, entries in table order: for picture row y and mesh cell
+// i < nx - 1 the displacement line cell_terms gives, and at i = nx - 1 the homography's row terms (kw, ku, kv).
 __device__ __forceinline__ void cell_table_entry(const SrcDev &src, int per_frame, float4 *ctab, int f, int t) {
   if (t >= per_frame) return;
   const SampleDev &sd = src.sd;
   const float *H = src.reg + (int64_t)f * src.regstride;
+  const int nn = sd.nx, y = t / nn, i = t - y * nn;
+  const RowTerms r = row_terms(H, sd.rowt[y]);
   float4 o;
-  if (sd.read == LIZG_READ_DECODE) {
-    if (t < sd.n) {
-      const RowTerms r = row_terms(H, sd.rowt[t]);
-      o = make_float4(r.kw, r.ku, r.kv, 0.0f);
-    } else {
-      const int j = (t - sd.n) / sd.n, x = t - sd.n - j * sd.n;
-      o = lin_cell(sd, H + 9, sd.colt[x], j);
-    }
+  if (i == nn - 1) {
+    o = make_float4(r.kw, r.ku, r.kv, 0.0f);
   } else {
-    const int nn = sd.nx, y = t / nn, i = t - y * nn;
-    const RowTerms r = row_terms(H, sd.rowt[y]);
-    if (i == nn - 1) {
-      o = make_float4(r.kw, r.ku, r.kv, 0.0f);
-    } else {
-      const float inv = __fdiv_rn(1.0f, __fsub_rn(sd.node_x[i + 1], sd.node_x[i]));
-      const CellTerms c = cell_terms(sd, H + 9, i, inv, r);
-      o = make_float4(c.ex, c.cx, c.ey, c.cy);
-    }
+    const float inv = __fdiv_rn(1.0f, __fsub_rn(sd.node_x[i + 1], sd.node_x[i]));
+    const CellTerms c = cell_terms(sd, H + 9, i, inv, r);
+    o = make_float4(c.ex, c.cx, c.ey, c.cy);
   }
   ctab[(int64_t)f * per_frame + t] = o;
+}
+
+// Two floats in a 64-bit register, added in one instruction on sm_103a, each rounded as its scalar sum is. (Not multiplied
+// so: the assembler fuses a packed product with the sum it goes into, rounding modifier or not.)
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) { f32x2 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b)); return d; }
+__device__ __forceinline__ void unpack2(f32x2 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 addx2(f32x2 a, f32x2 b) { f32x2 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+
+// The place of picture sample (x, y) in a frame of 16-bit samples: a column tile's samples together, row by row, a line's
+// two columns side by side, so that a warp of the column pass loads one run of bytes (row by row of the picture they
+// were 16 bytes a line, 279 us a pass over 32 frames of n = 1536 against 210).
+__device__ __forceinline__ int g16_at(int n, int lines, int x, int y) {
+  const int c = x % (2 * lines);
+  return (x - c) * n + y * 2 * lines + (c < lines ? 2 * c : 2 * (c - lines) + 1);
+}
+
+// The decode's read of a strip of 64 columns of a frame's rows, the blend's whole numbers (16 bits a sample,
+// exact) into g16 for the column pass. A warp takes `rows` rows, two at a time, lane l columns l and l + 32 of the
+// strip: a load reads neighbouring pixels of one row of the picture, the homography's lanes are stepped two rows
+// to an instruction (on to the lane's column, then eight steps to the second), and a column's displacement terms are
+// worked out once a mesh row.
+// Bound: instruction issue (77%; 103 instructions a sample) and the luma's latency. Fused into the column pass instead,
+// the samples waited on a third of the warps between the transform's barriers: 32 frames of n = 1536 decoded in 906 us
+// against 883, one of n = 384 in 135 against 123.
+constexpr int kSampleThreads = kHoleThreads, kSampleWarps = kSampleThreads / 32;
+template <class Off>
+__device__ __forceinline__ void sample_strip(const SrcDev &src, int16_t *g16, int f, int strip, int y0, int y1) {
+  const SampleDev &sd = src.sd;
+  const int n = sd.n, lane = threadIdx.x & 31, x = strip * 64 + lane, w2 = src.w - 2, h2 = src.h - 2;
+  const float *reg = src.reg + (int64_t)f * src.regstride;
+  float H[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) H[k] = __ldg(reg + k);
+  const uint8_t *px = src.luma + f * src.fstride;
+  const LinCol lc = lin_col_grid(sd, H, x);
+  const f32x2 cw = pack2(lc.cw, lc.cw), cu = pack2(lc.cu, lc.cu), cv = pack2(lc.cv, lc.cv);
+  const float4 c0 = sd.colt[x], c1 = sd.colt[x + 32];
+  const int lines = plan_of(n).lines, row = 2 * lines;   // a row of a tile
+  int16_t *out = g16 + (int64_t)f * n * n + g16_at(n, lines, x, y0);
+  const int to32 = g16_at(n, lines, x + 32, 0) - g16_at(n, lines, x, 0);
+  float4 T0{}, T1{};
+  int j = -1;
+  for (int y = y0; y < y1;) {
+    const float4 ta = __ldg(sd.rowt + y), tb = __ldg(sd.rowt + min(y + 1, y1 - 1));
+    const RowTerms ra = row_terms(H, ta), rb = row_terms(H, tb);
+    const bool two = y + 1 < y1 && rb.j == ra.j;   // else the row alone (its pair's work goes nowhere)
+    if (ra.j != j) {
+      j = ra.j;
+      T0 = lin_cell(sd, reg + 9, c0, j); T1 = lin_cell(sd, reg + 9, c1, j);
+    }
+    f32x2 W = pack2(__fadd_rn(lc.bw, __fadd_rn(lc.w0, ra.kw)), __fadd_rn(lc.bw, __fadd_rn(lc.w0, rb.kw)));
+    f32x2 U = pack2(__fadd_rn(lc.bu, __fadd_rn(lc.u0, ra.ku)), __fadd_rn(lc.bu, __fadd_rn(lc.u0, rb.ku)));
+    f32x2 V = pack2(__fadd_rn(lc.bv, __fadd_rn(lc.v0, ra.kv)), __fadd_rn(lc.bv, __fadd_rn(lc.v0, rb.kv)));
+#pragma unroll
+    for (int s = 0; s < 7; s++)
+      if (s < lc.g) { W = addx2(W, cw); U = addx2(U, cu); V = addx2(V, cv); }
+    int o[2][2];
+#pragma unroll
+    for (int half = 0; half < 2; half++) {
+      const float4 T = half ? T1 : T0;
+      float wa, wb, ua, ub, va, vb;
+      unpack2(W, wa, wb); unpack2(U, ua, ub); unpack2(V, va, vb);
+      const float rwa = __frcp_rn(wa), rwb = __frcp_rn(wb);
+      const float xa = __fadd_rn(__fadd_rn(T.x, __fmul_rn(T.y, ra.v)), __fmul_rn(ua, rwa));
+      const float xb = __fadd_rn(__fadd_rn(T.x, __fmul_rn(T.y, rb.v)), __fmul_rn(ub, rwb));
+      const float ya = __fadd_rn(__fadd_rn(T.z, __fmul_rn(T.w, ra.v)), __fmul_rn(va, rwa));
+      const float yb = __fadd_rn(__fadd_rn(T.z, __fmul_rn(T.w, rb.v)), __fmul_rn(vb, rwb));
+      o[half][0] = lin_read_whole<Off>(px, w2, h2, src.pitch, lin_hold(xa), lin_hold(ya));
+      o[half][1] = lin_read_whole<Off>(px, w2, h2, src.pitch, lin_hold(xb), lin_hold(yb));
+      if (half == 0) {
+#pragma unroll
+        for (int s = 0; s < 8; s++) { W = addx2(W, cw); U = addx2(U, cu); V = addx2(V, cv); }
+      }
+    }
+    out[0] = (int16_t)o[0][0]; out[to32] = (int16_t)o[1][0];
+    if (two) { out[row] = (int16_t)o[0][1]; out[row + to32] = (int16_t)o[1][1]; }
+    const int step = two ? 2 : 1;
+    y += step; out += step * row;
+  }
+}
+// The sampler's CTAs a frame at `rows` rows a warp.
+__host__ __device__ constexpr int sample_ctas(int n, int rows) { return (n / 64) * ((n + kSampleWarps * rows - 1) / (kSampleWarps * rows)); }
+// Rows a warp: 16 spread a column's set-up over 32 samples; where they would leave SMs idle (two CTAs each), 4, for a
+// shorter chain of rows.
+static int sample_rows(int n, int frames, int sms) { return frames * sample_ctas(n, 16) >= 2 * sms ? 16 : 4; }
+__device__ __forceinline__ void sample_cta(const SrcDev &src, int16_t *g16, int rows, int f, int b) {
+  const int strips = src.sd.n / 64, y0 = (b / strips * kSampleWarps + (threadIdx.x >> 5)) * rows, y1 = min(src.sd.n, y0 + rows);
+  if (y0 >= y1) return;
+  if ((int64_t)src.pitch * src.h <= UINT32_MAX) sample_strip<uint32_t>(src, g16, f, b % strips, y0, y1);
+  else sample_strip<int64_t>(src, g16, f, b % strips, y0, y1);
+}
+__global__ void __launch_bounds__(kSampleThreads, 2) sample16_kernel(SrcDev src, int16_t *g16, int rows) {
+  const int per = sample_ctas(src.sd.n, rows);
+  sample_cta(src, g16, rows, blockIdx.x / per, blockIdx.x % per);
 }
 __global__ void __launch_bounds__(256) cell_table_kernel(SrcDev src, int per_frame, float4 *ctab) {
   cell_table_entry(src, per_frame, ctab, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// One column tile's samples: thread t takes line l = t mod L (columns xa = x0 + l as the real part, xb = x0 + L + l as
-// the imaginary part) at rows y = t / L, t / L + kThreads / L, ...; the anchors' squares erased to the shading
-// surface as they are read. Each row's two samples are summed into the five detrend projections' raw sums, z c(x),
-// z c(y), z c(x) c(y), z q(x), z q(y) (liblizard/src/lizard_phy.c:1584-1591, 1657-1667), in p. SRC: kSrcGrid reads a
-// supplied grid; kSrcExact and kSrcDecode sample the captured frame by the exact walk or the decode's read. The squares'
-// values are in the lines already (erase_tile).
-constexpr int kSrcGrid = 0, kSrcExact = 1, kSrcDecode = 2;
-template <int N, int SRC>
-__device__ __forceinline__ void load_tile(const FftDev &xd, const SrcDev &src, const float4 *ctab, int f, int x0, float2 *line, float p[5]) {
-  constexpr int L = plan_of(N).lines, ystep = kThreads / L;
-  const int l = threadIdx.x % L, xa = x0 + l, xb = x0 + L + l;
-  const bool ina = in_square(xd, xa), inb = in_square(xd, xb);
-  const float cxa = __ldg(xd.cx + xa), qxa = __ldg(xd.qx + xa), cxb = __ldg(xd.cx + xb), qxb = __ldg(xd.qx + xb);
-  float mxa = 0, mxb = 0, h6a = 0, h0a = 0, h3a = 0, h6b = 0, h0b = 0, h3b = 0;
-  int ia = 0, ib = 0, nn = 1;
-  const uint8_t *px = nullptr;
-  const float4 *T = nullptr;   // the frame's row and cell table
-  LinCol lc{};                 // the decode's read: column xa's lanes (xb shares its lane, L / 4 steps on)
-  if (SRC != kSrcGrid) {
-    const float *H = src.reg + (int64_t)f * src.regstride;
-    nn = src.sd.nx;
-    T = ctab + (int64_t)f * N * nn;
-    px = src.luma + f * src.fstride;
-    const float4 ca = src.sd.colt[xa], cb = src.sd.colt[xb];
-    mxa = ca.x; ia = __float_as_int(ca.y);
-    mxb = cb.x; ib = __float_as_int(cb.y);
-    if (SRC == kSrcExact) {
-      h6a = __fmul_rn(H[6], mxa); h0a = __fmul_rn(H[0], mxa); h3a = __fmul_rn(H[3], mxa);
-      h6b = __fmul_rn(H[6], mxb); h0b = __fmul_rn(H[0], mxb); h3b = __fmul_rn(H[3], mxb);
-    } else {
-      lc = lin_col_grid(src.sd, H, xa);   // a tile's 2L columns lie in one strip of 64 (2L divides 64)
-    }
-  }
-#pragma unroll 2   // 2 of 2, 4 and 8 is the fastest on a GB300 (61.1k, 59.3k, 57.7k batch frames/s)
-  for (int y = threadIdx.x / L; y < N; y += ystep) {
-    const bool ysq = (ina || inb) && in_square(xd, y);
-    float va, vb;
-    if (SRC == kSrcGrid) {
-      const float *g = src.grid + f * src.gstride + (int64_t)y * N;
-      va = g[xa]; vb = g[xb];
-    } else if (SRC == kSrcExact) {
-      const float4 *Ty = T + y * nn;
-      const float4 rt = Ty[nn - 1], ta = Ty[ia], tb = ib == ia ? ta : Ty[ib];
-      RowTerms r;
-      r.kw = rt.x; r.ku = rt.y; r.kv = rt.z;
-      const CellTerms ca{ta.x, ta.y, ta.z, ta.w}, cb{tb.x, tb.y, tb.z, tb.w};
-      va = sample_at(px, src.w, src.h, src.pitch, mxa, h6a, h0a, h3a, r, ca);
-      vb = sample_at(px, src.w, src.h, src.pitch, mxb, h6b, h0b, h3b, r, cb);
-    } else {
-      const float4 rt = T[y], rw = __ldg(&src.sd.rowt[y]);
-      const int j = __float_as_int(rw.y);
-      const float4 ta = T[N + j * N + xa], tb = T[N + j * N + xb];
-      LinNum s = lin_start(lc, rt.x, rt.y, rt.z);
-      lin_steps(lc, s, lc.g);
-      va = lin_point(px, src.w, src.h, src.pitch, s, ta, rw.z);
-      lin_steps(lc, s, L / 4);
-      vb = lin_point(px, src.w, src.h, src.pitch, s, tb, rw.z);
-    }
-    if (ysq) {
-      const float2 erased = line[pad(y)];
-      if (ina) va = erased.x;
-      if (inb) vb = erased.y;
-    }
-    const float cy = __ldg(xd.cx + y), qy = __ldg(xd.qx + y);
+// A column tile's samples. Line l holds column xa = x0 + l as its real part and xb = x0 + L + l as its imaginary part; inside
+// the anchors' squares the value is the one erase_tile laid into the line. The five detrend projections' raw sums, z c(x),
+// z c(y), z c(x) c(y), z q(x), z q(y) (liblizard/src/lizard_phy.c:1584-1591, 1657-1667), run over a thread's rows t / L,
+// + kThreads / L, ... of line t mod L in order, whatever the samples come from.
+struct TileSums {
+  float cxa, qxa, cxb, qxb;
+  float p[5] = {0, 0, 0, 0, 0};
+  __device__ __forceinline__ TileSums(const FftDev &xd, int xa, int xb)
+      : cxa(__ldg(xd.cx + xa)), qxa(__ldg(xd.qx + xa)), cxb(__ldg(xd.cx + xb)), qxb(__ldg(xd.qx + xb)) {}
+  __device__ __forceinline__ void add(float cy, float qy, float va, float vb) {
     const float t0 = va + vb, t1 = cxa * va + cxb * vb, t2 = qxa * va + qxb * vb;
     p[0] += t1; p[1] += cy * t0; p[2] += cy * t1; p[3] += t2; p[4] += qy * t0;
-    line[pad(y)] = make_float2(va, vb);
   }
+};
+
+// By the exact walk of the captured frame, into the lines: thread t takes column x0 + t mod 2L at rows t / 2L, +
+// kThreads / 2L, ... (a warp's 8 columns by 4 rows of the largest sizes touch half the cache lines of 4 by 8).
+template <int N>
+__device__ __forceinline__ void load_exact(const FftDev &xd, const SrcDev &src, const float4 *ctab, int f, int x0, float2 *buf) {
+  constexpr int L = plan_of(N).lines, C = 2 * L, G = kThreads / C;
+  const int q = threadIdx.x % C, x = x0 + q;
+  const bool in = in_square(xd, x);
+  float *col = reinterpret_cast<float *>(buf + (q % L) * lstride_of(N)) + q / L;   // the column's row y at col[2 pad(y)]
+  const float *H = src.reg + (int64_t)f * src.regstride;
+  const int nn = src.sd.nx;
+  const float4 *T = ctab + (int64_t)f * N * nn;   // the frame's row and cell table
+  const uint8_t *px = src.luma + f * src.fstride;
+  const float4 cx = src.sd.colt[x];
+  const float mx = cx.x, h6 = __fmul_rn(H[6], mx), h0 = __fmul_rn(H[0], mx), h3 = __fmul_rn(H[3], mx);
+  const int i = __float_as_int(cx.y);
+#pragma unroll 4
+  for (int y = threadIdx.x / C; y < N; y += G) {
+    if (in && __float_as_int(__ldg(xd.rowc + y).x)) continue;   // erased
+    const float4 *Ty = T + y * nn;
+    const float4 rt = Ty[nn - 1], tc = Ty[i];
+    RowTerms rr;
+    rr.kw = rt.x; rr.ku = rt.y; rr.kv = rt.z;
+    col[2 * pad(y)] = sample_at(px, src.w, src.h, src.pitch, mx, h6, h0, h3, rr, CellTerms{tc.x, tc.y, tc.z, tc.w});
+  }
+  __syncthreads();
+}
+
+// The samples with the transform's first pass: from a supplied grid of floats (kSrcGrid), from the decode's read as the
+// sampler left it (kSrcSampled), or from the lines (kSrcExact: load_exact before). Where a first-pass butterfly reads the
+// rows a thread sums over (N / r0 = kThreads / L: n = 384, 768, 1536) the thread transforms what it loads, all of its
+// loads in flight together and nothing passing through shared memory on the way; at the other sizes the rows go to the
+// lines first. Called by every thread; ends with the first pass's outputs in the lines, the CTA synchronised.
+constexpr int kSrcGrid = 0, kSrcExact = 1, kSrcSampled = 2;
+template <int N, int SRC>
+__device__ __forceinline__ void load_first_pass(const FftDev &xd, const SrcDev &src, const int16_t *g16, int f, int x0, float2 *buf,
+                                                const float2 *tw, float p[5]) {
+  constexpr int L = plan_of(N).lines, R = plan_of(N).r0, G = kThreads / L;
+  constexpr bool kFused = N / R == G;
+  const int l = threadIdx.x % L, j = threadIdx.x / L, xa = x0 + l, xb = x0 + L + l;
+  const bool ina = in_square(xd, xa), inb = in_square(xd, xb);
+  float2 *line = buf + l * lstride_of(N);
+  const short2 *gs = reinterpret_cast<const short2 *>(g16 + (int64_t)f * N * N + (int64_t)x0 * N) + l;
+  const float *gf = src.grid + f * src.gstride;
+  TileSums sum(xd, xa, xb);
+  // row y's samples, erased where a square holds them, into the sums
+  auto take = [&](int y, float2 v) {
+    const float4 rc = __ldg(xd.rowc + y);
+    if (SRC != kSrcExact && (ina || inb) && __float_as_int(rc.x)) {
+      const float2 e = line[pad(y)];
+      if (ina) v.x = e.x;
+      if (inb) v.y = e.y;
+    }
+    sum.add(rc.z, rc.w, v.x, v.y);
+    return v;
+  };
+  // B rows y0, y0 + G, ... loaded together (past the last row, the last again)
+  auto load = [&](int y0, float2 *v, auto count) {
+    constexpr int B = decltype(count)::value;
+    if (SRC == kSrcSampled) {
+      short2 w[B];
+#pragma unroll
+      for (int k = 0; k < B; k++) w[k] = __ldg(gs + (kFused ? y0 + k * G : min(y0 + k * G, N - 1)) * L);
+#pragma unroll
+      for (int k = 0; k < B; k++) v[k] = make_float2(lin_sample(w[k].x), lin_sample(w[k].y));
+    } else {
+#pragma unroll
+      for (int k = 0; k < B; k++) {
+        const int y = kFused ? y0 + k * G : min(y0 + k * G, N - 1);
+        if (SRC == kSrcExact) v[k] = line[pad(y)];
+        else v[k] = make_float2(__ldg(gf + (int64_t)y * N + xa), __ldg(gf + (int64_t)y * N + xb));
+      }
+    }
+  };
+  if constexpr (kFused) {
+    float2 v[R];
+    load(j, v, std::integral_constant<int, R>{});
+#pragma unroll
+    for (int r = 0; r < R; r++) v[r] = take(j + r * G, v[r]);
+    dft<R>(v);
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < R; r++) line[pad(j * R + r)] = v[r];
+    __syncthreads();
+  } else {
+    constexpr int B = 8;
+    for (int y0 = j; y0 < N; y0 += B * G) {
+      float2 v[B];
+      load(y0, v, std::integral_constant<int, B>{});
+#pragma unroll
+      for (int k = 0; k < B; k++)
+        if (y0 + k * G < N) line[pad(y0 + k * G)] = take(y0 + k * G, v[k]);
+    }
+    __syncthreads();
+    pass<N, R, 1, L>(buf, tw, L);
+  }
+#pragma unroll
+  for (int q = 0; q < 5; q++) p[q] = sum.p[q];
 }
 
 // The column pass's per-CTA scalars in shared memory.
@@ -534,7 +670,7 @@ __device__ __forceinline__ void erase_tile(const FftDev &xd, int x0, float2 *buf
 // y, and the two real columns of each line separated: A(v) = (Z(v) + conj Z(n - v)) / 2, B(v) = -i (Z(v) - conj
 // Z(n - v)) / 2, written to Y[f][v][x] for the kept rows v. Every thread of the CTA takes part.
 template <int N>
-__device__ __forceinline__ void cols_tile(const FftDev &xd, const SrcDev &src, const float4 *ctab, const double *beta,
+__device__ __forceinline__ void cols_tile(const FftDev &xd, const SrcDev &src, const float4 *ctab, const int16_t *g16, const double *beta,
                                           double *part, float2 *Y, int f, int tile, unsigned char *smraw, ColsShared &s) {
   constexpr int n = N, L = plan_of(N).lines, LSTR = lstride_of(N), tiles = n / (2 * L), ystep = kThreads / L;
   const SmemMap sm = smem_map<N>(smraw);
@@ -544,10 +680,15 @@ __device__ __forceinline__ void cols_tile(const FftDev &xd, const SrcDev &src, c
   if (tid < 6) s.beta[tid] = beta[6 * f + tid];
   __syncthreads();
   erase_tile<N>(xd, x0, sm.buf, s);
-  float p[5] = {0, 0, 0, 0, 0};
-  if (src.grid) load_tile<N, kSrcGrid>(xd, src, ctab, f, x0, line, p);
-  else if (src.sd.read == LIZG_READ_DECODE) load_tile<N, kSrcDecode>(xd, src, ctab, f, x0, line, p);
-  else load_tile<N, kSrcExact>(xd, src, ctab, f, x0, line, p);
+  float p[5];
+  if (src.grid) {
+    load_first_pass<N, kSrcGrid>(xd, src, g16, f, x0, sm.buf, sm.tw, p);
+  } else if (src.sd.read == LIZG_READ_DECODE) {
+    load_first_pass<N, kSrcSampled>(xd, src, g16, f, x0, sm.buf, sm.tw, p);
+  } else {
+    load_exact<N>(xd, src, ctab, f, x0, sm.buf);
+    load_first_pass<N, kSrcExact>(xd, src, g16, f, x0, sm.buf, sm.tw, p);
+  }
 #pragma unroll
   for (int q = 0; q < 5; q++)
     for (int o = 16; o > 0; o >>= 1) p[q] += __shfl_xor_sync(0xffffffffu, p[q], o);
@@ -559,7 +700,7 @@ __device__ __forceinline__ void cols_tile(const FftDev &xd, const SrcDev &src, c
     for (int w = 0; w < kThreads / 32; w++) acc += s.part[w][tid];
     part[((int64_t)f * tiles + tile) * 5 + tid] = acc;
   }
-  fft_lines<N>(sm.buf, sm.tw, L);
+  later_passes<N>(sm.buf, sm.tw, L);
   float2 *Yf = Y + (int64_t)f * xd.vrows * n;
   const int xa = x0 + l, xb = x0 + L + l;
   for (int v = tid / L; v < xd.vrows; v += ystep) {
@@ -571,12 +712,12 @@ __device__ __forceinline__ void cols_tile(const FftDev &xd, const SrcDev &src, c
 
 // The column pass of one picture size: CTA b takes tile b mod tiles of frame b / tiles.
 template <int N>
-__global__ void __launch_bounds__(kThreads, 3) fft_cols_kernel(FftDev xd, SrcDev src, const float4 *ctab, const double *beta, double *part,
+__global__ void __launch_bounds__(kThreads, 3) fft_cols_kernel(FftDev xd, SrcDev src, const float4 *ctab, const int16_t *g16, const double *beta, double *part,
                                                                 float2 *Y) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ ColsShared s;
   constexpr int tiles = N / (2 * plan_of(N).lines);
-  cols_tile<N>(xd, src, ctab, beta, part, Y, blockIdx.x / tiles, blockIdx.x % tiles, smraw, s);
+  cols_tile<N>(xd, src, ctab, g16, beta, part, Y, blockIdx.x / tiles, blockIdx.x % tiles, smraw, s);
 }
 
 // The column pass over several picture sizes in one grid: a queue of (format, frame, tile) items, format k's at CTAs
@@ -590,13 +731,13 @@ __global__ void __launch_bounds__(kThreads, 3) fft_cols_mixed_kernel(const __gri
   const FftColsSeg &g = m.seg[k];
   const int b = (int)blockIdx.x - m.first[k], tiles = g.xd.n / (2 * plan_of(g.xd.n).lines), f = b / tiles, tile = b - f * tiles;
   switch (g.xd.n) {
-    case 384: cols_tile<384>(g.xd, g.src, g.ctab, g.beta, g.part, g.Y, f, tile, smraw, s); break;
-    case 512: cols_tile<512>(g.xd, g.src, g.ctab, g.beta, g.part, g.Y, f, tile, smraw, s); break;
-    case 768: cols_tile<768>(g.xd, g.src, g.ctab, g.beta, g.part, g.Y, f, tile, smraw, s); break;
-    case 1024: cols_tile<1024>(g.xd, g.src, g.ctab, g.beta, g.part, g.Y, f, tile, smraw, s); break;
-    case 1152: cols_tile<1152>(g.xd, g.src, g.ctab, g.beta, g.part, g.Y, f, tile, smraw, s); break;
-    case 1280: cols_tile<1280>(g.xd, g.src, g.ctab, g.beta, g.part, g.Y, f, tile, smraw, s); break;
-    default: cols_tile<1536>(g.xd, g.src, g.ctab, g.beta, g.part, g.Y, f, tile, smraw, s); break;
+    case 384: cols_tile<384>(g.xd, g.src, g.ctab, g.g16, g.beta, g.part, g.Y, f, tile, smraw, s); break;
+    case 512: cols_tile<512>(g.xd, g.src, g.ctab, g.g16, g.beta, g.part, g.Y, f, tile, smraw, s); break;
+    case 768: cols_tile<768>(g.xd, g.src, g.ctab, g.g16, g.beta, g.part, g.Y, f, tile, smraw, s); break;
+    case 1024: cols_tile<1024>(g.xd, g.src, g.ctab, g.g16, g.beta, g.part, g.Y, f, tile, smraw, s); break;
+    case 1152: cols_tile<1152>(g.xd, g.src, g.ctab, g.g16, g.beta, g.part, g.Y, f, tile, smraw, s); break;
+    case 1280: cols_tile<1280>(g.xd, g.src, g.ctab, g.g16, g.beta, g.part, g.Y, f, tile, smraw, s); break;
+    default: cols_tile<1536>(g.xd, g.src, g.ctab, g.g16, g.beta, g.part, g.Y, f, tile, smraw, s); break;
   }
 }
 
@@ -645,6 +786,7 @@ struct FftLightSeg {
   double *hole, *beta, *part;
   int *ticket;
   float4 *ctab;
+  int16_t *g16;
   float2 *fac;
   int bands, per_frame, tblocks, tiles;
 };
@@ -659,7 +801,7 @@ __device__ __forceinline__ int seg_at(const int *first, int nseg, int b) {
   while (k < nseg - 1 && b >= first[k + 1]) k++;
   return k;
 }
-__global__ void __launch_bounds__(kHoleThreads) fft_pre_mixed_kernel(const __grid_constant__ FftLightMix m) {
+__global__ void __launch_bounds__(kHoleThreads, 2) fft_pre_mixed_kernel(const __grid_constant__ FftLightMix m) {
   const int b = blockIdx.x;
   if (b < m.hf[m.nseg]) {
     const int k = seg_at(m.hf, m.nseg, b);
@@ -670,7 +812,8 @@ __global__ void __launch_bounds__(kHoleThreads) fft_pre_mixed_kernel(const __gri
     const int k = seg_at(m.tf, m.nseg, b);
     const FftLightSeg &g = m.seg[k];
     const int lb = b - m.tf[k], f = lb / g.tblocks;
-    cell_table_entry(g.src, g.per_frame, g.ctab, f, (lb - f * g.tblocks) * kHoleThreads + threadIdx.x);
+    if (g.src.sd.read == LIZG_READ_DECODE) sample_cta(g.src, g.g16, 16, f, lb - f * g.tblocks);
+    else cell_table_entry(g.src, g.per_frame, g.ctab, f, (lb - f * g.tblocks) * kHoleThreads + threadIdx.x);
   }
 }
 __global__ void __launch_bounds__(256) fac_mixed_kernel(const __grid_constant__ FftLightMix m) {
@@ -801,6 +944,16 @@ __global__ void __launch_bounds__(kThreads, 3) fft_rows_mixed_kernel(const __gri
   }
 }
 
+// The column pass's row entries: 256 where row y is inside an anchor's square, c(y), q(y).
+__global__ void row_table_kernel(FftDev xd, float4 *rowc) {
+  const int y = blockIdx.x * blockDim.x + threadIdx.x;
+  if (y < xd.n) rowc[y] = make_float4(__int_as_float(in_square(xd, y) ? 256 : 0), 0.0f, xd.cx[y], xd.qx[y]);
+}
+cudaError_t fft_row_table_launch(const FftDev &xd, float4 *rowc, cudaStream_t st) {
+  row_table_kernel<<<(xd.n + 255) / 256, 256, 0, st>>>(xd, rowc);
+  return cudaGetLastError();
+}
+
 int fft_plan(int n, int radix[3], int *lines) {
   const Plan p = plan_of(n);
   if (!p.lines) return -1;
@@ -827,10 +980,14 @@ int fft_y_map(CUtensorMap *map, float2 *Y, int n, int64_t rows) {
 }
 
 // The shading fit's partial sums, then (captured frames only) the sampler's row and cell table.
-cudaError_t fft_pre_launch(const FftSegArgs &a, cudaStream_t st) {
+cudaError_t fft_pre_launch(const FftSegArgs &a, int sms, cudaStream_t st) {
   const int bands = fft_hole_bands(a.xd.n);
   hole_rhs_kernel<<<a.frames * bands, kHoleThreads, 0, st>>>(a.xd, a.src, bands, a.b.hole, a.b.beta, a.b.ticket);
-  if (!a.src.grid) {
+  if (!a.src.grid && a.src.sd.read == LIZG_READ_DECODE) {
+    if (!a.b.g16) return cudaErrorInvalidValue;
+    const int rows = sample_rows(a.xd.n, a.frames, sms);
+    sample16_kernel<<<a.frames * sample_ctas(a.xd.n, rows), kSampleThreads, 0, st>>>(a.src, a.b.g16, rows);
+  } else if (!a.src.grid) {
     if (!a.b.ctab || a.src.sd.nx != a.src.sd.ny) return cudaErrorInvalidValue;
     const int per_frame = a.xd.n * a.src.sd.nx;
     cell_table_kernel<<<dim3((per_frame + 255) / 256, a.frames), 256, 0, st>>>(a.src, per_frame, a.b.ctab);
@@ -853,10 +1010,9 @@ static cudaError_t fft_launch_n(const FftDev &xd, int frames, const SrcDev &src,
   if ((e = opt_cols.set(reinterpret_cast<const void *>(fft_cols_kernel<N>), smem)) != cudaSuccess ||
       (e = opt_rows.set(reinterpret_cast<const void *>(fft_rows_kernel<N>), smem)) != cudaSuccess)
     return e;
-  (void)sms;
   const FftSegArgs a{xd, src, b, frames};
-  if ((e = fft_pre_launch(a, st)) != cudaSuccess) return e;
-  fft_cols_kernel<N><<<frames * tiles, kThreads, smem, st>>>(xd, src, b.ctab, b.beta, b.part, b.Y);
+  if ((e = fft_pre_launch(a, sms, st)) != cudaSuccess) return e;
+  fft_cols_kernel<N><<<frames * tiles, kThreads, smem, st>>>(xd, src, b.ctab, b.g16, b.beta, b.part, b.Y);
   if ((e = fft_fac_launch(a, st)) != cudaSuccess) return e;
   if (!b.ymap || !b.err) return cudaErrorInvalidValue;
   fft_rows_kernel<N><<<frames * ((xd.vrows + L - 1) / L), kThreads, smem, st>>>(xd, b.fac, *b.ymap, b.tpos, b.need, b.C, b.err);
@@ -878,8 +1034,8 @@ static cudaError_t light_mix(const FftSegArgs *a, int count, FftLightMix &m) {
     const FftSegArgs &s = a[k];
     if (!ladder_size(s.xd.n) || s.frames < 1 || s.src.grid || !s.b.ctab || s.src.sd.nx != s.src.sd.ny) return cudaErrorInvalidValue;
     FftLightSeg &g = m.seg[k];
-    g.xd = s.xd; g.src = s.src; g.hole = s.b.hole; g.beta = s.b.beta; g.ticket = s.b.ticket; g.part = s.b.part; g.ctab = s.b.ctab; g.fac = s.b.fac;
-    g.bands = fft_hole_bands(s.xd.n); g.per_frame = s.xd.n * s.src.sd.nx; g.tblocks = (g.per_frame + kHoleThreads - 1) / kHoleThreads;
+    g.xd = s.xd; g.src = s.src; g.hole = s.b.hole; g.beta = s.b.beta; g.ticket = s.b.ticket; g.g16 = s.b.g16; g.part = s.b.part; g.ctab = s.b.ctab; g.fac = s.b.fac;
+    g.bands = fft_hole_bands(s.xd.n); g.per_frame = s.xd.n * s.src.sd.nx; g.tblocks = s.src.sd.read == LIZG_READ_DECODE ? sample_ctas(s.xd.n, 16) : (g.per_frame + kHoleThreads - 1) / kHoleThreads;
     g.tiles = s.xd.n / (2 * plan_of(s.xd.n).lines);
     m.hf[k + 1] = m.hf[k] + s.frames * g.bands;
     m.ff[k + 1] = m.ff[k] + s.frames * kFacCtas;
@@ -915,7 +1071,7 @@ cudaError_t fft_cols_mixed_launch(const FftSegArgs *a, int count, cudaStream_t s
     const FftSegArgs &s = a[k];
     if (!ladder_size(s.xd.n) || s.frames < 1) return cudaErrorInvalidValue;
     FftColsSeg &g = m.seg[k];
-    g.xd = s.xd; g.src = s.src; g.ctab = s.b.ctab; g.beta = s.b.beta; g.part = s.b.part; g.Y = s.b.Y;
+    g.xd = s.xd; g.src = s.src; g.ctab = s.b.ctab; g.g16 = s.b.g16; g.beta = s.b.beta; g.part = s.b.part; g.Y = s.b.Y;
     m.first[k + 1] = m.first[k] + s.frames * (s.xd.n / (2 * plan_of(s.xd.n).lines));
     smem = cmax_i(smem, smem_bytes_of(s.xd.n));
   }

@@ -48,6 +48,7 @@ struct FftDev {
   int n, vrows;                      // picture size; rows v kept (the used coefficients' v <= vrows - 1)
   const float2 *tws;                 // the passes' twiddles: pass s at Ns, [r - 1][k] = e^{-2 pi i r k / (Ns R)}
   const float *cx, *qx;              // detrend basis
+  const float4 *rowc;                // per picture row: 256 inside a square (float bits), 0, c, q
   const float2 *x1, *x2;             // their DFTs
   double sx2, sq2;
   int elo[7], ehi[7];                // anchors' erase ranges
@@ -63,11 +64,9 @@ struct FftBufs {
   const int32_t *tpos;               // vrows x n: the pos index of spectrum point (u mod n, v), -1 where unused
   int need;                          // used coefficients a frame (subch x 320)
   float2 *C;                         // frames x need: the detrended spectrum's used coefficients in pos order
-  // frames x n x nx, filled before the column pass when the samples come straight from captured frames. The exact
-  // walk: for each picture row y of a frame, the mesh displacement line of each cell i < nx - 1 (ex, cx, ey, cy, as
-  // cell_terms gives them) and at i = nx - 1 the homography's row terms (kw, ku, kv, 0). The decode's read: the
-  // homography's row terms of row y at y (n entries), then each column x's displacement terms at mesh row j
-  // (lin_cell) at n + j n + x (j < ny - 1, ny = nx)
+  // frames x n x nx, filled before the column pass when captured frames are read by the exact walk: for each picture
+  // row y of a frame, the mesh displacement line of each cell i < nx - 1 (ex, cx, ey, cy, as cell_terms gives them) and
+  // at i = nx - 1 the homography's row terms (kw, ku, kv, 0)
   float4 *ctab;
   // Y as a 2D tensor (rows frames x vrows, each n complex as 2n floats; boxes of 128 complex by one row) for the row
   // pass's bulk tensor loads, and a device word the passes set when a bounded wait gave up
@@ -75,6 +74,7 @@ struct FftBufs {
   int *err;
   double *beta;                      // frames x 6: the shading surface
   int *ticket;                       // frames: the shading fit's CTAs done, 0 between calls
+  int16_t *g16;                      // frames x n x n: the decode's read, the blend's whole numbers, by column tiles
 };
 // Encodes the tensor map of a Y buffer of `rows` rows of n complex points (the row pass's loads). 0, or a CUresult.
 int fft_y_map(CUtensorMap *map, float2 *Y, int n, int64_t rows);
@@ -160,6 +160,8 @@ struct DemapSeg {
   uint8_t *decl;
 };
 cudaError_t demap_mixed_launch(const DemapSeg *a, int count, cudaStream_t st);
+// The row entries of xd.rowc.
+cudaError_t fft_row_table_launch(const FftDev &xd, float4 *rowc, cudaStream_t st);
 cudaError_t fft_launch(const FftDev &xd, int frames, const SrcDev &src, const FftBufs &b, int sms, cudaStream_t st);
 // One format's share of a transform stage run across formats (the engine's stage-wise run): its tables, source,
 // buffers and frames. fft_pre_launch: the shading fit's sums and the sampler's table; fft_fac_launch: the surface
@@ -171,7 +173,7 @@ struct FftSegArgs {
   FftBufs b;
   int frames;
 };
-cudaError_t fft_pre_launch(const FftSegArgs &a, cudaStream_t st);
+cudaError_t fft_pre_launch(const FftSegArgs &a, int sms, cudaStream_t st);
 cudaError_t fft_fac_launch(const FftSegArgs &a, cudaStream_t st);
 cudaError_t fft_cols_mixed_launch(const FftSegArgs *a, int count, cudaStream_t st);
 // The light stages across formats (captured frames only): the shading sums and the sampler's tables in one launch,

@@ -31,6 +31,7 @@ struct lizg_rx {
   int *counters = nullptr;
   double *hole = nullptr, *beta = nullptr, *part = nullptr;
   int *ticket = nullptr;
+  int16_t *g16 = nullptr;               // the decode's read of a batch's frames
   float2 *fac = nullptr;
   lizg::SampleDev sd{};
   float *node_xy = nullptr;
@@ -166,10 +167,12 @@ lizg_rx *lizg_rx_new(int n, int subch, int span, int max_frames) {
     r->sd.n = n; r->sd.nx = nn; r->sd.ny = nn;
     r->sd.g0 = lizg::kMargin + 0.5f / f.scale; r->sd.step = 1.0f / f.scale;
     r->sd.node_x = r->node_xy; r->sd.node_y = r->node_xy + nn;
-    ok(dev_alloc(r, &r->sample_t, 2 * (size_t)n));
+    ok(dev_alloc(r, &r->sample_t, 3 * (size_t)n));
     if (e == cudaSuccess) {
       r->sd.colt = r->sample_t; r->sd.rowt = r->sample_t + n;
       ok(lizg::sample_tables_launch(r->sd, r->sample_t, r->sample_t + n, nullptr));
+      ok(lizg::fft_row_table_launch(r->xd, r->sample_t + 2 * n, nullptr));
+      r->xd.rowc = r->sample_t + 2 * n;
       ok(cudaDeviceSynchronize());
     }
   }
@@ -177,6 +180,7 @@ lizg_rx *lizg_rx_new(int n, int subch, int span, int max_frames) {
   ok(dev_alloc(r, &r->hole, F * lizg::fft_hole_bands(n) * 6));
   ok(dev_alloc(r, &r->beta, F * 6));
   ok(dev_alloc(r, &r->ticket, F));
+  ok(dev_alloc(r, &r->g16, F * n * n));
   if (e == cudaSuccess) e = cudaMemset(r->ticket, 0, F * sizeof(int));
   ok(dev_alloc(r, &r->fac, F * (2 * (size_t)n + r->xd.vrows)));
   ok(dev_alloc(r, &r->part, F * (size_t)(n / 2) * 5));   // column tiles (at most n / 2) x 5
@@ -382,7 +386,7 @@ int lizg_rx_finish_coef_dev(lizg_rx *r, const float *d_coef, int frames, const l
 static int finish_src(lizg_rx *r, const lizg::SrcDev &src, int frames, const lizg_rx_out *out, float *d_coef, cudaStream_t st, int sms) {
   const int need = r->f.subch * lizg::kSub;
   float2 *C = d_coef ? reinterpret_cast<float2 *>(d_coef) : r->C;   // the caller's spectrum buffer when given
-  const lizg::FftBufs b{r->hole, r->part, r->fac, r->Y, r->tpos, need, C, r->ctab, &r->ymap, r->dev_err, r->beta, r->ticket};
+  const lizg::FftBufs b{r->hole, r->part, r->fac, r->Y, r->tpos, need, C, r->ctab, &r->ymap, r->dev_err, r->beta, r->ticket, r->g16};
   cudaError_t e = lizg::fft_launch(r->xd, frames, src, b, sms, st);
   if (e != cudaSuccess) return lizg::record_error(LIZG_E_CUDA, (std::string("transform: ") + cudaGetErrorString(e)).c_str());
   r->launches += src.grid ? 4 : 5;   // sampling in the column pass adds the sampler's row and cell table
@@ -408,7 +412,7 @@ int lizg_rx_spectrum_grid_dev(lizg_rx *r, const float *d_grid, int frames, float
   lizg::SrcDev src{};
   src.grid = d_grid; src.gstride = (int64_t)r->f.n * r->f.n; src.sd = r->sd;
   const int need = r->f.subch * lizg::kSub;
-  const lizg::FftBufs b{r->hole, r->part, r->fac, r->Y, r->tpos, need, reinterpret_cast<float2 *>(d_coef), r->ctab, &r->ymap, r->dev_err, r->beta, r->ticket};
+  const lizg::FftBufs b{r->hole, r->part, r->fac, r->Y, r->tpos, need, reinterpret_cast<float2 *>(d_coef), r->ctab, &r->ymap, r->dev_err, r->beta, r->ticket, r->g16};
   cudaError_t e = lizg::fft_launch(r->xd, frames, src, b, sms, static_cast<cudaStream_t>(stream));
   r->launches = 4;
   return e == cudaSuccess ? 0 : lizg::record_error(LIZG_E_CUDA, (std::string("lizg_rx_spectrum_grid_dev: ") + cudaGetErrorString(e)).c_str());
@@ -451,7 +455,7 @@ int lizg::rx_spectrum_luma(lizg_rx *r, const uint8_t *d_luma, int w, int h, int 
   src.sd = r->sd;
   src.luma = d_luma; src.w = w; src.h = h; src.pitch = pitch; src.fstride = frame_stride; src.reg = d_reg;
   src.regstride = 9 + 2 * r->sd.nx * r->sd.ny;
-  const lizg::FftBufs b{r->hole, r->part, r->fac, r->Y, r->tpos, r->f.subch * lizg::kSub, reinterpret_cast<float2 *>(d_coef), r->ctab, &r->ymap, r->dev_err, r->beta, r->ticket};
+  const lizg::FftBufs b{r->hole, r->part, r->fac, r->Y, r->tpos, r->f.subch * lizg::kSub, reinterpret_cast<float2 *>(d_coef), r->ctab, &r->ymap, r->dev_err, r->beta, r->ticket, r->g16};
   const cudaError_t e = lizg::fft_launch(r->xd, frames, src, b, sms, st);
   return e == cudaSuccess ? 0 : lizg::record_error(LIZG_E_CUDA, (std::string("spectrum from frames: ") + cudaGetErrorString(e)).c_str());
 }
@@ -470,7 +474,7 @@ int lizg::rx_call(lizg_rx *r, const uint8_t *d_luma, int w, int h, int pitch, in
   src.sd = r->sd;
   src.luma = d_luma; src.w = w; src.h = h; src.pitch = pitch; src.fstride = frame_stride; src.reg = d_reg;
   src.regstride = 9 + 2 * r->sd.nx * r->sd.ny;
-  c.fft.b = FftBufs{r->hole, r->part, r->fac, r->Y, r->tpos, r->f.subch * lizg::kSub, r->C, r->ctab, &r->ymap, r->dev_err, r->beta, r->ticket};
+  c.fft.b = FftBufs{r->hole, r->part, r->fac, r->Y, r->tpos, r->f.subch * lizg::kSub, r->C, r->ctab, &r->ymap, r->dev_err, r->beta, r->ticket, r->g16};
   c.fd = fmt_dev(r, frames);
   c.tiers = r->f.tiers;
   c.out = out;

@@ -181,6 +181,27 @@ __device__ __forceinline__ float lin_read(const uint8_t *px, int w, int h, int p
   const int r = ((((bot - top) >> 1) * fy + (1 << 14)) >> 15) + (top >> 1);
   return __fmul_rn((float)r, 257.0f / 8388608.0f);
 }
+// The blend's whole number (-1 to 32640) from coordinates in [0, 32767] with no conversion instruction: a magic sum
+// truncated (round toward zero) leaves the wanted bits of the coordinate in its mantissa. x: 2^15 + X keeps X's 8
+// fraction bits; y: 2^23 + Y its whole part, then 2^8 + the rest its 15 fraction bits (both exact, as 65536 Y is). w2, h2:
+// w - 2, h - 2. Off: the type a pixel's offset in its frame takes (32 bits where the frame's bytes allow).
+template <class Off>
+__device__ __forceinline__ int lin_read_whole(const uint8_t *px, int w2, int h2, int pitch, float X, float Y) {
+  const int mx = __float_as_int(__fadd_rz(X, 32768.0f));
+  const float yw = __fadd_rz(Y, 8388608.0f);
+  const int fy = __float_as_int(__fadd_rz(__fsub_rn(Y, __fsub_rn(yw, 8388608.0f)), 256.0f)) & 0x7fff;
+  const int xi = min((mx >> 8) & 0x7fff, w2), yi = min(__float_as_int(yw) & 0x7fffff, h2), fx = mx & 0xff;
+  const uint8_t *p = px + ((Off)yi * (Off)pitch + (Off)xi), *pb = p + pitch;
+  const int a = p[0], b = p[1], c = pb[0], d = pb[1];
+  const int gx = 256 - fx, top = a * gx + b * fx, bot = c * gx + d * fx;
+  return ((((bot - top) >> 1) * fy + (1 << 14)) >> 15) + (top >> 1);
+}
+// The sample of that whole number: 257 / 2^23 of it, exact (through the mantissa of 1.5 2^23 + r, the fused product less
+// the bias exact too).
+__device__ __forceinline__ float lin_sample(int r) { return __fmaf_rn(__int_as_float(0x4b400000 + r), 257.0f / 8388608.0f, -385.5f); }
+// A coordinate held in [0, 32767], NaN at 0.
+__device__ __forceinline__ float lin_hold(float v) { return fminf(fmaxf(v, 0.0f), 32767.0f); }
+
 // The point of lanes s (at the column's step) with the column's displacement terms T at the row's place vv.
 __device__ __forceinline__ float lin_point(const uint8_t *px, int w, int h, int pitch, const LinNum &s, float4 T, float vv) {
   const float rw = __fdiv_rn(1.0f, s.w);
