@@ -28,10 +28,9 @@
 namespace lizg {
 
 constexpr int kEncThreads = 256, kCp = 3, kQuiet = 2, kMaxCheckRows = 30;
-constexpr float kQpsk = 0.70710678f;
 
 struct EncTier {
-  const int16_t *perm;
+  const uint32_t *bit;   // per coefficient that carries codeword bits: its two bits' places, 16 bits each (data bits in order, parity bit k + i mb + r at k + 128 r + i)
   const uint8_t *rowptr;
   const uint16_t *circ;
   int nt, k, m, slots, mb;
@@ -39,9 +38,11 @@ struct EncTier {
 
 struct EncDev {
   int n, subch, blocks, used, vrows;
-  const int32_t *tix, *block_tier, *block_slot;
-  const uint8_t *white;
+  const uint32_t *tixw;   // per coefficient, its place in the half-plane << 3 | 1 | its whitening's real bit << 1 | imaginary bit << 2
+  const int32_t *block_tier, *block_slot;
+  const uint32_t *crc;   // x^(8 (476 - 4 j)) mod P for word j of a block, then the all-ones init's term
   EncTier tier[kMaxTiers];
+  int lines;   // the picture's column tiles are 2 lines wide
   int pxm, px, W, q, o, side, aside, a0[kAnchK];   // drive geometry (pixels), the anchors' first pixels
   int copy;   // every tap is the one sample's (the ring's pixels an exact copy of the picture's samples)
   const int32_t *rs_i0;
@@ -54,84 +55,103 @@ struct EncDev {
 
 // ---------------------------------------------------------------- blocks to coefficients
 
-// A block of a frame, one CTA: its bits, its codeword, its slots, its coefficients into the spectrum S.
-__global__ void __launch_bounds__(kEncThreads) enc_blocks_kernel(EncDev e, const uint8_t *blocks, int pilots, float2 *S) {
-  __shared__ uint8_t bits[8192];   // data bits, then parity bits
-  __shared__ uint8_t syn[kMaxCheckRows * LIZG_Z];
-  __shared__ uint32_t crc_tab[256];
-  __shared__ uint32_t s_crc, s_carry[kEncThreads / 32];
-  const int f = blockIdx.x / e.blocks, b = blockIdx.x % e.blocks, tid = threadIdx.x;
+// a * b mod the CRC's polynomial in the reflected representation (bit 31 is x^0).
+__device__ __forceinline__ uint32_t crc_mul(uint32_t a, uint32_t b) {
+  uint32_t p = 0;
+#pragma unroll
+  for (int i = 0; i < 32; i++) {
+    p ^= b & (0u - ((a >> (31 - i)) & 1u));
+    b = (b >> 1) ^ (0x82f63b78u & (0u - (b & 1u)));
+  }
+  return p;
+}
+
+// A block of kFrameGroup frames, one CTA: their bits, their codewords, their slots, their coefficients' signs into the
+// half-plane, a byte a frame of a word a point (the frames of a group share the place, and the scattered stores, a
+// sector each, are what a byte a store is bound by). Everything is words: a column of 128 data bits is four, a check row's
+// data bits the XOR of its circulants' columns rotated (check c = i mb + r holds data bit col z + (i - shift) mod z of row
+// r's circulants), CRC-32C (Castagnoli, reflected 0x82F63B78, liblizard/src/layout.c:44-54) a word a thread times its
+// place, the parity's running XOR over the checks (i, then r) a prefix over the rows and one over the 128 bits of their sum. 3,968 blocks (32 pages of n = 1536): 140 us a bit a byte with
+// the CRC on one thread, 92 in words a frame at a time (the stores), 27 four frames at a time.
+constexpr int kBlockThreads = 128 * kFrameGroup, kBlockWords = 244;
+__global__ void __launch_bounds__(kBlockThreads) enc_blocks_kernel(EncDev e, const uint8_t *blocks, int frames, int pilots, uint32_t *signs) {
+  // frame g's word w at [w][g]: bit t of the codeword at bit t & 31 of word t >> 5, the parity rows of 128 past the data
+  __shared__ __align__(16) uint32_t bits[kBlockWords][kFrameGroup];
+  __shared__ uint32_t syn[kFrameGroup][4 * kMaxCheckRows], before[kFrameGroup][4], s_crc[kFrameGroup][4];
+  const int group = blockIdx.x / e.blocks, b = blockIdx.x % e.blocks, g = threadIdx.x >> 7, tid = threadIdx.x & 127, lane = tid & 31;
+  const int held = min(kFrameGroup, frames - group * kFrameGroup);
+  const bool mine = g < held;
   const EncTier &t = e.tier[e.block_tier[b]];
-  const uint8_t *src = blocks + ((int64_t)f * e.blocks + b) * LIZG_BLOCK_BYTES;
-  // CRC-32C of the block (Castagnoli, reflected 0x82F63B78, liblizard/src/layout.c:44-54), a byte table
-  for (int i = tid; i < 256; i += blockDim.x) {
-    uint32_t c = (uint32_t)i;
-    for (int k = 0; k < 8; k++) c = (c >> 1) ^ (0x82f63b78u & (0u - (c & 1)));
-    crc_tab[i] = c;
+  const uint8_t *src = blocks + ((int64_t)(group * kFrameGroup + g) * e.blocks + b) * LIZG_BLOCK_BYTES;
+  constexpr int kWords = LIZG_BLOCK_BYTES / 4;
+  uint32_t c = 0;
+  if (tid < kWords) {
+    uint32_t w = 0;
+    if (!mine) w = 0;
+    else if ((reinterpret_cast<uintptr_t>(src) & 3) == 0) w = __ldg(reinterpret_cast<const uint32_t *>(src) + tid);
+    else w = src[4 * tid] | src[4 * tid + 1] << 8 | src[4 * tid + 2] << 16 | (uint32_t)src[4 * tid + 3] << 24;
+    bits[tid][g] = __brev(__byte_perm(w, 0u, 0x0123u));   // bytes MSB first
+    c = crc_mul(w, __ldg(e.crc + tid));
   }
+  c = __reduce_xor_sync(0xffffffffu, c);
+  if (lane == 0) s_crc[g][tid >> 5] = c;
+  for (int w = kWords + 1 + tid; w < t.k / 32; w += 128) bits[w][g] = 0;
   __syncthreads();
-  if (tid == 0) {
-    uint32_t c = 0xffffffffu;
-    for (int i = 0; i < LIZG_BLOCK_BYTES; i++) c = (c >> 8) ^ crc_tab[(c ^ src[i]) & 255];
-    s_crc = ~c;
-  }
+  if (tid == 0) bits[kWords][g] = __brev(~(s_crc[g][0] ^ s_crc[g][1] ^ s_crc[g][2] ^ s_crc[g][3] ^ __ldg(e.crc + kWords)));   // MSB first
   __syncthreads();
-  const uint32_t crc = s_crc;
-  for (int i = tid; i < t.k; i += blockDim.x) {   // the block MSB first, its CRC MSB first, zeros past them
-    uint8_t v = 0;
-    if (i < 8 * LIZG_BLOCK_BYTES) v = (src[i >> 3] >> (7 - (i & 7))) & 1;
-    else if (i < 8 * LIZG_BLOCK_BYTES + 32) v = (crc >> (31 - (i - 8 * LIZG_BLOCK_BYTES))) & 1;
-    bits[i] = v;
-  }
-  __syncthreads();
-  // each check's data bits: check c = i mb + r holds data bit col z + (i - shift) mod z of row r's circulants
-  for (int c = tid; c < t.m; c += blockDim.x) {
-    const int i = c / t.mb, r = c - i * t.mb;
+  if (tid < 4 * t.mb) {
+    const int r = tid >> 2, w = tid & 3;
     uint32_t acc = 0;
     for (int k = t.rowptr[r]; k < t.rowptr[r + 1]; k++) {
-      const int col = t.circ[k] >> 8, sh = t.circ[k] & 255;
-      acc ^= bits[col * LIZG_Z + ((i - sh) & (LIZG_Z - 1))];
+      const int cs = t.circ[k], sh = cs & 255, at = w - (sh >> 5), col = 4 * (cs >> 8);
+      acc ^= __funnelshift_l(bits[col + ((at - 1) & 3)][g], bits[col + (at & 3)][g], sh & 31);
     }
-    syn[c] = (uint8_t)acc;
+    syn[g][tid] = acc;
   }
   __syncthreads();
-  // the parity: the running XOR over the checks, a run of checks a thread, the runs' carries scanned
-  const int run = (t.m + kEncThreads - 1) / kEncThreads, c0 = tid * run, c1 = min(t.m, c0 + run);
-  uint32_t mine = 0;
-  for (int c = c0; c < c1; c++) mine ^= syn[c];
-  uint32_t incl = mine;
-  const int lane = tid & 31, warp = tid >> 5;
+  if (tid < 4) {
+    uint32_t q = 0;
+    for (int r = 0; r < t.mb; r++) { q ^= syn[g][4 * r + tid]; syn[g][4 * r + tid] = q; }
+    // over the bits: each word's inclusive prefix, what the words before hold, one bit on
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl ^= up;
+    for (int o = 1; o < 32; o <<= 1) q ^= q << o;
+    uint32_t carry = 0;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const uint32_t up = __shfl_sync(0xfu, q, k) >> 31;
+      if (tid > k) carry ^= up;
+    }
+    q ^= 0u - carry;
+    const uint32_t last = __shfl_up_sync(0xfu, q, 1) >> 31;
+    before[g][tid] = q << 1 | (tid ? last : 0u);
   }
-  if (lane == 31) s_carry[warp] = incl;
   __syncthreads();
-  uint32_t carry = incl ^ mine;   // the XOR of every run before this thread's within its warp
-  for (int w = 0; w < warp; w++) carry ^= s_carry[w];
-  for (int c = c0; c < c1; c++) {
-    carry ^= syn[c];
-    bits[t.k + c] = (uint8_t)carry;
-  }
+  if (tid < 4 * t.mb) bits[t.k / 32 + tid][g] = syn[g][tid] ^ before[g][tid & 3];
   __syncthreads();
-  // the slots and their coefficients: slot i = codeword bit perm[i] (i < nt) or the pilots' count bit, whitened
+  // the coefficients: two codeword bits or the pilots' count bit twice, whitened
   const int first = e.block_slot[b] / 2;
-  const uint32_t qbit = (uint32_t)(pilots >> (b & 1)) & 1;
-  const uint8_t *wh = e.white + 2 * (int64_t)first;
-  float2 *Sf = S + (int64_t)f * e.vrows * e.n;
-  for (int s = tid; s < t.slots / 2; s += blockDim.x) {
-    const int i0 = 2 * s, i1 = 2 * s + 1;
-    const uint32_t b0 = (i0 < t.nt ? bits[t.perm[i0]] : qbit) ^ wh[i0], b1 = (i1 < t.nt ? bits[t.perm[i1]] : qbit) ^ wh[i1];
-    Sf[e.tix[first + s]] = make_float2(b0 ? -kQpsk : kQpsk, b1 ? -kQpsk : kQpsk);
+  const uint32_t present = 0x01010101u >> 8 * (kFrameGroup - held), q = present * (((uint32_t)(pilots >> (b & 1)) & 1) * 6);
+  uint32_t *out = signs + (int64_t)group * e.vrows * e.n;
+#pragma unroll 2
+  for (int s = threadIdx.x; s < t.slots / 2; s += kBlockThreads) {
+    const uint32_t at = __ldg(e.tixw + first + s);
+    uint32_t v = q;
+    if (2 * s < t.nt) {
+      const uint32_t p = __ldg(t.bit + s), p0 = p & 31, p1 = p >> 16 & 31;
+      const uint4 a = *reinterpret_cast<const uint4 *>(bits[(p & 0xffffu) >> 5]), d = *reinterpret_cast<const uint4 *>(bits[p >> 21]);
+      v = (a.x >> p0 & 1) << 1 | (d.x >> p1 & 1) << 2 | (a.y >> p0 & 1) << 9 | (d.y >> p1 & 1) << 10 | (a.z >> p0 & 1) << 17 |
+          (d.z >> p1 & 1) << 18 | (a.w >> p0 & 1) << 25 | (d.w >> p1 & 1) << 26;
+    }
+    out[at >> 3] = (v ^ (at & 7) * 0x01010101u) & present * 7;
   }
 }
 
 // The coefficients past the last block: the whitening alone.
-__global__ void __launch_bounds__(kEncThreads) enc_pad_kernel(EncDev e, int per, float2 *S) {
-  const int f = blockIdx.x / per, s = e.used / 2 + (blockIdx.x % per) * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kEncThreads) enc_pad_kernel(EncDev e, int frames, int per, uint32_t *signs) {
+  const int group = blockIdx.x / per, s = e.used / 2 + (blockIdx.x % per) * blockDim.x + threadIdx.x;
   if (s >= e.subch * kSub) return;
-  S[(int64_t)f * e.vrows * e.n + e.tix[s]] = make_float2(e.white[2 * s] ? -kQpsk : kQpsk, e.white[2 * s + 1] ? -kQpsk : kQpsk);
+  const uint32_t at = e.tixw[s], present = 0x01010101u >> 8 * (kFrameGroup - min(kFrameGroup, frames - group * kFrameGroup));
+  signs[(int64_t)group * e.vrows * e.n + (at >> 3)] = (at & 7) * present;
 }
 
 // ---------------------------------------------------------------- resample and paint
@@ -141,73 +161,134 @@ __global__ void __launch_bounds__(kEncThreads) enc_vert_kernel(EncDev e, const f
   const int f = blockIdx.x / e.q, y = blockIdx.x % e.q;
   const float *wt = e.rs_w + 6 * y;
   const float *pf = pic + (int64_t)f * e.n * e.n;
-  const float *r[6];
+  int r[6];
 #pragma unroll
   for (int t = 0; t < 6; t++) {
     int i = (e.rs_i0[y] + t) % e.n;
     if (i < 0) i += e.n;
-    r[t] = pf + (int64_t)i * e.n;
+    r[t] = i * 2 * e.lines;
   }
   float *out = tmp + ((int64_t)f * e.q + y) * e.n;
-  for (int k = threadIdx.x; k < e.n; k += blockDim.x)
-    out[k] = wt[0] * r[0][k] + wt[1] * r[1][k] + wt[2] * r[2][k] + wt[3] * r[3][k] + wt[4] * r[4][k] + wt[5] * r[5][k];
+  for (int k = threadIdx.x; k < e.n; k += blockDim.x) {
+    const float *col = pf + pic_at(e.n, e.lines, k);
+    out[k] = wt[0] * col[r[0]] + wt[1] * col[r[1]] + wt[2] * col[r[2]] + wt[3] * col[r[3]] + wt[4] * col[r[4]] + wt[5] * col[r[5]];
+  }
 }
 
-// A row of the page: the white margin, the border's cells, the picture resampled across, the anchors over it, each
-// drive value to its grey level as lizard_paint_grey rounds it.
-__global__ void __launch_bounds__(kEncThreads) enc_paint_kernel(EncDev e, const float *tmp, float *drive, uint8_t *grey) {
-  const int f = blockIdx.x / e.W, Y = blockIdx.x % e.W, m = kQuiet * e.pxm;
-  uint8_t *g = grey ? grey + ((int64_t)f * e.W + Y) * e.W : nullptr;
-  const bool in_rows = Y >= m && Y < m + e.px;
-  const int dy = Y - m;
-  int aj = -1;
-  if (in_rows)
-    for (int j = 0; j < kAnchK; j++) if (dy >= e.a0[j] && dy < e.a0[j] + e.aside) aj = j;
-  const float half = 0.5f * (float)e.aside;
-  // the row's terms: the picture rows it reads (the exact copy's one, the resampled intermediate's one) and its cells
-  const bool pic_row = in_rows && dy >= e.o && dy < e.o + e.q;
-  const float *crow = pic_row ? tmp + ((int64_t)f * e.n + e.rs_cp[dy - e.o]) * e.n : nullptr;
-  const float *rrow = pic_row ? tmp + ((int64_t)f * e.q + (dy - e.o)) * e.n : nullptr;
-  const uint8_t *krow = in_rows ? e.kind + (int64_t)(dy / e.pxm) * e.side : nullptr;
-  for (int X = threadIdx.x; X < e.W; X += blockDim.x) {
-    if (!in_rows || X < m || X >= m + e.px) {
-      if (g) g[X] = 255;
-      continue;
+__device__ __forceinline__ float held01(float v) { return v < 0 ? 0.0f : v > 1 ? 1.0f : v; }
+
+// A row of modules of the page, one CTA: the white margin, the border's cells, the picture resampled across, the anchors
+// over it, put together in shared memory and written out in words. Margin, cells, picture and anchors all start and end
+// on whole modules, so what the border shows is worked out once for the pxm rows. PIC_GREY: an exact copy for the grey page,
+// of the picture in grey levels already, read tile by tile (a tile's pxm rows are one run of bytes); PIC_COPY: an exact
+// copy of the picture (both passes' six terms are 0 x, 1 x the sample, 0 x ..., whose sums are the sample itself);
+// PIC_TAPS: the taps across over the intermediate. 32 pages of 1944 x 1944: 290 us a page row a CTA with a pixel's place
+// worked out at the pixel, 373 a thread a column, 155 with the grey levels read a byte a pixel, 74 so (issue, 73%).
+enum { PIC_TAPS, PIC_COPY, PIC_GREY };
+template <int SRC>
+__global__ void __launch_bounds__(kEncThreads) enc_paint_kernel(EncDev e, int pitch, const void *src, float *drive, uint8_t *grey) {
+  extern __shared__ __align__(16) uint8_t page[];   // the rows, `pitch` bytes apart, or where they are alike one of them
+  const int strips = e.W / e.pxm, f = blockIdx.x / strips, cy = blockIdx.x % strips - kQuiet, m = kQuiet * e.pxm;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, dy0 = cy * e.pxm;
+  const bool cells = cy >= 0 && cy < e.side, pic = dy0 >= e.o && dy0 < e.o + e.q;
+  float *dr = drive && cells ? drive + ((int64_t)f * e.px + dy0) * e.px : nullptr;
+  // the margin and the border's cells, beside the picture where the strip has one
+  const int rows = pic ? e.pxm : 1, left = pic ? m + e.o : e.W;
+  for (int i = tid; i < (pic ? e.W - e.q : e.W); i += kEncThreads) {
+    const int X = i < left ? i : i + e.q, dx = X - m;
+    uint8_t level = 255;
+    if (cells && dx >= 0 && dx < e.px) {
+      const float d = (e.kind[cy * e.side + e.cellx[dx]] & 3) == 2 ? 0.0f : 1.0f;
+      level = grey_level(d);
+      if (dr) for (int r = 0; r < e.pxm; r++) dr[(int64_t)r * e.px + dx] = d;
     }
-    const int dx = X - m;
-    int ai = -1;
-    if (aj >= 0)
-      for (int i = 0; i < kAnchK; i++) if (dx >= e.a0[i] && dx < e.a0[i] + e.aside) ai = i;
-    const bool pic = pic_row && dx >= e.o && dx < e.o + e.q;
-    float d;
-    if (ai >= 0) {   // the anchor's pattern: light middle and rim, a dark ring (Chebyshev distance from its middle)
-      const float ddx = fabsf((float)(dx - e.a0[ai]) + 0.5f - half), ddy = fabsf((float)(dy - e.a0[aj]) + 0.5f - half);
-      const float r = fmaxf(ddx, ddy) / half;
-      d = r < 0.25f || r >= 0.6f ? 1.0f : 0.0f;
-    } else if (e.copy && pic) {
-      // an exact copy: both passes' six terms are 0 x, 1 x the sample, 0 x ..., whose sums are the sample itself
-      const float v = crow[e.rs_cp[dx - e.o]];
-      d = v < 0 ? 0.0f : v > 1 ? 1.0f : v;
-    } else if (pic) {   // the picture and its guard interval
-      const int x = dx - e.o;
-      const float *wt = e.rs_w + 6 * x;
-      int c = e.rs_c0[x];
-      float v = wt[0] * rrow[c];
-#pragma unroll
-      for (int t = 1; t < 6; t++) {
-        c = c + 1 == e.n ? 0 : c + 1;
-        v = v + wt[t] * rrow[c];
+    for (int r = 0; r < rows; r++) page[r * pitch + X] = level;
+  }
+  if (pic) {
+    const int y0 = dy0 - e.o;
+    uint8_t *to = page + m + e.o;
+    if (SRC == PIC_GREY) {
+      // two of a tile's bytes a thread, columns l and L + l of row r; the tiles in the order the page shows them
+      const int L = e.lines, C = 2 * L, per = e.pxm * L, groups = max(1, kEncThreads / per), cp0 = e.rs_cp[0], tiles = e.n / C;
+      const int skip = cp0 % C, units = (e.q + skip + C - 1) / C;
+      const uint8_t *lev = static_cast<const uint8_t *>(src) + (int64_t)f * e.n * e.n;
+      for (int i = tid; i < groups * per; i += kEncThreads) {
+        const int g = i / per, r = (i - g * per) / L, l = i - g * per - r * L;
+        const uint8_t *at = lev + e.rs_cp[y0 + r] * C + 2 * l;
+        uint8_t *row = to + r * pitch;
+        int tile = (cp0 / C + g) % tiles, x = g * C - skip + l;
+        const int hop = groups % tiles;
+#pragma unroll 4
+        for (int u = g; u < units; u += groups, x += groups * C) {
+          const uint32_t ab = __ldg(reinterpret_cast<const uint16_t *>(at + tile * C * e.n));
+          if (x >= 0 && x < e.q) row[x] = (uint8_t)ab;
+          if (x + L >= 0 && x + L < e.q) row[x + L] = (uint8_t)(ab >> 8);
+          tile += hop;
+          tile = tile >= tiles ? tile - tiles : tile;
+        }
       }
-      d = v < 0 ? 0.0f : v > 1 ? 1.0f : v;
-    } else {   // the border's cell
-      d = (krow[e.cellx[dx]] & 3) == 2 ? 0.0f : 1.0f;
+    } else {
+      for (int x = tid; x < e.q; x += kEncThreads) {
+        float *d = dr ? dr + e.o + x : nullptr;
+        if (SRC == PIC_COPY) {
+          const float *col = static_cast<const float *>(src) + (int64_t)f * e.n * e.n + pic_at(e.n, e.lines, e.rs_cp[x]);
+#pragma unroll 4
+          for (int r = 0; r < e.pxm; r++) {
+            const float v = held01(__ldg(col + e.rs_cp[y0 + r] * 2 * e.lines));
+            to[r * pitch + x] = grey_level(v);
+            if (d) d[(int64_t)r * e.px] = v;
+          }
+        } else {
+          const float *row = static_cast<const float *>(src) + ((int64_t)f * e.q + y0) * e.n;
+          int c[6];
+          float wt[6];
+          c[0] = e.rs_c0[x];
+#pragma unroll
+          for (int t = 0; t < 6; t++) {
+            wt[t] = e.rs_w[6 * x + t];
+            if (t) c[t] = c[t - 1] + 1 == e.n ? 0 : c[t - 1] + 1;
+          }
+#pragma unroll 2
+          for (int r = 0; r < e.pxm; r++, row += e.n) {
+            float v = wt[0] * __ldg(row + c[0]);
+#pragma unroll
+            for (int t = 1; t < 6; t++) v = v + wt[t] * __ldg(row + c[t]);
+            v = held01(v);
+            to[r * pitch + x] = grey_level(v);
+            if (d) d[(int64_t)r * e.px] = v;
+          }
+        }
+      }
     }
-    if (drive) drive[((int64_t)f * e.px + dy) * e.px + dx] = d;
-    if (g) {
-      const float tt = d * 255.0f + 0.5f;
-      int v = tt >= 2147483647.0f ? 255 : tt <= -2147483648.0f ? 0 : (int)tt;
-      g[X] = (uint8_t)(v < 0 ? 0 : v > 255 ? 255 : v);
+    // the anchors' pattern over it: light middle and rim, a dark ring (Chebyshev distance from its middle)
+    int aj = -1;
+#pragma unroll
+    for (int j = 0; j < kAnchK; j++) if (dy0 >= e.a0[j] && dy0 < e.a0[j] + e.aside) aj = dy0 - e.a0[j];
+    if (aj >= 0) {
+      __syncthreads();
+      const float half = 0.5f * (float)e.aside;
+      for (int i = tid; i < kAnchK * e.aside; i += kEncThreads) {
+        const int k = i / e.aside, ax = i - k * e.aside, dx = e.a0[k] + ax;
+        const float ddx = fabsf((float)ax + 0.5f - half);
+        for (int r = 0; r < e.pxm; r++) {
+          const float rr = fmaxf(ddx, fabsf((float)(aj + r) + 0.5f - half)) / half, d = rr < 0.25f || rr >= 0.6f ? 1.0f : 0.0f;
+          page[r * pitch + m + dx] = grey_level(d);
+          if (dr) dr[(int64_t)r * e.px + dx] = d;
+        }
+      }
     }
+  }
+  if (!grey) return;
+  __syncthreads();
+  for (int r = warp; r < e.pxm; r += kEncThreads / 32) {   // a row a warp: bytes up to a word's edge, words, bytes
+    uint8_t *out = grey + ((int64_t)f * e.W + (cy + kQuiet) * e.pxm + r) * e.W;
+    const uint8_t *row = page + (pic ? r * pitch : 0);
+    const int head = (int)(-reinterpret_cast<uintptr_t>(out) & 3), words = (e.W - head) / 4, tail = e.W - head - 4 * words;
+    const uint32_t *from = reinterpret_cast<const uint32_t *>(row);   // pitch is whole words
+    if (lane < head) out[lane] = row[lane];
+    if (lane < tail) out[head + 4 * words + lane] = row[head + 4 * words + lane];
+    for (int i = lane; i < words; i += 32)
+      reinterpret_cast<uint32_t *>(out + head)[i] = __funnelshift_r(from[i], from[i + 1], 8 * head);
   }
 }
 
@@ -306,7 +387,8 @@ struct lizg_encoder {
   lizg::EncFft xf{};
   int max_frames = 0, fps = 0;
   std::vector<void *> owned;
-  float2 *S = nullptr, *tws = nullptr;
+  float2 *S = nullptr;      // the row transforms, by column tiles
+  uint32_t *signs = nullptr; // the half-plane's signs
   float *pic = nullptr, *tmp = nullptr;
   uint8_t *kind = nullptr;
 };
@@ -361,15 +443,31 @@ lizg_encoder *lizg_encoder_new(int n, int subch, int span, int max_frames) {
   const int a = span / 64;
   e.aside = a * e.pxm;
   for (int i = 0; i < kAnchK; i++) e.a0[i] = (int)std::floor(kMargin + (double)span * (i + 0.5) / kAnchK - a / 2.0 + 0.5) * e.pxm;
-  bool ok = upload(x, &e.tix, f.tix.data(), f.tix.size()) && upload(x, &e.white, f.white.data(), f.white.size()) &&
+  std::vector<uint32_t> tixw(f.tix.size());
+  for (size_t i = 0; i < tixw.size(); i++) tixw[i] = (uint32_t)f.tix[i] << 3 | 1u | (f.white[2 * i] ? 2u : 0u) | (f.white[2 * i + 1] ? 4u : 0u);
+  bool ok = upload(x, &e.tixw, tixw.data(), tixw.size()) &&
             upload(x, &e.block_tier, f.block_tier.data(), f.block_tier.size()) && upload(x, &e.block_slot, f.block_slot.data(), f.block_slot.size());
   for (int t = 0; ok && t < f.tiers; t++) {
     const lizg_code_def_t &d = LIZG_CODES[f.tier[t].code];
     EncTier &et = e.tier[t];
     et.nt = f.tier[t].nt; et.k = f.tier[t].k; et.mb = d.mb; et.m = d.mb * LIZG_Z; et.slots = f.tier[t].slots;
-    ok = upload(x, &et.perm, f.perm[t].data(), f.perm[t].size()) && upload(x, &et.rowptr, d.rowptr, (size_t)d.mb + 1) &&
-         upload(x, &et.circ, d.circ, (size_t)d.rowptr[d.mb]) && et.m <= kMaxCheckRows * LIZG_Z && et.k + et.m <= 8192;
+    std::vector<uint32_t> bit((size_t)et.nt / 2);
+    for (int i = 0; i < et.nt / 2 * 2; i++) {
+      const int v = f.perm[t][i], at = v < et.k ? v : et.k + (v - et.k) % d.mb * LIZG_Z + (v - et.k) / d.mb;
+      bit[i / 2] |= (uint32_t)at << 16 * (i & 1);
+    }
+    ok = upload(x, &et.bit, bit.data(), bit.size()) && upload(x, &et.rowptr, d.rowptr, (size_t)d.mb + 1) &&
+         upload(x, &et.circ, d.circ, (size_t)d.rowptr[d.mb]) && et.m <= kMaxCheckRows * LIZG_Z && et.k + et.m <= 32 * kBlockWords && et.nt % 2 == 0;
   }
+  {
+    // CRC-32C as a sum of word products: x^(8 (476 - 4 j)) mod P, and the all-ones init's x^(8 476) times itself
+    auto step = [](uint32_t r, int bits) { while (bits-- > 0) r = (r >> 1) ^ (0x82f63b78u & (0u - (r & 1u))); return r; };
+    std::vector<uint32_t> crc;
+    for (int j = 0; j < LIZG_BLOCK_BYTES / 4; j++) crc.push_back(step(0x80000000u, 8 * (LIZG_BLOCK_BYTES - 4 * j)));
+    crc.push_back(step(0xffffffffu, 8 * LIZG_BLOCK_BYTES));
+    ok = ok && upload(x, &e.crc, crc.data(), crc.size());
+  }
+  e.lines = lines;
   // the resampler's taps (liblizard/src/lizard_phy.c:980-1000)
   std::vector<int32_t> i0(e.q);
   std::vector<float> w(6 * (size_t)e.q);
@@ -415,6 +513,7 @@ lizg_encoder *lizg_encoder_new(int n, int subch, int span, int max_frames) {
   x->xf.lim = 2.0f * 2.0f * std::sqrt(0.5f * (float)(subch * kSub));   // LIZARD_CLIP 2, twice the half-plane's rms
   x->xf.sc = 0.5f / x->xf.lim;
   ok = ok && alloc(x, reinterpret_cast<void **>(&x->S), sizeof(float2) * (size_t)max_frames * e.vrows * n) &&
+       alloc(x, reinterpret_cast<void **>(&x->signs), sizeof(uint32_t) * (size_t)((max_frames + kFrameGroup - 1) / kFrameGroup) * e.vrows * n) &&
        alloc(x, reinterpret_cast<void **>(&x->pic), sizeof(float) * (size_t)max_frames * n * n) &&
        alloc(x, reinterpret_cast<void **>(&x->tmp), sizeof(float) * (size_t)max_frames * e.q * n) &&
        alloc(x, reinterpret_cast<void **>(&x->kind), (size_t)e.side * e.side);
@@ -460,17 +559,29 @@ int lizg_encode_dev(lizg_encoder *x, const uint8_t *d_blocks, int frames, int pi
     return record_error(LIZG_E_ARG, "lizg_encode_dev: NULL argument, frames outside 1..max_frames or pilots outside 0..3");
   const EncDev &e = x->e;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  cudaError_t err = cudaMemsetAsync(x->S, 0, sizeof(float2) * (size_t)frames * e.vrows * e.n, st);
+  const int groups = (frames + kFrameGroup - 1) / kFrameGroup;
+  cudaError_t err = cudaMemsetAsync(x->signs, 0, sizeof(uint32_t) * (size_t)groups * e.vrows * e.n, st);
   if (err == cudaSuccess) {
-    enc_blocks_kernel<<<frames * e.blocks, kEncThreads, 0, st>>>(e, d_blocks, pilots, x->S);
+    enc_blocks_kernel<<<groups * e.blocks, kBlockThreads, 0, st>>>(e, d_blocks, frames, pilots, x->signs);
     const int pad = e.subch * kSub - e.used / 2, per = (pad + kEncThreads - 1) / kEncThreads;
-    if (per > 0) enc_pad_kernel<<<frames * per, kEncThreads, 0, st>>>(e, per, x->S);
+    if (per > 0) enc_pad_kernel<<<groups * per, kEncThreads, 0, st>>>(e, frames, per, x->signs);
     err = cudaGetLastError();
   }
-  if (err == cudaSuccess) err = enc_fft_launch(x->xf, frames, x->S, x->pic, st);
+  // a copy for the grey page alone has its grey levels taken by the transform, a byte a sample written and read instead of
+  // four: the column pass 154 us against 145, the paint's 302 MB of samples 75
+  const bool bytes = e.copy && !d_drive;
+  if (err == cudaSuccess) err = enc_page_launch(x->xf, frames, x->signs, x->S, x->pic, bytes, st);
   if (err == cudaSuccess) {
-    if (!e.copy) enc_vert_kernel<<<frames * e.q, kEncThreads, 0, st>>>(e, x->pic, x->tmp);
-    enc_paint_kernel<<<frames * e.W, kEncThreads, 0, st>>>(e, e.copy ? x->pic : x->tmp, d_drive, d_grey);   // a copy reads the picture
+    // rows an odd number of words apart, with one to read past the last
+    const int pitch = ((e.W + 4) / 4 | 1) * 4, smem = pitch * e.pxm, grid = frames * (e.W / e.pxm);
+    if (bytes) {
+      enc_paint_kernel<PIC_GREY><<<grid, kEncThreads, smem, st>>>(e, pitch, x->pic, d_drive, d_grey);
+    } else if (e.copy) {
+      enc_paint_kernel<PIC_COPY><<<grid, kEncThreads, smem, st>>>(e, pitch, x->pic, d_drive, d_grey);
+    } else {
+      enc_vert_kernel<<<frames * e.q, kEncThreads, 0, st>>>(e, x->pic, x->tmp);
+      enc_paint_kernel<PIC_TAPS><<<grid, kEncThreads, smem, st>>>(e, pitch, x->tmp, d_drive, d_grey);
+    }
     err = cudaGetLastError();
   }
   return err == cudaSuccess ? 0 : record_error(LIZG_E_CUDA, (std::string("lizg_encode_dev: ") + cudaGetErrorString(err)).c_str());

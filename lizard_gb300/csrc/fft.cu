@@ -413,10 +413,7 @@ __device__ __forceinline__ f32x2 addx2(f32x2 a, f32x2 b) { f32x2 d; asm("add.rn.
 // The place of picture sample (x, y) in a frame of 16-bit samples: a column tile's samples together, row by row, a line's
 // two columns side by side, so that a warp of the column pass loads one run of bytes (row by row of the picture they
 // were 16 bytes a line, 279 us a pass over 32 frames of n = 1536 against 210).
-__device__ __forceinline__ int g16_at(int n, int lines, int x, int y) {
-  const int c = x % (2 * lines);
-  return (x - c) * n + y * 2 * lines + (c < lines ? 2 * c : 2 * (c - lines) + 1);
-}
+__device__ __forceinline__ int g16_at(int n, int lines, int x, int y) { return pic_at(n, lines, x) + y * 2 * lines; }
 
 // The decode's read of a strip of 64 columns of a frame's rows, the blend's whole numbers (16 bits a sample,
 // exact) into g16 for the column pass. A warp takes `rows` rows, two at a time, lane l columns l and l + 32 of the
@@ -1101,28 +1098,48 @@ cudaError_t fft_rows_mixed_launch(const FftSegArgs *a, int count, cudaStream_t s
 }
 
 // ---------------------------------------------------------------- the sender's inverse (liblizard/src/lizard_phy.c:1134-1199)
+//
+// The half-plane spectrum's rows (v < vrows, each along u), then the picture's columns, in one of two forms. Over rows
+// (the refinement's adjoint): the spectrum complex, transformed in place, the picture row-major. PAGE (the sender): the
+// spectrum a byte a point and frame (its two signs), and both results by column tiles, a line's two columns side by side, so that
+// the column pass reads and writes runs of bytes (row by row they are 16 to 32 bytes a cache line, and the pass is bound
+// by the lines it touches: 250 us over 32 pages of n = 1536, 145 so).
 
-// The half-plane spectrum's rows (v < vrows, each along u) inverse-transformed in place: S[v][x] = sum_u S[v][u]
-// e^{+2 pi i u x / n}, as the conjugate of the forward transform of the conjugate. L rows a CTA.
-template <int N>
-__global__ void __launch_bounds__(kThreads, 3) enc_cols_kernel(EncFft e, float2 *S) {
+// The half-plane spectrum's rows inverse-transformed: S[v][x] = sum_u S[v][u] e^{+2 pi i u x / n}, as the conjugate of the
+// forward transform of the conjugate. L rows a CTA.
+template <int N, bool PAGE>
+__global__ void __launch_bounds__(kThreads, 3) enc_cols_kernel(EncFft e, const uint32_t *signs, float2 *S) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  constexpr int L = plan_of(N).lines, LSTR = lstride_of(N);
+  constexpr int L = plan_of(N).lines, LSTR = lstride_of(N), C = 2 * L;
   float2 *buf = reinterpret_cast<float2 *>(smraw), *tw = buf + L * LSTR;
   const int tiles = (e.vrows + L - 1) / L, f = blockIdx.x / tiles, v0 = (blockIdx.x % tiles) * L, Lr = min(L, e.vrows - v0);
   for (int i = threadIdx.x; i < N; i += kThreads) tw[i] = e.tws[i];
-  float2 *rows = S + ((int64_t)f * e.vrows + v0) * N;
-  for (int t = threadIdx.x; t < Lr * N; t += kThreads) {
-    const int l = t / N, p = t - l * N;
-    const float2 z = rows[(int64_t)l * N + p];
-    buf[l * LSTR + pad(p)] = make_float2(z.x, -z.y);
+  if (PAGE) {
+    const uint32_t *rows = signs + ((int64_t)(f / kFrameGroup) * e.vrows + v0) * N;
+    const int at = 8 * (f % kFrameGroup);
+#pragma unroll 4
+    for (int t = threadIdx.x; t < Lr * N; t += kThreads) {
+      const int l = t / N, p = t - l * N;
+      const uint32_t s = __ldg(rows + t) >> at;
+      const float a = s & 1 ? kEncQpsk : 0.0f;
+      buf[l * LSTR + pad(p)] = make_float2(s & 2 ? -a : a, s & 4 ? a : -a);
+    }
+  } else {
+    float2 *rows = S + ((int64_t)f * e.vrows + v0) * N;
+    for (int t = threadIdx.x; t < Lr * N; t += kThreads) {
+      const int l = t / N, p = t - l * N;
+      const float2 z = rows[(int64_t)l * N + p];
+      buf[l * LSTR + pad(p)] = make_float2(z.x, -z.y);
+    }
   }
   __syncthreads();
   fft_lines<N>(buf, tw, Lr);
+  float2 *out = S + (int64_t)f * e.vrows * N;
   for (int t = threadIdx.x; t < Lr * N; t += kThreads) {
-    const int l = t / N, p = t - l * N;
+    const int l = t / N, p = t - l * N, c = p % C;
     const float2 z = buf[l * LSTR + pad(p)];
-    rows[(int64_t)l * N + p] = make_float2(z.x, -z.y);
+    const int at = PAGE ? (p - c) * e.vrows + (v0 + l) * C + (c < L ? 2 * c : 2 * (c - L) + 1) : (v0 + l) * N + p;
+    out[at] = make_float2(z.x, -z.y);
   }
 }
 
@@ -1130,34 +1147,44 @@ __global__ void __launch_bounds__(kThreads, 3) enc_cols_kernel(EncFft e, float2 
 // H the column's Hermitian completion over v (H(0) = 2 Re T(0), H(v) = T(v), H(n - v) = conj T(v) for 0 < v < vrows,
 // zero between), inverse-transformed along v: the real part column xa, the imaginary part column xb
 // (liblizard/src/lizard_phy.c:733-773 turn_pack). Then clipped at +-lim and mapped to 0.5 + v sc (clip_row, :775-782),
-// into pic[y][x].
-template <int N>
-__global__ void __launch_bounds__(kThreads, 3) enc_rows_kernel(EncFft e, const float2 *T, float *pic) {
+// into pic[y][x], or by column tiles (pic_at), then as they
+// are or (GREY) as the page's grey levels.
+template <int N, bool PAGE, bool GREY>
+__global__ void __launch_bounds__(kThreads, 3) enc_rows_kernel(EncFft e, const float2 *T, void *pic) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  constexpr int L = plan_of(N).lines, LSTR = lstride_of(N), tiles = N / (2 * L);
+  constexpr int L = plan_of(N).lines, LSTR = lstride_of(N), C = 2 * L, tiles = N / C;
   float2 *buf = reinterpret_cast<float2 *>(smraw), *tw = buf + L * LSTR;
-  const int f = blockIdx.x / tiles, x0 = (blockIdx.x % tiles) * 2 * L;
+  const int f = blockIdx.x / tiles, x0 = (blockIdx.x % tiles) * C;
   for (int i = threadIdx.x; i < N; i += kThreads) tw[i] = e.tws[i];
   const float2 *Tf = T + (int64_t)f * e.vrows * N;
-  for (int t = threadIdx.x; t < L * N; t += kThreads) {   // l fastest: a row's 2L columns read together
+  const float4 *Tt = reinterpret_cast<const float4 *>(Tf + (int64_t)x0 * e.vrows);   // the tile's (a, b) pairs, row by row
+  // l fastest: a row's 2L columns read together, each row v < vrows once for the rows v and n - v that it fills
+#pragma unroll 4
+  for (int t = threadIdx.x; t < L * e.vrows; t += kThreads) {
     const int v = t / L, l = t - v * L;
-    float2 z = make_float2(0.0f, 0.0f);
-    if (v == 0) {
-      const float2 a = Tf[x0 + l], b = Tf[x0 + L + l];
-      z = make_float2(2.0f * a.x, 2.0f * b.x);
-    } else if (v < e.vrows) {
-      const float2 a = Tf[(int64_t)v * N + x0 + l], b = Tf[(int64_t)v * N + x0 + L + l];
-      z = make_float2(a.x - b.y, a.y + b.x);
-    } else if (v > N - e.vrows) {
-      const int m = N - v;
-      const float2 a = Tf[(int64_t)m * N + x0 + l], b = Tf[(int64_t)m * N + x0 + L + l];
-      z = make_float2(a.x + b.y, b.x - a.y);
+    float2 a, b;
+    if (PAGE) {
+      const float4 ab = __ldg(Tt + t);
+      a = make_float2(ab.x, ab.y); b = make_float2(ab.z, ab.w);
+    } else {
+      a = Tf[(int64_t)v * N + x0 + l]; b = Tf[(int64_t)v * N + x0 + L + l];
     }
-    buf[l * LSTR + pad(v)] = make_float2(z.x, -z.y);
+    float2 *line = buf + l * LSTR;
+    if (v == 0) {
+      line[0] = make_float2(2.0f * a.x, -(2.0f * b.x));
+    } else {
+      line[pad(v)] = make_float2(a.x - b.y, -(a.y + b.x));
+      line[pad(N - v)] = make_float2(a.x + b.y, -(b.x - a.y));
+    }
+  }
+  for (int t = threadIdx.x; t < L * (N - 2 * e.vrows + 1); t += kThreads) {
+    const int v = e.vrows + t / L, l = t % L;
+    buf[l * LSTR + pad(v)] = make_float2(0.0f, -0.0f);
   }
   __syncthreads();
   fft_lines<N>(buf, tw, L);
-  float *pf = pic + (int64_t)f * N * N;
+  float *pf = static_cast<float *>(pic) + (int64_t)f * N * N;
+  uint8_t *gf = static_cast<uint8_t *>(pic) + (int64_t)f * N * N;
   for (int t = threadIdx.x; t < L * N; t += kThreads) {
     const int y = t / L, l = t - y * L;
     const float2 z = buf[l * LSTR + pad(y)];
@@ -1166,35 +1193,52 @@ __global__ void __launch_bounds__(kThreads, 3) enc_rows_kernel(EncFft e, const f
     a = a < -e.lim ? -e.lim : a;
     b = b > e.lim ? e.lim : b;
     b = b < -e.lim ? -e.lim : b;
-    pf[(int64_t)y * N + x0 + l] = __fadd_rn(0.5f, __fmul_rn(a, e.sc));   // rounded as clip_row rounds, unfused
-    pf[(int64_t)y * N + x0 + L + l] = __fadd_rn(0.5f, __fmul_rn(b, e.sc));
+    a = __fadd_rn(0.5f, __fmul_rn(a, e.sc)); b = __fadd_rn(0.5f, __fmul_rn(b, e.sc));   // rounded as clip_row rounds, unfused
+    if (GREY) {   // held to 0..1 and rounded as the page's paint does
+      a = a < 0 ? 0.0f : a > 1 ? 1.0f : a;
+      b = b < 0 ? 0.0f : b > 1 ? 1.0f : b;
+      reinterpret_cast<uchar2 *>(gf + (int64_t)x0 * N)[t] =
+          make_uchar2(grey_level(a), grey_level(b));
+    } else if (PAGE) {
+      reinterpret_cast<float2 *>(pf + (int64_t)x0 * N)[t] = make_float2(a, b);
+    } else {
+      pf[(int64_t)y * N + x0 + l] = a;
+      pf[(int64_t)y * N + x0 + L + l] = b;
+    }
   }
 }
 
-template <int N>
-static cudaError_t enc_fft_launch_n(const EncFft &e, int frames, float2 *S, float *pic, cudaStream_t st) {
+template <int N, bool PAGE, bool GREY>
+static cudaError_t enc_fft_launch_n(const EncFft &e, int frames, const uint32_t *signs, float2 *S, void *pic, cudaStream_t st) {
   constexpr int L = plan_of(N).lines, smem = (L * lstride_of(N) + N) * (int)sizeof(float2);
   static SmemOptIn opt_cols, opt_rows;
   cudaError_t err;
-  if ((err = opt_cols.set(reinterpret_cast<const void *>(enc_cols_kernel<N>), smem)) != cudaSuccess ||
-      (err = opt_rows.set(reinterpret_cast<const void *>(enc_rows_kernel<N>), smem)) != cudaSuccess)
+  if ((err = opt_cols.set(reinterpret_cast<const void *>(enc_cols_kernel<N, PAGE>), smem)) != cudaSuccess ||
+      (err = opt_rows.set(reinterpret_cast<const void *>(enc_rows_kernel<N, PAGE, GREY>), smem)) != cudaSuccess)
     return err;
-  enc_cols_kernel<N><<<frames * ((e.vrows + L - 1) / L), kThreads, smem, st>>>(e, S);
-  enc_rows_kernel<N><<<frames * (N / (2 * L)), kThreads, smem, st>>>(e, S, pic);
+  enc_cols_kernel<N, PAGE><<<frames * ((e.vrows + L - 1) / L), kThreads, smem, st>>>(e, signs, S);
+  enc_rows_kernel<N, PAGE, GREY><<<frames * (N / (2 * L)), kThreads, smem, st>>>(e, S, pic);
   return cudaGetLastError();
 }
-
-cudaError_t enc_fft_launch(const EncFft &e, int frames, float2 *S, float *pic, cudaStream_t st) {
+template <bool PAGE, bool GREY>
+static cudaError_t enc_fft_launch_of(const EncFft &e, int frames, const uint32_t *signs, float2 *S, void *pic, cudaStream_t st) {
+  if (e.vrows < 1 || 2 * e.vrows > e.n + 1) return cudaErrorInvalidValue;
   switch (e.n) {
-    case 384: return enc_fft_launch_n<384>(e, frames, S, pic, st);
-    case 512: return enc_fft_launch_n<512>(e, frames, S, pic, st);
-    case 768: return enc_fft_launch_n<768>(e, frames, S, pic, st);
-    case 1024: return enc_fft_launch_n<1024>(e, frames, S, pic, st);
-    case 1152: return enc_fft_launch_n<1152>(e, frames, S, pic, st);
-    case 1280: return enc_fft_launch_n<1280>(e, frames, S, pic, st);
-    case 1536: return enc_fft_launch_n<1536>(e, frames, S, pic, st);
+    case 384: return enc_fft_launch_n<384, PAGE, GREY>(e, frames, signs, S, pic, st);
+    case 512: return enc_fft_launch_n<512, PAGE, GREY>(e, frames, signs, S, pic, st);
+    case 768: return enc_fft_launch_n<768, PAGE, GREY>(e, frames, signs, S, pic, st);
+    case 1024: return enc_fft_launch_n<1024, PAGE, GREY>(e, frames, signs, S, pic, st);
+    case 1152: return enc_fft_launch_n<1152, PAGE, GREY>(e, frames, signs, S, pic, st);
+    case 1280: return enc_fft_launch_n<1280, PAGE, GREY>(e, frames, signs, S, pic, st);
+    case 1536: return enc_fft_launch_n<1536, PAGE, GREY>(e, frames, signs, S, pic, st);
     default: return cudaErrorInvalidValue;
   }
+}
+cudaError_t enc_fft_launch(const EncFft &e, int frames, float2 *S, float *pic, cudaStream_t st) {
+  return enc_fft_launch_of<false, false>(e, frames, nullptr, S, pic, st);
+}
+cudaError_t enc_page_launch(const EncFft &e, int frames, const uint32_t *signs, float2 *T, void *pic, bool grey, cudaStream_t st) {
+  return grey ? enc_fft_launch_of<true, true>(e, frames, signs, T, pic, st) : enc_fft_launch_of<true, false>(e, frames, signs, T, pic, st);
 }
 
 cudaError_t fft_launch(const FftDev &xd, int frames, const SrcDev &src, const FftBufs &b, int sms, cudaStream_t st) {

@@ -190,6 +190,22 @@ struct EncFft {
   float lim, sc;
 };
 cudaError_t enc_fft_launch(const EncFft &e, int frames, float2 *S, float *pic, cudaStream_t st);
+// The same for the sender: the spectrum as bytes, a frame's in byte f % kFrameGroup of the words of its group of frames
+// (signs, ceil(frames / kFrameGroup) x vrows x n: 0 no coefficient, else 1 | real sign << 1 | imaginary sign << 2, each of
+// magnitude kEncQpsk), T frames x vrows x n of scratch, the picture by column tiles (pic_at), as floats, or with `grey`
+// the samples' grey levels as bytes.
+constexpr float kEncQpsk = 0.70710678f;
+constexpr int kFrameGroup = 4;
+cudaError_t enc_page_launch(const EncFft &e, int frames, const uint32_t *signs, float2 *T, void *pic, bool grey, cudaStream_t st);
+// A held drive value's (0..1) grey level as lizard_paint_grey rounds it.
+#ifdef __CUDACC__
+__device__ __forceinline__ uint8_t grey_level(float d) { return (uint8_t)(int)__fadd_rn(__fmul_rn(d, 255.0f), 0.5f); }
+#endif
+// Column x of a picture by column tiles of 2 `lines` columns: its place in row 0; a row further is 2 lines further.
+__host__ __device__ __forceinline__ int pic_at(int n, int lines, int x) {
+  const int c = x % (2 * lines);
+  return (x - c) * n + (c < lines ? 2 * c : 2 * (c - lines) + 1);
+}
 // The border's cell kinds of a ring of span modules, (span + 30)^2: 2 dark, 1 light, 0 the picture's, | 8 on the format
 // word's cells (encode.cu).
 void layout_kind(int span, int version, int fps, std::vector<uint8_t> &kind);

@@ -70,3 +70,27 @@ def test_encoder_arguments():
         enc.encode(np.zeros((2, enc.blocks, 476), np.uint8))
     with pytest.raises(lz.LizgError):
         enc.set_fps(256)
+
+
+@pytest.mark.parametrize("n,subch,span", FORMATS)
+def test_grey_alone_is_the_drive_pages_grey(n, subch, span):
+    """The grey page painted alone (an exact copy's levels taken in the transform) is byte for byte the one painted with
+    the drive, and what its drive rounds to; from blocks and into pages at any byte."""
+    import ctypes
+    import torch
+    enc = lz.Encoder(n, subch, span, max_frames=3)
+    blocks = np.stack([synth.random_blocks(enc.blocks, 50 + k) for k in range(3)])
+    drive, want = enc.encode(blocks, pilots=1)
+    m = 2 * enc.pxm
+    page = np.floor(drive * np.float32(255) + np.float32(0.5)).astype(np.uint8)
+    assert np.array_equal(want[:, m:m + enc.px, m:m + enc.px], page)
+    for at in (0, 1, 3):
+        src = torch.zeros(blocks.size + 8, dtype=torch.uint8, device="cuda")
+        src[at:at + blocks.size] = torch.from_numpy(blocks.reshape(-1)).cuda()
+        out = torch.zeros(want.size + 8, dtype=torch.uint8, device="cuda")
+        lz._check(lz.lib().lizg_encode_dev(enc._h, ctypes.c_void_p(src.data_ptr() + at), 3, 1, None, ctypes.c_void_p(out.data_ptr() + at), None),
+                  "lizg_encode_dev")
+        torch.cuda.synchronize()
+        got = out.cpu().numpy()
+        assert np.array_equal(got[at:at + want.size].reshape(want.shape), want), at
+        assert not got[:at].any() and not got[at + want.size:].any()
