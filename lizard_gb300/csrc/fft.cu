@@ -154,10 +154,6 @@ __host__ __device__ constexpr Plan plan_of(int n) {
 // 16 / L rows a half-warp stores while loading (and reads while separating) fall on 16 distinct slots.
 __host__ __device__ constexpr int lstride_of(int n) { return (n + n / 16 + 15) / 16 * 16 + 16 / plan_of(n).lines; }
 
-// One Stockham pass of radix R over the CTA's lines (Lr <= L of them) in place, n = N points a line. Butterfly j of
-// a line (j < NR = N / R, k = j mod NS) reads points j + r NR, turns point r by e^{-2 pi i r k / (NS R)}
-// (tw[NS + (r - 1) NS + k]) and writes its DFT's output r to (j / NS) NS R + k + r NS. A thread takes butterflies tid,
-// tid + kThreads, ... (at most B = ceil(L NR / kThreads) of them).
 // The thread's index, read afresh: the passes' offsets hang on it, so a loop round the passes recomputes them pass by
 // pass instead of holding every pass's offsets live across the loop.
 __device__ __forceinline__ int tid_fresh() {
@@ -166,55 +162,116 @@ __device__ __forceinline__ int tid_fresh() {
   return t;
 }
 
-template <int N, int R, int NS, int L>
-__device__ __forceinline__ void pass(float2 *buf, const float2 *tw, int Lr) {
-  constexpr int NR = N / R, LSTR = lstride_of(N), B = (L * NR + kThreads - 1) / kThreads;
+// pad(a + r S) for a butterfly's points r S apart, S a multiple of 8 (or, from a multiple of 16, 16 points 1 apart): a slot
+// worked out once (or once for the even points and once for the odd) and constant steps from it, which the accesses hold
+// as offsets. Worked out point by point, slots were most of the integer instructions the passes were bound by (the ALU pipe
+// 62 to 65% busy, the FMA pipe 26 to 31%): with them and the outer passes straight from and to memory, 32 pages of n = 1536
+// by rows 98 us then 66 and by columns 154 then 127; 24 frames of the refinement's adjoint 74 then 52, 189 then 148.
+template <int S> struct Slots {
+  static_assert(S == 1 || S % 8 == 0, "the slots' steps");
+  int even, odd;
+  __device__ __forceinline__ explicit Slots(int a) : even(pad(a)), odd(S % 16 == 8 ? pad(a + S) : 0) {}
+  __device__ __forceinline__ int operator()(int r) const {
+    return S == 1 ? even + r : S % 16 == 0 ? even + r * (S + S / 16) : (r & 1 ? odd : even) + (r >> 1) * (2 * S + S / 8);
+  }
+};
+
+// One Stockham pass of radix R over the CTA's lines (Lr <= L of them) in place, n = N points a line. Butterfly j of
+// a line (j < NR = N / R, k = j mod NS) reads points j + r NR, turns point r by e^{-2 pi i r k / (NS R)}
+// (tw[NS + (r - 1) NS + k]) and writes its DFT's output r to point (j / NS) NS R + k + r NS. A thread takes butterflies
+// tid, tid + kThreads, ... (at most B = ceil(L NR / kThreads) of them), a line's one after another, or with LFAST the
+// lines' j-th ones together (Lr = L). `in(l, j)` gives a butterfly's points and `out(l, point)` takes its outputs, as
+// callables of r; LinesIn and LinesOut are the lines themselves. An output elsewhere is the last pass's: nothing waits
+// for its reads, and the CTA is not synchronised after it.
+template <int N, int NR> struct LinesIn {
+  const float2 *buf;
+  struct At {
+    const float2 *line;
+    Slots<NR> at;
+    __device__ __forceinline__ float2 operator()(int r) const { return line[at(r)]; }
+  };
+  __device__ __forceinline__ At operator()(int l, int j) const { return At{buf + l * lstride_of(N), Slots<NR>(j)}; }
+};
+template <int N, int NS> struct LinesOut {
+  float2 *buf;
+  struct At {
+    float2 *line;
+    Slots<NS> at;
+    __device__ __forceinline__ void operator()(int r, float2 v) const { line[at(r)] = v; }
+  };
+  __device__ __forceinline__ At operator()(int l, int p) const { return At{buf + l * lstride_of(N), Slots<NS>(p)}; }
+};
+template <int N, int R, int NS, int L, bool LFAST, bool ELSEWHERE, class In, class Out>
+__device__ __forceinline__ void pass_via(const float2 *tw, int Lr, const In &in, const Out &out) {
+  constexpr int NR = N / R, B = (L * NR + kThreads - 1) / kThreads;
+  static_assert(NS != 1 || R == 16, "a first pass's outputs start on a multiple of 16");
   const int total = Lr * NR, tid = tid_fresh();
-  float2 v[B][R];
+  float2 v[ELSEWHERE ? 1 : B][R];
 #pragma unroll
   for (int b = 0; b < B; b++) {
     const int t = tid + b * kThreads;
+    float2 *x = v[ELSEWHERE ? 0 : b];
     if (t < total) {
-      const int l = t / NR, j = t - l * NR, k = j % NS;
-      const float2 *in = buf + l * LSTR;
+      const int l = LFAST ? t % L : t / NR, j = LFAST ? t / L : t - l * NR, k = j % NS;
+      const auto from = in(l, j);
 #pragma unroll
-      for (int r = 0; r < R; r++) v[b][r] = in[pad(j + r * NR)];
+      for (int r = 0; r < R; r++) x[r] = from(r);
       if (NS > 1) {
 #pragma unroll
-        for (int r = 1; r < R; r++) v[b][r] = cmul(v[b][r], tw[NS + (r - 1) * NS + k]);
+        for (int r = 1; r < R; r++) x[r] = cmul(x[r], tw[NS + (r - 1) * NS + k]);
       }
-      dft<R>(v[b]);
+      dft<R>(x);
+      if (ELSEWHERE) {
+        const auto to = out(l, (j / NS) * NS * R + k);
+#pragma unroll
+        for (int r = 0; r < R; r++) to(r, x[r]);
+      }
     }
   }
+  if (ELSEWHERE) return;
   __syncthreads();
 #pragma unroll
   for (int b = 0; b < B; b++) {
     const int t = tid + b * kThreads;
     if (t < total) {
-      const int l = t / NR, j = t - l * NR, jq = j / NS, k = j - jq * NS;
-      float2 *out = buf + l * LSTR;
-      const int base = jq * NS * R + k;
+      const int l = LFAST ? t % L : t / NR, j = LFAST ? t / L : t - l * NR, jq = j / NS, k = j - jq * NS;
+      const auto to = out(l, jq * NS * R + k);
 #pragma unroll
-      for (int r = 0; r < R; r++) out[pad(base + r * NS)] = v[b][r];
+      for (int r = 0; r < R; r++) to(r, v[ELSEWHERE ? 0 : b][r]);
     }
   }
   __syncthreads();
 }
+template <int N, int R, int NS, int L>
+__device__ __forceinline__ void pass(float2 *buf, const float2 *tw, int Lr) {
+  pass_via<N, R, NS, L, false, false>(tw, Lr, LinesIn<N, N / R>{buf}, LinesOut<N, NS>{buf});
+}
 
-// The Lr lines at buf (line l at buf + l lstride_of(N), point p at slot pad(p)) transformed along their N points in
-// place by the size's three passes. tw: the passes' twiddles, pass s's at NS (a multiple of 16 past the first pass,
-// so a half-warp's 16 twiddles are one aligned 128-byte row). Every thread of the CTA takes part.
+// The Lr lines at buf (line l at buf + l lstride_of(N), point p at slot pad(p)) transformed along their N points by the
+// size's three passes. tw: the passes' twiddles, pass s's at NS (a multiple of 16 past the first pass, so a
+// half-warp's 16 twiddles are one aligned 128-byte row). Every thread of the CTA takes part. In place (later_passes);
+// or with the first pass's points from elsewhere (first_pass_from, in(l, j) at points r N / r0 apart from j) and the last
+// pass's outputs elsewhere (last_pass_to, out(l, p) at points r N / r2 apart from p).
+template <int N, bool LFAST = false, class In>
+__device__ __forceinline__ void first_pass_from(float2 *buf, const float2 *tw, int Lr, const In &in) {
+  constexpr Plan P = plan_of(N);
+  pass_via<N, P.r0, 1, P.lines, LFAST, false>(tw, Lr, in, LinesOut<N, 1>{buf});
+}
+template <int N>
+__device__ __forceinline__ void middle_pass(float2 *buf, const float2 *tw, int Lr) {
+  constexpr Plan P = plan_of(N);
+  pass<N, P.r1, P.r0, P.lines>(buf, tw, Lr);
+}
+template <int N, bool LFAST = false, class Out>
+__device__ __forceinline__ void last_pass_to(const float2 *buf, const float2 *tw, int Lr, const Out &out) {
+  constexpr Plan P = plan_of(N);
+  pass_via<N, P.r2, P.r0 * P.r1, P.lines, LFAST, true>(tw, Lr, LinesIn<N, N / P.r2>{buf}, out);
+}
 template <int N>
 __device__ __forceinline__ void later_passes(float2 *buf, const float2 *tw, int Lr) {
   constexpr Plan P = plan_of(N);
-  pass<N, P.r1, P.r0, P.lines>(buf, tw, Lr);
+  middle_pass<N>(buf, tw, Lr);
   pass<N, P.r2, P.r0 * P.r1, P.lines>(buf, tw, Lr);
-}
-template <int N>
-__device__ __forceinline__ void fft_lines(float2 *buf, const float2 *tw, int Lr) {
-  constexpr Plan P = plan_of(N);
-  pass<N, P.r0, 1, P.lines>(buf, tw, Lr);
-  later_passes<N>(buf, tw, Lr);
 }
 
 // A frame's shading-fit sample (x, y) = (8 kx, 8 ky) from a supplied grid or by the exact walk of the captured frame
@@ -594,7 +651,7 @@ __device__ __forceinline__ void load_first_pass(const FftDev &xd, const SrcDev &
     dft<R>(v);
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < R; r++) line[pad(j * R + r)] = v[r];
+    for (int r = 0; r < R; r++) line[pad(j * R) + r] = v[r];   // R = 16
     __syncthreads();
   } else {
     constexpr int B = 8;
@@ -837,11 +894,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int lim
 // coefficients go straight to their place in pos order: C[f][tpos[v][u]] (tpos -1 where (u, v) is not used).
 // The tile's rows come in by the tensor memory accelerator: bulk tensor copies of 128 complex points of a row each,
 // issued by one thread, landing densely at the start of each line's slots (at a 128-byte boundary) and counted on an
-// mbarrier; then every thread moves its points from the dense rows to the padded lines (all read, then all written).
+// mbarrier; the first transform pass reads its points from the dense rows and writes the padded lines (all read, then all
+// written), and the last one's outputs go to their coefficients from registers. 32 frames of n = 1536: 120 us with a copy
+// from dense to padded before the passes and the lines read again after them, 97 so.
 template <int N>
 __device__ __forceinline__ void rows_tile(const FftDev &xd, const float2 *fac, const CUtensorMap *ymap, const int32_t *tpos, int need, float2 *C,
                                           int *err, int f, int rtile, unsigned char *smraw, uint64_t *s_bar) {
-  constexpr int n = N, L = plan_of(N).lines, LSTR = lstride_of(N), SEGS = N / 128, PER = (L * N + kThreads - 1) / kThreads;
+  constexpr int n = N, L = plan_of(N).lines, LSTR = lstride_of(N), SEGS = N / 128;
   static_assert(LSTR >= N + 16, "a line's slots hold its dense row at a 128-byte boundary");
   const SmemMap sm = smem_map<N>(smraw);
   const int tid = threadIdx.x;
@@ -868,47 +927,35 @@ __device__ __forceinline__ void rows_tile(const FftDev &xd, const float2 *fac, c
     mbar_wait(bar, 0, 1 << 22);
     return;
   }
-  // dense rows to padded lines: thread t takes points t, t + kThreads, ... of the tile (line-major), all read first
-  float2 v[PER];
-#pragma unroll
-  for (int k = 0; k < PER; k++) {
-    const int p = tid + k * kThreads, l = p / N, u = p - l * N;
-    if (p < L * N && l < Lr) {
-      float2 t;
-      asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];\n" : "=f"(t.x), "=f"(t.y) : "r"(dense(l) + 8u * u));
-      v[k] = t;
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < PER; k++) {
-    const int p = tid + k * kThreads, l = p / N, u = p - l * N;
-    if (p < L * N && l < Lr) sm.buf[l * LSTR + pad(u)] = v[k];
-  }
-  __syncthreads();
-  fft_lines<N>(sm.buf, sm.tw, Lr);
+  __syncthreads();   // the twiddles
+  first_pass_from<N>(sm.buf, sm.tw, Lr, [&](int l, int j) {
+    const uint32_t row = dense(l) + 8u * j;
+    return [=](int r) {
+      float2 p;
+      asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];\n" : "=f"(p.x), "=f"(p.y) : "r"(row + 8u * (N / plan_of(N).r0) * r));
+      return p;
+    };
+  });
+  middle_pass<N>(sm.buf, sm.tw, Lr);
   float2 *Cf = C + (int64_t)f * need;
   const int32_t *tp = tpos + (int64_t)v0 * n;
   const float2 *fx = fac + (int64_t)f * (2 * n + xd.vrows), *fx0 = fx + n, *fy0 = fx + 2 * n;
-  for (int u = tid; u < n; u += kThreads) {
-    int iv[L];   // the rows' pos indices at this u, loaded ahead of their use
-#pragma unroll
-    for (int l = 0; l < L; l++) iv[l] = l < Lr ? __ldg(tp + l * n + u) : -1;
-    const float2 a = fx[u];
-#pragma unroll
-    for (int l = 0; l < L; l++) {
-      const int i = iv[l];
-      if (i < 0) continue;
-      const int v = v0 + l;
-      float2 o = sm.buf[l * LSTR + pad(u)];
-      const float2 x1v = xd.x1[v];
-      o.x -= a.x * x1v.x - a.y * x1v.y;
-      o.y -= a.x * x1v.y + a.y * x1v.x;
+  last_pass_to<N>(sm.buf, sm.tw, Lr, [&](int l, int p) {
+    const int v = v0 + l;
+    const float2 x1v = xd.x1[v];
+    const int32_t *at = tp + l * n + p;
+    const float2 *a0 = fx + p;
+    return [=](int r, float2 o) {
+      const int u = p + r * (N / plan_of(N).r2), i = __ldg(at + r * (N / plan_of(N).r2));
+      if (i < 0) return;
+      const float2 a = a0[r * (N / plan_of(N).r2)];
+      o.x -= __fmaf_rn(a.x, x1v.x, -__fmul_rn(a.y, x1v.y));   // the contraction named: the compiler's hangs on the code round it
+      o.y -= __fmaf_rn(a.y, x1v.x, __fmul_rn(a.x, x1v.y));
       if (v == 0) { const float2 c = fx0[u]; o.x -= c.x; o.y -= c.y; }
       if (u == 0) { const float2 c = fy0[v]; o.x -= c.x; o.y -= c.y; }
       Cf[i] = o;
-    }
-  }
+    };
+  });
 }
 
 // The row pass of one picture size: CTA b takes row tile b mod tiles of frame b / tiles.
@@ -1114,33 +1161,36 @@ __global__ void __launch_bounds__(kThreads, 3) enc_cols_kernel(EncFft e, const u
   float2 *buf = reinterpret_cast<float2 *>(smraw), *tw = buf + L * LSTR;
   const int tiles = (e.vrows + L - 1) / L, f = blockIdx.x / tiles, v0 = (blockIdx.x % tiles) * L, Lr = min(L, e.vrows - v0);
   for (int i = threadIdx.x; i < N; i += kThreads) tw[i] = e.tws[i];
+  __syncthreads();
+  constexpr int from = N / plan_of(N).r0, to = N / plan_of(N).r2;   // a butterfly's points, its outputs
   if (PAGE) {
     const uint32_t *rows = signs + ((int64_t)(f / kFrameGroup) * e.vrows + v0) * N;
-    const int at = 8 * (f % kFrameGroup);
-#pragma unroll 4
-    for (int t = threadIdx.x; t < Lr * N; t += kThreads) {
-      const int l = t / N, p = t - l * N;
-      const uint32_t s = __ldg(rows + t) >> at;
-      const float a = s & 1 ? kEncQpsk : 0.0f;
-      buf[l * LSTR + pad(p)] = make_float2(s & 2 ? -a : a, s & 4 ? a : -a);
-    }
+    const int shift = 8 * (f % kFrameGroup);
+    first_pass_from<N>(buf, tw, Lr, [&](int l, int j) {
+      const uint32_t *at = rows + l * N + j;
+      return [=](int r) {
+        const uint32_t s = __ldg(at + r * from) >> shift;
+        const float a = s & 1 ? kEncQpsk : 0.0f;
+        return make_float2(s & 2 ? -a : a, s & 4 ? a : -a);
+      };
+    });
   } else {
-    float2 *rows = S + ((int64_t)f * e.vrows + v0) * N;
-    for (int t = threadIdx.x; t < Lr * N; t += kThreads) {
-      const int l = t / N, p = t - l * N;
-      const float2 z = rows[(int64_t)l * N + p];
-      buf[l * LSTR + pad(p)] = make_float2(z.x, -z.y);
-    }
+    const float2 *rows = S + ((int64_t)f * e.vrows + v0) * N;
+    first_pass_from<N>(buf, tw, Lr, [&](int l, int j) {
+      const float2 *at = rows + l * N + j;
+      return [=](int r) { const float2 z = at[r * from]; return make_float2(z.x, -z.y); };
+    });
   }
-  __syncthreads();
-  fft_lines<N>(buf, tw, Lr);
+  middle_pass<N>(buf, tw, Lr);
   float2 *out = S + (int64_t)f * e.vrows * N;
-  for (int t = threadIdx.x; t < Lr * N; t += kThreads) {
-    const int l = t / N, p = t - l * N, c = p % C;
-    const float2 z = buf[l * LSTR + pad(p)];
-    const int at = PAGE ? (p - c) * e.vrows + (v0 + l) * C + (c < L ? 2 * c : 2 * (c - L) + 1) : (v0 + l) * N + p;
-    out[at] = make_float2(z.x, -z.y);
-  }
+  last_pass_to<N>(buf, tw, Lr, [&](int l, int p) {
+    // by column tiles: outputs `to` columns apart are as far into their tiles where that is whole tiles
+    const int c = p % C;
+    float2 *at = PAGE ? out + (p - c) * e.vrows + (v0 + l) * C + (c < L ? 2 * c : 2 * (c - L) + 1) : out + (v0 + l) * N + p;
+    const int step = PAGE ? to * e.vrows : to;
+    return [=](int r, float2 z) { at[r * step] = make_float2(z.x, -z.y); };
+  });
+  static_assert(!PAGE || to % C == 0, "a butterfly's outputs in like places of their tiles");
 }
 
 // The picture's columns: 2L of them a CTA, columns xa = x0 + l and xb = x0 + L + l sharing line l as H_a + i H_b, each
@@ -1182,30 +1232,32 @@ __global__ void __launch_bounds__(kThreads, 3) enc_rows_kernel(EncFft e, const f
     buf[l * LSTR + pad(v)] = make_float2(0.0f, -0.0f);
   }
   __syncthreads();
-  fft_lines<N>(buf, tw, L);
+  pass<N, plan_of(N).r0, 1, L>(buf, tw, L);
+  middle_pass<N>(buf, tw, L);
   float *pf = static_cast<float *>(pic) + (int64_t)f * N * N;
   uint8_t *gf = static_cast<uint8_t *>(pic) + (int64_t)f * N * N;
-  for (int t = threadIdx.x; t < L * N; t += kThreads) {
-    const int y = t / L, l = t - y * L;
-    const float2 z = buf[l * LSTR + pad(y)];
-    float a = z.x, b = -z.y;
-    a = a > e.lim ? e.lim : a;
-    a = a < -e.lim ? -e.lim : a;
-    b = b > e.lim ? e.lim : b;
-    b = b < -e.lim ? -e.lim : b;
-    a = __fadd_rn(0.5f, __fmul_rn(a, e.sc)); b = __fadd_rn(0.5f, __fmul_rn(b, e.sc));   // rounded as clip_row rounds, unfused
-    if (GREY) {   // held to 0..1 and rounded as the page's paint does
-      a = a < 0 ? 0.0f : a > 1 ? 1.0f : a;
-      b = b < 0 ? 0.0f : b > 1 ? 1.0f : b;
-      reinterpret_cast<uchar2 *>(gf + (int64_t)x0 * N)[t] =
-          make_uchar2(grey_level(a), grey_level(b));
-    } else if (PAGE) {
-      reinterpret_cast<float2 *>(pf + (int64_t)x0 * N)[t] = make_float2(a, b);
-    } else {
-      pf[(int64_t)y * N + x0 + l] = a;
-      pf[(int64_t)y * N + x0 + L + l] = b;
-    }
-  }
+  constexpr int to = N / plan_of(N).r2;
+  last_pass_to<N, true>(buf, tw, L, [&](int l, int y) {
+    return [=](int r, float2 z) {
+      float a = z.x, b = -z.y;
+      a = a > e.lim ? e.lim : a;
+      a = a < -e.lim ? -e.lim : a;
+      b = b > e.lim ? e.lim : b;
+      b = b < -e.lim ? -e.lim : b;
+      a = __fadd_rn(0.5f, __fmul_rn(a, e.sc)); b = __fadd_rn(0.5f, __fmul_rn(b, e.sc));   // rounded as clip_row rounds, unfused
+      const int yr = y + r * to;
+      if (GREY) {   // held to 0..1 and rounded as the page's paint does
+        a = a < 0 ? 0.0f : a > 1 ? 1.0f : a;
+        b = b < 0 ? 0.0f : b > 1 ? 1.0f : b;
+        reinterpret_cast<uchar2 *>(gf + (int64_t)x0 * N)[yr * L + l] = make_uchar2(grey_level(a), grey_level(b));
+      } else if (PAGE) {
+        reinterpret_cast<float2 *>(pf + (int64_t)x0 * N)[yr * L + l] = make_float2(a, b);
+      } else {
+        pf[(int64_t)yr * N + x0 + l] = a;
+        pf[(int64_t)yr * N + x0 + L + l] = b;
+      }
+    };
+  });
 }
 
 template <int N, bool PAGE, bool GREY>
