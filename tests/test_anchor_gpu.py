@@ -44,6 +44,30 @@ def test_gpu_batch_matches_oracle(span, n, subch, W, Hh):
     assert same({f: got0[f][0] for f in FIELDS}, want0)
 
 
+@pytest.mark.parametrize("span", [128, 256, 512])
+def test_gpu_matches_oracle_on_pictures_without_anchors(span):
+    """Where the float bounds decide little or nothing: flat pictures (no variance), one grey level of noise, exact ties
+    (a picture that repeats), edges, full-range noise, one anchor-like square among flats, and a map without a finite
+    place. Every output bit for bit, ties and refusals included."""
+    w, h = 700, 660
+    side = span + 30
+    y, x = np.mgrid[:h, :w]
+    rng = np.random.default_rng(span)
+    cell = (x // 3 + y // 3) % 2
+    square = np.maximum(np.abs(x - 350), np.abs(y - 330))
+    pictures = [np.full((h, w), 255), np.zeros((h, w)), 128 + rng.integers(0, 2, (h, w)), 255 * cell, 255 * (x // 16 % 2), 255 * (x > 350) + 0 * y,
+                rng.integers(0, 256, (h, w)), np.where(square < 2, 255, np.where(square < 5, 0, 255)), 254 + (x + y) % 2, (x + y) % 256]
+    luma = np.stack(pictures).astype(np.uint8)
+    s = 640.0 / side
+    H = np.tile(np.array([s, 0.01, 12.0, -0.013, s, 9.0, 1e-6, -1e-6, 1], np.float32), (len(luma) + 1, 1))
+    luma = np.concatenate([luma, luma[6:7]])
+    H[-1, 6:8] = -1.0 / 40, 0   # the line at infinity crosses the anchors
+    got = lz.anchor_find(span, luma, H)
+    for k in range(len(luma)):
+        want = oracle.anchor_find(oracle.port(), "orc_anchor_find", span, luma[k], H[k], None)
+        assert same({f: got[f][k] for f in FIELDS}, want), "picture %d" % k
+
+
 def test_skip_leaves_outputs():
     span, luma, H, lens, skip, want = next(iter(golden_cases()))
     skip = np.ones(49, np.uint8)
