@@ -103,14 +103,13 @@ __device__ __forceinline__ int cell_of(const float *pos, int nn, float m) {
   while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (m >= pos[mid]) lo = mid; else hi = mid - 1; }
   return lo;
 }
-// The warp at (mx, my) in node cell (i, j) at place (uu, vv).
-__device__ __forceinline__ WarpAt warp_in(const FieldArgs &a, const float *reg, float mx, float my, int i, int j, float uu, float vv) {
+// The warp at (mx, my) in node cell (i, j) at place (uu, vv), the cell's displacements n00 .. n11 (right, then below).
+__device__ __forceinline__ WarpAt warp_cell(const float *h, float mx, float my, int i, int j, float uu, float vv, float2 n00, float2 n10,
+                                            float2 n01, float2 n11) {
   WarpAt o;
   o.i = i; o.j = j; o.uu = uu; o.vv = vv;
-  const float *n00 = reg + 9 + 2 * (o.j * a.nn + o.i), *n10 = n00 + 2, *n01 = n00 + 2 * a.nn, *n11 = n01 + 2;
-  const float mdx = (n00[0] * (1 - o.uu) + n10[0] * o.uu) * (1 - o.vv) + (n01[0] * (1 - o.uu) + n11[0] * o.uu) * o.vv;
-  const float mdy = (n00[1] * (1 - o.uu) + n10[1] * o.uu) * (1 - o.vv) + (n01[1] * (1 - o.uu) + n11[1] * o.uu) * o.vv;
-  const float *h = reg;
+  const float mdx = (n00.x * (1 - o.uu) + n10.x * o.uu) * (1 - o.vv) + (n01.x * (1 - o.uu) + n11.x * o.uu) * o.vv;
+  const float mdy = (n00.y * (1 - o.uu) + n10.y * o.uu) * (1 - o.vv) + (n01.y * (1 - o.uu) + n11.y * o.uu) * o.vv;
   o.wd = h[6] * mx + h[7] * my + 1;
   o.iw = 1.0f / o.wd;
   o.U = (h[0] * mx + h[1] * my + h[2]) * o.iw;
@@ -118,6 +117,11 @@ __device__ __forceinline__ WarpAt warp_in(const FieldArgs &a, const float *reg, 
   o.u = o.U + mdx;
   o.v = o.V + mdy;
   return o;
+}
+__device__ __forceinline__ WarpAt warp_in(const FieldArgs &a, const float *reg, float mx, float my, int i, int j, float uu, float vv) {
+  const float *n00 = reg + 9 + 2 * (j * a.nn + i), *n01 = n00 + 2 * a.nn;
+  return warp_cell(reg, mx, my, i, j, uu, vv, make_float2(n00[0], n00[1]), make_float2(n00[2], n00[3]), make_float2(n01[0], n01[1]),
+                   make_float2(n01[2], n01[3]));
 }
 // pos, inv: the node positions (a.pos) and each cell's 1 / width, in the caller's CTA's shared memory (lanes search
 // them at different places, which a kernel parameter would serve one address at a time).
@@ -272,6 +276,12 @@ __global__ void __launch_bounds__(kFThreads) field_pilot_kernel(FieldArgs a, con
 // blend (1 - uu) W_i[k] + uu W_{i+1}[k] of its cell's two nodes, so the lane sums g Iu, g Iv and the squares' terms
 // against (1 - uu), uu and their products over the samples of one cell (10 sums), and adds them into its knot sums (in
 // shared memory, a slot a lane) each time its run leaves a cell.
+//
+// A lane's run puts its neighbours' columns n / 32 apart, so a load a column of a row of floats touches 32 lines: the
+// gradients come in fours (rows and runs are whole 16 bytes), the detrend basis and the row's two rows of nodes from
+// shared memory (the basis a run an odd number of slots apart). Bound: issue (66%, 286 instructions a sample's warp). 24
+// frames of n = 1536: 760 us with the loads a column (L1 70% busy), 633 so. Parking a left cell's sums until the run's
+// end: 629, not kept.
 constexpr int kCellSums = 10;
 __global__ void __launch_bounds__(kFThreads, 2) field_grad_kernel(FieldArgs a, const float *regs, const float *G, const PilotTerms *pt,
                                                                const uint8_t *skip, float *part) {
@@ -286,9 +296,14 @@ __global__ void __launch_bounds__(kFThreads, 2) field_grad_kernel(FieldArgs a, c
   __shared__ float s_kn[kFRows][kFK * 4][32];   // each lane's knot sums: g tx, g ty, tx^2, ty^2 at each knot a
   __shared__ float s_pq[kFRows][kFK][4];        // a row's field sums over its lanes
   __shared__ float s_wy[kFRows][kFK];
+  __shared__ float2 s_node[kFRows][2][40];
   __shared__ float s_h[kFThreads / 32][kFHs];
   float (*kn)[32] = s_kn[warp];
   for (int e = 0; e < kFK * 4; e++) kn[e][lane] = 0;
+  const int per = n / 32, x0 = lane * per;
+  extern __shared__ __align__(16) unsigned char gsm[];
+  float2 *s_basis = reinterpret_cast<float2 *>(gsm);   // c(x), q(x) at x + x / per
+  for (int x = threadIdx.x; x < n; x += kFThreads) s_basis[x + x / per] = make_float2(a.cx[x], a.qx[x]);
   // the detrend's adjoint constants in float: the gradient's share of them needs no more (FP64 is a narrow pipe here)
   const float K0 = (float)pt[f].k[0], K1 = (float)pt[f].k[1], K2 = (float)pt[f].k[2], K3 = (float)pt[f].k[3], K4 = (float)pt[f].k[4];
   const float my = a.g0 + (float)y * a.step;
@@ -303,7 +318,18 @@ __global__ void __launch_bounds__(kFThreads, 2) field_grad_kernel(FieldArgs a, c
   for (int q = 0; q < kCellSums; q++) cs[q] = 0;
   const int jrow = cell_of(fs.pos, a.nn, my);
   const float vrow = (my - fs.pos[jrow]) * fs.inv[jrow];
-  const int per = n / 32, x0 = lane * per;
+  float2 (*node)[40] = s_node[warp];
+  for (int t = lane; t < 2 * a.nn; t += 32) {
+    const int below = t >= a.nn, i = t - below * a.nn;
+    const float *p = reg + 9 + 2 * ((jrow + below) * a.nn + i);
+    node[below][i] = make_float2(p[0], p[1]);
+  }
+  __syncthreads();
+  const float2 *basis = s_basis + lane * (per + 1);
+  float hreg[9];
+#pragma unroll
+  for (int q = 0; q < 9; q++) hreg[q] = reg[q];
+  float4 G4 = make_float4(0, 0, 0, 0);
   int icell = cell_of(fs.pos, a.nn, a.g0 + (float)x0 * a.step), ccell = icell;
   // the cell sums of cell ic into the lane's knot sums
   auto flush = [&](int ic) {
@@ -320,17 +346,20 @@ __global__ void __launch_bounds__(kFThreads, 2) field_grad_kernel(FieldArgs a, c
     for (int q = 0; q < kCellSums; q++) cs[q] = 0;
   };
   for (int x = x0; x < x0 + per; x++) {
+    if ((x & 3) == 0) G4 = *reinterpret_cast<const float4 *>(Gf + x);   // runs are whole fours
+    const float Gx = G4.x;
+    G4.x = G4.y; G4.y = G4.z; G4.z = G4.w;
     const float mx = a.g0 + (float)x * a.step;
     while (icell < a.nn - 2 && mx >= fs.pos[icell + 1]) icell++;
     if (icell != ccell) { flush(ccell); ccell = icell; }
     const float uu = (mx - fs.pos[icell]) * fs.inv[icell];
-    const WarpAt o = warp_in(a, reg, mx, my, icell, jrow, uu, vrow);
+    const WarpAt o = warp_cell(hreg, mx, my, icell, jrow, uu, vrow, node[0][icell], node[0][icell + 1], node[1][icell], node[1][icell + 1]);
     float Iu, Iv;
     const float z = read_grad(px, a.w, a.h, o.u, o.v, &Iu, &Iv);
     zs += z; zz += z * z;
     if (ysq && in_sq(a, x)) continue;   // erased: the shading surface, held constant
-    const float cxx = a.cx[x], qxx = a.qx[x];
-    const float g = Gf[x] - 0.5f - (K0 * cxx * cy + K1 * cxx + K2 * qxx + K3 * cy + K4 * qy);
+    const float cxx = basis[x - x0].x, qxx = basis[x - x0].y;
+    const float g = Gx - 0.5f - (K0 * cxx * cy + K1 * cxx + K2 * qxx + K3 * cy + K4 * qy);
     const float ta = o.iw * Iu, tb = o.iw * Iv, tc = -o.iw * (Iu * o.U + Iv * o.V), m2 = mx * mx;
     const float gta = g * ta, gtb = g * tb, gtc = g * tc;
     ga[0] += gta; ga[1] += gta * mx; ga[2] += gtb; ga[3] += gtb * mx; ga[4] += gtc; ga[5] += gtc * mx;
@@ -953,7 +982,10 @@ int field_eval(lizg_field *g, const lizg::FieldArgs &a, const float *base, int f
   field_pilot_kernel<<<fc, kFThreads, 0, st>>>(a, g->coef, g->skip, g->R, g->pt);
   if (adjoint) {
     if (enc_fft_launch(g->enc, fc, g->R, g->G, st) != cudaSuccess) return record_error(LIZG_E_CUDA, "lizg_field: adjoint transform launch");
-    field_grad_kernel<<<fc * (a.n / kFRows), kFThreads, 0, st>>>(a, g->eff, g->G, g->pt, g->skip, g->part);
+    static SmemOptIn opt;
+    const int basis = (int)sizeof(float2) * (a.n + 32);
+    if (opt.set(reinterpret_cast<const void *>(field_grad_kernel), 16 * 1024) != cudaSuccess) return record_error(LIZG_E_CUDA, "lizg_field: adjoint pass");
+    field_grad_kernel<<<fc * (a.n / kFRows), kFThreads, basis, st>>>(a, g->eff, g->G, g->pt, g->skip, g->part);
   }
   const float *au = anchors ? anchors->u + (int64_t)f0 * 49 : nullptr, *av = anchors ? anchors->v + (int64_t)f0 * 49 : nullptr;
   const uint8_t *ao = anchors ? anchors->ok + (int64_t)f0 * 49 : nullptr;
