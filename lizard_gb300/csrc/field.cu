@@ -456,6 +456,31 @@ __device__ __forceinline__ void point_row(const FieldShared &fs, const WarpAt &o
   }
 }
 
+// The adjoint pass's partial sums over a frame's blocks, in block order within each of 8 interleaved sums (a warp each, a
+// lane a sum), the 8 then added pairwise (blocks is a multiple of 8 for every picture size; any rest is summed after).
+// The solve (a CTA a frame) is bound by its SM's double pipe: 322 us for 24 frames with these sums in it and L's entries
+// worked out by every thread that uses them, 270 without, and 11 here.
+constexpr int kSumCols = 32;
+__global__ void __launch_bounds__(8 * kSumCols) field_sum_kernel(int blocks, const float *part, const uint8_t *skip, double *sum) {
+  constexpr int tiles = (kFPart + kSumCols - 1) / kSumCols;
+  const int f = blockIdx.x / tiles, lane = threadIdx.x % kSumCols, u = threadIdx.x / kSumCols, q = blockIdx.x % tiles * kSumCols + lane;
+  if (skip && skip[f]) return;
+  __shared__ double s_acc[8][kSumCols];
+  const float *p = part + (int64_t)f * blocks * kFPart + q;
+  double acc = 0;
+  const int whole = blocks / 8 * 8;
+  if (q < kFPart)
+#pragma unroll 8
+    for (int b = u; b < whole; b += 8) acc += p[(int64_t)b * kFPart];
+  s_acc[u][lane] = acc;
+  __syncthreads();
+  if (u != 0 || q >= kFPart) return;
+  double tail = 0;
+  for (int b = whole; b < blocks; b++) tail += p[(int64_t)b * kFPart];
+  sum[(int64_t)f * kFPart + q] = ((s_acc[0][lane] + s_acc[1][lane]) + (s_acc[2][lane] + s_acc[3][lane])) +
+                                 ((s_acc[4][lane] + s_acc[5][lane]) + (s_acc[6][lane] + s_acc[7][lane])) + tail;
+}
+
 // The normal equations of the three terms at the evaluation in hand, the loss, and the step (kept or halved). A CTA a
 // frame; A (kFP x kFP doubles) in dynamic shared memory, then the staged rows. The track's and the anchors' residual
 // rows are staged kRowBatch at a time as dense rows (a thread a row); each thread then sums a 4 x 4 tile of the upper
@@ -466,17 +491,17 @@ constexpr int kRowBatch = 128;
 constexpr int kFTiles = kFPad / 4, kFTileCount = kFTiles * (kFTiles + 1) / 2;
 constexpr size_t kSolveSmem = sizeof(double) * kFP * kFP + sizeof(float) * kRowBatch * kFPad;
 static_assert((sizeof(double) * kFP * kFP) % 16 == 0, "the staged rows start on a 16-byte boundary");
-__global__ void __launch_bounds__(256, 1) field_solve_kernel(FieldArgs a, const float *regs, const float *part, const PilotTerms *pt,
+__global__ void __launch_bounds__(256, 1) field_solve_kernel(FieldArgs a, const float *regs, const double *sum, const PilotTerms *pt,
                                                           const float *anc_u, const float *anc_v, const uint8_t *anc_ok,
                                                           const uint8_t *skip, FieldState *st, int last, double *terms) {
   extern __shared__ __align__(16) double smA[];
   float *Jd = reinterpret_cast<float *>(smA + kFP * kFP);   // kRowBatch x kFPad
   __shared__ double bv[3][kFP], red[8], s_sum[kFPart], s_lvl[2], s_loss[3], s_cnt[3];
-  __shared__ double x[kFP], sc[kFP], isc[kFP], s_inv[kFP];
+  __shared__ double x[kFP], sc[kFP], isc[kFP], s_inv[kFP], lcol[2][kFP];
   __shared__ float r_w[kRowBatch], r_r[kRowBatch];
   __shared__ int r_term[kRowBatch];
   __shared__ FieldShared fs;
-  const int f = blockIdx.x, tid = threadIdx.x, blocks = a.n / kFRows;
+  const int f = blockIdx.x, tid = threadIdx.x;
   if (skip && skip[f]) return;
   stage_shared(a, fs);
   const float *reg = regs + (int64_t)f * a.reg_stride;
@@ -484,20 +509,7 @@ __global__ void __launch_bounds__(256, 1) field_solve_kernel(FieldArgs a, const 
   FieldState &S = st[f];
   // the last evaluation of a refinement only weighs its point against the best so far: no gradient, no system
   const bool only_loss = last && !terms;
-  // the adjoint pass's partial sums, in block order within each of 8 interleaved sums (8 loads in flight a thread),
-  // the 8 then added pairwise (blocks is a multiple of 8 for every picture size; any rest is summed after)
-  for (int q = tid; q < (only_loss ? 0 : kFPart); q += blockDim.x) {
-    const float *p = part + (int64_t)f * blocks * kFPart + q;
-    double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    int b = 0;
-    for (; b + 8 <= blocks; b += 8) {
-#pragma unroll
-      for (int u = 0; u < 8; u++) acc[u] += p[(int64_t)(b + u) * kFPart];
-    }
-    double tail = 0;
-    for (; b < blocks; b++) tail += p[(int64_t)b * kFPart];
-    s_sum[q] = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7])) + tail;
-  }
+  for (int q = tid; q < (only_loss ? 0 : kFPart); q += blockDim.x) s_sum[q] = sum[(int64_t)f * kFPart + q];   // field_sum_kernel
   for (int q = tid; q < (only_loss ? 0 : 3 * kFP); q += blockDim.x) bv[q / kFP][q % kFP] = 0;
   for (int q = tid; q < (only_loss ? 0 : kFP * kFP); q += blockDim.x) smA[q] = 0;
   __syncthreads();
@@ -693,21 +705,22 @@ __global__ void __launch_bounds__(256, 1) field_solve_kernel(FieldArgs a, const 
   if (tid == 0) s_inv[0] = 1.0 / smA[0];
   __syncthreads();
   // L D L^T (the system is symmetric positive definite: J^T J, the prior and the damping) in the lower triangle, in
-  // place, a column a step across the CTA (16 x 16 threads over the trailing rows and columns); a column's entries
-  // become L's one step later, once nothing reads them. Every thread reads the same pivot, so all stop together; the
+  // place, a column a step across the CTA: L's column worked out once, then 16 x 16 threads over the trailing rows and
+  // columns; a column's entries become L's one step later, once nothing reads them. Every thread reads the same pivot, so all stop together; the
   // thread that finishes the next pivot takes its reciprocal (one double division a column).
   const int tx = tid & 15, ty = tid >> 4;
   bool ok = true;
   for (int c = 0; c < kFP; c++) {
     const double d = smA[c * kFP + c];
     if (!(d > 1e-300)) { ok = false; break; }
-    if (c > 0) {
-      const double ip = s_inv[c - 1];
-      for (int r = c + tid; r < kFP; r += blockDim.x) smA[r * kFP + c - 1] *= ip;
-    }
+    double *lc = lcol[c & 1];
+    if (c > 0)
+      for (int r = c + tid; r < kFP; r += blockDim.x) smA[r * kFP + c - 1] = lcol[(c & 1) ^ 1][r];
     const double id = s_inv[c];
+    for (int r = c + 1 + tid; r < kFP; r += blockDim.x) lc[r] = smA[r * kFP + c] * id;
+    __syncthreads();
     for (int r = c + 1 + ty; r < kFP; r += 16) {
-      const double lr = smA[r * kFP + c] * id;
+      const double lr = lc[r];
       for (int q = c + 1 + tx; q <= r; q += 16) smA[r * kFP + q] -= lr * smA[q * kFP + c];
     }
     if (tid == 0 && c + 1 < kFP) s_inv[c + 1] = 1.0 / smA[(c + 1) * kFP + c + 1];   // this thread's own last update
@@ -781,6 +794,7 @@ struct lizg_field {
   int chunk = 0;
   lizg::EncFft enc{};
   float *eff = nullptr, *G = nullptr, *part = nullptr, *base = nullptr;
+  double *sum = nullptr;
   float2 *coef = nullptr, *R = nullptr;
   lizg::FieldState *state = nullptr;
   lizg::PilotTerms *pt = nullptr;
@@ -933,6 +947,7 @@ lizg_field *lizg_field_new(int n, int subch, int span, int chunk) {
   g->base = static_cast<float *>(up(nullptr, C * a.reg_stride * 4));
   g->G = static_cast<float *>(up(nullptr, C * n * n * 4));
   g->part = static_cast<float *>(up(nullptr, C * (n / kFRows) * kFPart * 4));
+  g->sum = static_cast<double *>(up(nullptr, C * kFPart * sizeof(double)));
   g->coef = static_cast<float2 *>(up(nullptr, C * a.need * sizeof(float2)));
   g->R = static_cast<float2 *>(up(nullptr, C * a.vrows * n * sizeof(float2)));
   g->state = static_cast<FieldState *>(up(nullptr, C * sizeof(FieldState)));
@@ -986,10 +1001,11 @@ int field_eval(lizg_field *g, const lizg::FieldArgs &a, const float *base, int f
     const int basis = (int)sizeof(float2) * (a.n + 32);
     if (opt.set(reinterpret_cast<const void *>(field_grad_kernel), 16 * 1024) != cudaSuccess) return record_error(LIZG_E_CUDA, "lizg_field: adjoint pass");
     field_grad_kernel<<<fc * (a.n / kFRows), kFThreads, basis, st>>>(a, g->eff, g->G, g->pt, g->skip, g->part);
+    field_sum_kernel<<<fc * ((kFPart + kSumCols - 1) / kSumCols), 8 * kSumCols, 0, st>>>(a.n / kFRows, g->part, g->skip, g->sum);
   }
   const float *au = anchors ? anchors->u + (int64_t)f0 * 49 : nullptr, *av = anchors ? anchors->v + (int64_t)f0 * 49 : nullptr;
   const uint8_t *ao = anchors ? anchors->ok + (int64_t)f0 * 49 : nullptr;
-  field_solve_kernel<<<fc, 256, kSolveSmem, st>>>(a, g->eff, g->part, g->pt, au, av, ao, g->skip, g->state, last, terms);
+  field_solve_kernel<<<fc, 256, kSolveSmem, st>>>(a, g->eff, g->sum, g->pt, au, av, ao, g->skip, g->state, last, terms);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : record_error(LIZG_E_CUDA, (std::string("lizg_field: ") + cudaGetErrorString(e)).c_str());
 }
