@@ -53,31 +53,38 @@ struct FitArgs {
 };
 
 // Gauss-Jordan with partial pivoting on the first p rows of A (the right-hand side in column kLP) across a warp, the
-// reference's solve_lens (liblizard/src/acquire.c:1491-1504) operation for operation: lane 0 finds the pivot (the
-// first largest magnitude), the lanes swap the two rows, take each row's factor from its pivot-column entry, then
-// update every (row, column) entry, each with the product and subtraction the serial loop makes. Returns (on every
-// lane) 0 where a pivot falls under thresh.
-__device__ bool warp_gj(double (*A)[kLP + 1], int p, double thresh, double *s_f, int *s_piv) {
+// reference's solve_lens (liblizard/src/acquire.c:1491-1504) operation for operation: the pivot (the first largest
+// magnitude, found over the lanes as whole numbers: a double's bits order as it does; a NaN beats nothing and, first, is
+// beaten by nothing), the lanes swap the two rows, take each row's factor from its pivot-column entry, then update every
+// (row, column) entry, half a warp a row, each with the product and subtraction the serial loop makes. Returns (on every
+// lane) 0 where a pivot falls under thresh. Bound: latency, a division and an update a column.
+__device__ bool warp_gj(double (*A)[kLP + 1], int p, double thresh, double *s_f) {
+  static_assert(kLP <= 16, "a lane a row, half a warp a row's columns");
   const int lane = threadIdx.x & 31;
   for (int c = 0; c < p; c++) {
-    if (lane == 0) {
-      int pv = c;
-      for (int r = c + 1; r < p; r++) if (fabs(A[r][c]) > fabs(A[pv][c])) pv = r;
-      s_piv[0] = pv;
-      s_piv[1] = fabs(A[pv][c]) < thresh;
+    unsigned long long key = 0;
+    int pv = lane & 15;
+    if (pv >= c && pv < p) {
+      const double v = fabs(A[pv][c]);
+      key = v == v ? (unsigned long long)__double_as_longlong(v) + 1 : pv == c ? ~0ull : 0;
     }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      const unsigned long long ok = __shfl_xor_sync(0xffffffffu, key, o);
+      const int oa = __shfl_xor_sync(0xffffffffu, pv, o);
+      if (ok > key || (ok == key && oa < pv)) { key = ok; pv = oa; }
+    }
+    if (fabs(A[pv][c]) < thresh) return false;
     __syncwarp();
-    if (s_piv[1]) return false;
-    const int pv = s_piv[0];
-    if (pv != c)
-      for (int k = lane; k <= kLP; k += 32) { const double t = A[c][k]; A[c][k] = A[pv][k]; A[pv][k] = t; }
+    if (pv != c && lane <= kLP) { const double t = A[c][lane]; A[c][lane] = A[pv][lane]; A[pv][lane] = t; }
     __syncwarp();
-    for (int r = lane; r < p; r += 32) s_f[r] = r == c ? 0.0 : A[r][c] / A[c][c];
+    if (lane < p) s_f[lane] = lane == c ? 0.0 : A[lane][c] / A[c][c];
     __syncwarp();
-    const int ncol = kLP + 1 - c;
-    for (int e = lane; e < p * ncol; e += 32) {
-      const int r = e / ncol, k = c + (e - r * ncol);
-      if (r != c) A[r][k] -= s_f[r] * A[c][k];
+    const int k = c + (lane & 15);
+#pragma unroll
+    for (int it = 0; it < (kLP + 1) / 2; it++) {
+      const int r = 2 * it + (lane >> 4);
+      if (r < p && r != c && k <= kLP) A[r][k] -= s_f[r] * A[c][k];
     }
     __syncwarp();
   }
@@ -89,7 +96,7 @@ constexpr int kFitThreads = 128;
 struct FitScratch {
   double A[4][kLP][kLP + 1];
   double f[4][kLP], t[4][kLP], term[4][kMaxPts], aicc[4], tb[kLP];
-  int ok[4], piv[4][2], K;
+  int ok[4], K;
 };
 
 // lensm_fit's models over the points (liblizard/src/acquire.c:1651-1668) from its summed normal equations sA (upper
@@ -112,21 +119,27 @@ __device__ void block_models(int np, int n, double (*rx)[kLP], double (*ry)[kLP]
       A[r][c] = sA[r][c] + (r == c && c < p ? 1e-12 : 0.0);
     }
     __syncwarp();
-    const bool ok = 2 * n - p - 1 > 0 && warp_gj(A, p, 1e-14, F.f[k], F.piv[k]);
+    const bool ok = 2 * n - p - 1 > 0 && warp_gj(A, p, 1e-14, F.f[k]);
     if (ok) {
       for (int c = lane; c < kLP; c += 32) F.t[k][c] = c < p ? A[c][kLP] / A[c][c] : 0.0;
       __syncwarp();
       for (int i = lane; i < np; i += 32) {
         if (drop && drop[i]) continue;
-        double fx = 0, fy = 0;
-        for (int c = 0; c < p; c++) { fx += F.t[k][c] * rx[i][c]; fy += F.t[k][c] * ry[i][c]; }
+        // the terms in order, but those of a coefficient and one of rows_of's zeros, which add nothing
+        const double *tk = F.t[k];
+        double fx = tk[0] * rx[i][0] + tk[1] * rx[i][1] + tk[4] + tk[6] * rx[i][6] + tk[7] * rx[i][7];
+        double fy = tk[2] * ry[i][2] + tk[3] * ry[i][3] + tk[5] + tk[6] * ry[i][6] + tk[7] * ry[i][7];
+        for (int c = 8; c < p; c++) { fx += tk[c] * rx[i][c]; fy += tk[c] * ry[i][c]; }
         F.term[k][i] = (d[i][0] - fx) * (d[i][0] - fx) + (d[i][1] - fy) * (d[i][1] - fy);
       }
       __syncwarp();
       if (lane == 0) {
         double rss = 0;
-        for (int i = 0; i < np; i++)
-          if (!(drop && drop[i])) rss += F.term[k][i];
+#pragma unroll 8
+        for (int i = 0; i < np; i++) {
+          const double with = rss + F.term[k][i];
+          rss = drop && drop[i] ? rss : with;
+        }
         const double n2 = 2.0 * n;
         F.aicc[k] = n2 * log(rss / n2 + 1e-30) + 2.0 * p + 2.0 * p * (p + 1) / (n2 - p - 1);
       }
@@ -145,15 +158,46 @@ __device__ void block_models(int np, int n, double (*rx)[kLP], double (*ry)[kLP]
 }
 
 // The normal equations' upper triangle and right side over the points not dropped (drop NULL: all), an entry a thread,
-// each summed over the points in their order.
+// each summed over the points in their order: rx rx' + ry ry', of which rows_of's zeros leave entries 0, 1, 4 the first
+// product alone, 2, 3, 5 the second, one of each nothing (adding a zero changes no sum). Warp 0 takes the entries of both,
+// warps 1 and 2 those of one, warp 3 the empty ones; no branch in a sum, so that its loads and products run ahead of it.
 __device__ void block_normal(int np, double (*rx)[kLP], double (*ry)[kLP], double (*d)[2], const uint8_t *drop, double (*sA)[kLP + 1]) {
-  for (int e = threadIdx.x; e < 77; e += blockDim.x) {
-    int p, q;
-    if (e < 66) { p = 0; int r = e; while (r >= kLP - p) { r -= kLP - p; p++; } q = p + r; }
-    else { p = e - 66; q = kLP; }
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int p = -1, q = 0;
+  if (w == 0 && lane < 20) {   // 6..10 against 6..10 and the right side
+    p = 0; q = lane;
+    while (q >= 6 - p) { q -= 6 - p; p++; }
+    q = p + q == 5 ? kLP : 6 + p + q;
+    p += 6;
+  } else if ((w == 1 || w == 2) && lane < 24) {   // a, b, c against one another, 6..10 and the right side
+    const int a = w == 1 ? 0 : 2, c = w == 1 ? 4 : 5;
+    auto own = [&](int k) { return k == 2 ? c : a + k; };
+    const int k = lane / 8, m = lane % 8;
+    p = own(k);
+    q = m < 3 ? (m < k ? -1 : own(m)) : m + 3;
+    if (q < 0) { q = kLP; p = own(k == 1 ? 0 : m + 1); }   // the three places under the diagonal: the right sides
+  } else if (w == 3 && lane < 9) {
+    const int x = lane % 3 == 2 ? 4 : lane % 3, y = lane / 3 == 2 ? 5 : 2 + lane / 3;
+    sA[min(x, y)][max(x, y)] = 0;
+  }
+  if (p >= 0) {
+    const double *xp = &rx[0][p], *yp = &ry[0][p], *xq = q < kLP ? &rx[0][q] : &d[0][0], *yq = q < kLP ? &ry[0][q] : &d[0][1];
+    const int step = q < kLP ? kLP : 2;
+    const double *fp = w == 2 ? yp : xp, *fq = w == 2 ? yq : xq;
     double acc = 0;
-    for (int i = 0; i < np; i++)
-      if (!(drop && drop[i])) acc += q < kLP ? rx[i][p] * rx[i][q] + ry[i][p] * ry[i][q] : rx[i][p] * d[i][0] + ry[i][p] * d[i][1];
+    if (w == 0) {
+#pragma unroll 4
+      for (int i = 0; i < np; i++) {
+        const double with = acc + (xp[i * kLP] * xq[i * step] + yp[i * kLP] * yq[i * step]);
+        acc = drop && drop[i] ? acc : with;
+      }
+    } else {
+#pragma unroll 4
+      for (int i = 0; i < np; i++) {
+        const double with = acc + fp[i * kLP] * fq[i * step];
+        acc = drop && drop[i] ? acc : with;
+      }
+    }
     sA[p][q] = acc;
   }
   __syncthreads();
@@ -254,8 +298,8 @@ __global__ void count_found_kernel(const uint8_t *ok, int32_t *found) {
 // (anchor_model_free with lensm_fit's rounds); then each corner judged by that map and, where it disagrees by more
 // than 3 modules, searched again (the border node search on the corner, through the corners' H and the joint model
 // of the anchors and the kept corners) and H made again from the four corners; then the anchors' model about H.
-// The serial parts run on one warp a frame: lanes sum the normal equations' entries (each entry over the points in
-// order), lane 0 solves, judges and sorts, in double as the reference does.
+// A block a frame: a thread a normal equations' entry (each over the points in order), a warp a solve, a thread a point's
+// distance, rank and verdict, in double as the reference does.
 
 constexpr int kRounds = 6, kAnchMin = 12, kCornerMod = 3;
 
@@ -290,12 +334,11 @@ struct RegArgs {
 // (on every thread) 1 where a model fitted.
 __device__ int block_lensm_fit(int np, double (*rx)[kLP], double (*ry)[kLP], double (*d)[2], const double *qx, const double *qy, uint8_t *drop,
                                bool robust, double tau_floor, double ax, double ay, double R, double *lens, double (*sA)[kLP + 1],
-                               FitScratch &F, double *res, double *srt, int *s_flag) {
+                               FitScratch &F, double *res, double *srt) {
   const int tid = threadIdx.x;
   int ok = 0;
   for (int round = 0; round < 4; round++) {
-    int n = 0;
-    for (int i = 0; i < np; i++) n += !drop[i];
+    const int n = __syncthreads_count(tid < np && !drop[tid]);
     block_normal(np, rx, ry, d, drop, sA);
     block_models(np, n, rx, ry, d, drop, sA, F);
     if (F.K < 0) break;
@@ -307,29 +350,32 @@ __device__ int block_lensm_fit(int np, double (*rx)[kLP], double (*ry)[kLP], dou
     __syncthreads();
     if (!robust || round == 3) break;
     // the robust rule: every point's distance from the model, tau from their median, the verdicts again
-    for (int i = tid; i < np; i += blockDim.x) {
+    static_assert(kMaxPts <= kFitThreads, "a thread a point");
+    if (tid < np) {
       float fx, fy;
-      lens_at(lens, qx[i] * R + ax, qy[i] * R + ay, &fx, &fy);
-      res[i] = hypot(d[i][0] - fx, d[i][1] - fy);
+      lens_at(lens, qx[tid] * R + ax, qy[tid] * R + ay, &fx, &fy);
+      res[tid] = hypot(d[tid][0] - fx, d[tid][1] - fy);
     }
     __syncthreads();
-    for (int i = tid; i < np; i += blockDim.x) {   // the ascending order, ties by index: the sort's array
+    if (tid < np) {   // the ascending order, ties by index: the sort's array (no distance is negative: bits order as doubles do)
+      const long long mine = __double_as_longlong(res[tid]);
       int rank = 0;
-      for (int j = 0; j < np; j++) rank += res[j] < res[i] || (res[j] == res[i] && j < i);
-      srt[rank] = res[i];
-    }
-    __syncthreads();
-    if (tid == 0) {
-      const double tau = fmax(tau_floor, 3 * 1.4826 * srt[np / 2]);
-      int changed = 0;
-      for (int i = 0; i < np; i++) {
-        const uint8_t bad = res[i] > tau;
-        if (bad != drop[i]) { drop[i] = bad; changed++; }
+#pragma unroll 8
+      for (int j = 0; j < np; j++) {
+        const long long v = __double_as_longlong(res[j]);
+        rank += v < mine || (v == mine && j < tid);
       }
-      s_flag[1] = changed > 0;
+      srt[rank] = res[tid];
     }
     __syncthreads();
-    if (!s_flag[1]) break;
+    bool changed = false;
+    if (tid < np) {
+      const double tau = fmax(tau_floor, 3 * 1.4826 * srt[np / 2]);
+      const uint8_t bad = res[tid] > tau;
+      changed = bad != drop[tid];
+      drop[tid] = bad;
+    }
+    if (!__syncthreads_or(changed)) break;
   }
   return ok;
 }
@@ -359,17 +405,20 @@ __global__ void reg_init_kernel(RegArgs a, int frames) {
 }
 
 // One round's bookkeeping after the search: the anchors found, the homography they say, the robust model about it,
-// the anchors it drops no longer found (acquire.c:2133-2143). A block of kFitThreads a frame.
+// the anchors it drops no longer found (acquire.c:2133-2143). A block of kFitThreads a frame. Bound: the latency of double
+// operations in the reference's order; what no order binds is a thread an anchor, an entry or a chain. 64 frames: 310 us
+// with the normal equations' quotients and the means' distances worked out serially or again by every thread, 117 so.
 __global__ void __launch_bounds__(kFitThreads) reg_round_kernel(RegArgs a, uint8_t *active) {
   const int f = blockIdx.x, tid = threadIdx.x;
   RegState &S = a.st[f];
   if (!S.active) return;
   __shared__ double s_rx[kNA][kLP], s_ry[kNA][kLP], s_d[kNA][2], s_qx[kNA], s_qy[kNA], s_A[kLP][kLP + 1], s_res[kNA], s_srt[kNA];
-  __shared__ double s_M[kLP][kLP + 1], s_mean[6], s_lens[kLensStride], s_gf[kLP];
+  __shared__ double s_M[kLP][kLP + 1], s_mean[6], s_lens[kLensStride], s_gf[kLP], s_g[9], s_gt[9], s_hh[9];
   __shared__ FitScratch F;
   __shared__ float s_X[kNA], s_Y[kNA], s_u[kNA], s_v[kNA];
   __shared__ uint8_t s_ok[kNA], s_drop[kNA];
-  __shared__ int s_at[kNA], s_pos[kNA], s_np, s_flag[2], s_go, s_piv[2];
+  __shared__ int s_at[kNA], s_pos[kNA], s_go;
+  __shared__ uint32_t s_bits[2];
   const float ah = a.a * 0.5f;
   for (int k = tid; k < kNA; k += blockDim.x) {
     const int64_t o = (int64_t)f * kNA + k;
@@ -377,69 +426,114 @@ __global__ void __launch_bounds__(kFitThreads) reg_round_kernel(RegArgs a, uint8
     s_X[k] = (float)a.m0[k % 7] + ah; s_Y[k] = (float)a.m0[k / 7] + ah;
   }
   __syncthreads();
+  if (tid < 64) {
+    const uint32_t bits = __ballot_sync(0xffffffffu, tid < kNA && s_ok[tid]);
+    if ((tid & 31) == 0) s_bits[tid >> 5] = bits;
+  }
+  __syncthreads();
+  const unsigned long long found = s_bits[0] | (unsigned long long)s_bits[1] << 32;
+  const int n = __popcll(found);
   if (tid == 0) {
-    int now = 0;
-    for (int k = 0; k < kNA; k++) now += s_ok[k];
-    s_go = 1;
-    if (now == S.nf || now < 4) { S.active = 0; active[f] = 0; s_go = 0; }
-    else {
-      S.nf = now;
-      // anchor_homo (acquire.c:2062-2094): centres and scales, in the anchors' order
-      int n = 0, rows = 0, cols = 0, rm = 0, cm = 0;
-      double mx = 0, my = 0, mu = 0, mv = 0;
-      for (int k = 0; k < kNA; k++) if (s_ok[k]) { n++; mx += s_X[k]; my += s_Y[k]; mu += s_u[k]; mv += s_v[k]; rm |= 1 << (k / 7); cm |= 1 << (k % 7); }
-      for (int b = 0; b < 7; b++) { rows += (rm >> b) & 1; cols += (cm >> b) & 1; }
-      double sx = 0, su = 0;
-      int fit = n >= 8 && rows >= 3 && cols >= 3;
-      if (fit) {
-        mx /= n; my /= n; mu /= n; mv /= n;
-        for (int k = 0; k < kNA; k++) if (s_ok[k]) { sx += hypot(s_X[k] - mx, s_Y[k] - my); su += hypot(s_u[k] - mu, s_v[k] - mv); }
-        sx = sx / n / 1.4142135623730951; su = su / n / 1.4142135623730951;
-        fit = sx > 0 && su > 0;
-      }
-      s_mean[0] = mx; s_mean[1] = my; s_mean[2] = mu; s_mean[3] = mv; s_mean[4] = sx; s_mean[5] = su;
-      s_flag[0] = fit;
+    s_go = !(n == S.nf || n < 4);
+    if (s_go) S.nf = n; else { S.active = 0; active[f] = 0; }
+  }
+  // anchor_homo (acquire.c:2062-2094): centres and scales, in the anchors' order, a chain a thread
+  int rows = 0, cols = 0;
+#pragma unroll
+  for (int b = 0; b < 7; b++) {
+    rows += (found >> (7 * b) & 127) != 0;
+    cols += (found & (0x40810204081ull << b)) != 0;
+  }
+  const bool enough = n >= 8 && rows >= 3 && cols >= 3;
+  if (tid < 4 && enough) {
+    const float *src = tid == 0 ? s_X : tid == 1 ? s_Y : tid == 2 ? s_u : s_v;
+    double sum = 0;
+#pragma unroll 7
+    for (int k = 0; k < kNA; k++) {
+      const double with = sum + src[k];
+      sum = s_ok[k] ? with : sum;
     }
+    s_mean[tid] = sum / n;
   }
   __syncthreads();
   if (!s_go) return;
-  if (s_flag[0]) {
-    const double mx = s_mean[0], my = s_mean[1], mu = s_mean[2], mv = s_mean[3], sx = s_mean[4], su = s_mean[5];
-    // the 8 x 8 normal equations and right side, an entry a thread, each over the anchors in order; the rest zero
-    for (int e = tid; e < kLP * (kLP + 1); e += blockDim.x) {
-      const int p = e / (kLP + 1), q = e - p * (kLP + 1);
-      if (p >= 8 || (q >= 8 && q < kLP)) { s_M[p][q] = 0; continue; }
-      double acc = 0;
+  double mx = 0, my = 0, mu = 0, mv = 0, sx = 0, su = 0;
+  if (enough) {
+    mx = s_mean[0]; my = s_mean[1]; mu = s_mean[2]; mv = s_mean[3];
+    if (tid < kNA) s_res[tid] = hypot(s_X[tid] - mx, s_Y[tid] - my);
+    else if (tid >= 64 && tid < 64 + kNA) s_srt[tid - 64] = hypot(s_u[tid - 64] - mu, s_v[tid - 64] - mv);
+    __syncthreads();
+    if (tid < 2) {
+      const double *src = tid ? s_srt : s_res;
+      double sum = 0;
+#pragma unroll 7
       for (int k = 0; k < kNA; k++) {
-        if (!s_ok[k]) continue;
-        const double x = (s_X[k] - mx) / sx, y = (s_Y[k] - my) / sx, uu = (s_u[k] - mu) / su, vv = (s_v[k] - mv) / su;
-        const double r0[8] = {x, y, 1, 0, 0, 0, -uu * x, -uu * y}, r1[8] = {0, 0, 0, x, y, 1, -vv * x, -vv * y};
-        acc += q < kLP ? r0[p] * r0[q] + r1[p] * r1[q] : r0[p] * uu + r1[p] * vv;
+        const double with = sum + src[k];
+        sum = s_ok[k] ? with : sum;
       }
-      s_M[p][q] = acc;
+      s_mean[4 + tid] = sum / n / 1.4142135623730951;
     }
     __syncthreads();
-    if (tid < 32) {   // solve_lens(M, 8) on warp 0, then H through the centring
-      const bool solved = warp_gj(s_M, 8, 1e-14, s_gf, s_piv);
-      if (solved && tid == 0) {
-        double g[9];
-        for (int p = 0; p < 8; p++) g[p] = s_M[p][kLP] / s_M[p][p];
-        g[8] = 1;
-        const double tx[9] = {1 / sx, 0, -mx / sx, 0, 1 / sx, -my / sx, 0, 0, 1}, ti[9] = {su, 0, mu, 0, su, mv, 0, 0, 1};
-        double gt[9], h[9];
-        for (int r = 0; r < 3; r++) for (int c = 0; c < 3; c++) { gt[3 * r + c] = 0; for (int k = 0; k < 3; k++) gt[3 * r + c] += g[3 * r + k] * tx[3 * k + c]; }
-        for (int r = 0; r < 3; r++) for (int c = 0; c < 3; c++) { h[3 * r + c] = 0; for (int k = 0; k < 3; k++) h[3 * r + c] += ti[3 * r + k] * gt[3 * k + c]; }
-        if (fabs(h[8]) > 1e-12) for (int k = 0; k < 9; k++) S.Ha[k] = (float)(h[k] / h[8]);
+    sx = s_mean[4]; su = s_mean[5];
+  }
+  if (enough && sx > 0 && su > 0) {
+    // each anchor's two rows and right sides, then the 8 x 8 normal equations, an entry of the upper triangle a thread,
+    // each over the anchors in order (its mirror the same products), the rest zero
+    if (tid < kNA) {
+      const double x = (s_X[tid] - mx) / sx, y = (s_Y[tid] - my) / sx, uu = (s_u[tid] - mu) / su, vv = (s_v[tid] - mv) / su;
+      const double r0[8] = {x, y, 1, 0, 0, 0, -uu * x, -uu * y}, r1[8] = {0, 0, 0, x, y, 1, -vv * x, -vv * y};
+#pragma unroll
+      for (int q = 0; q < 8; q++) { s_rx[tid][q] = r0[q]; s_ry[tid][q] = r1[q]; }
+      s_d[tid][0] = uu; s_d[tid][1] = vv;
+    }
+    for (int e = tid; e < kLP * (kLP + 1); e += blockDim.x) {
+      const int p = e / (kLP + 1), q = e - p * (kLP + 1);
+      if (p >= 8 || (q >= 8 && q < kLP)) s_M[p][q] = 0;
+    }
+    __syncthreads();
+    if (tid < 44) {
+      int p = 0, q = tid;
+      while (q >= 9 - p) { q -= 9 - p; p++; }
+      q += p;   // 8: the right side
+      const double *a0 = &s_rx[0][p], *a1 = &s_ry[0][p], *b0 = q < 8 ? &s_rx[0][q] : &s_d[0][0], *b1 = q < 8 ? &s_ry[0][q] : &s_d[0][1];
+      const int step = q < 8 ? kLP : 2;
+      double acc = 0;
+#pragma unroll 7
+      for (int k = 0; k < kNA; k++) {
+        const double with = acc + (a0[k * kLP] * b0[k * step] + a1[k * kLP] * b1[k * step]);
+        acc = s_ok[k] ? with : acc;
+      }
+      if (q < 8) { s_M[p][q] = acc; s_M[q][p] = acc; }
+      else s_M[p][kLP] = acc;
+    }
+    __syncthreads();
+    if (tid < 32) {   // solve_lens(M, 8) on warp 0, then H through the centring, an entry a lane
+      const bool solved = warp_gj(s_M, 8, 1e-14, s_gf);
+      if (solved) {
+        if (tid < 9) s_g[tid] = tid < 8 ? s_M[tid][kLP] / s_M[tid][tid] : 1.0;
+        __syncwarp();
+        const int r = tid / 3, c = tid % 3;
+        if (tid < 9) {
+          const double t0 = c == 0 ? 1 / sx : c == 2 ? -mx / sx : 0, t1 = c == 1 ? 1 / sx : c == 2 ? -my / sx : 0, t2 = c == 2;
+          double v = 0;
+          v += s_g[3 * r] * t0; v += s_g[3 * r + 1] * t1; v += s_g[3 * r + 2] * t2;
+          s_gt[tid] = v;
+        }
+        __syncwarp();
+        if (tid < 9) {
+          const double t0 = r == 0 ? su : 0, t1 = r == 1 ? su : 0, t2 = r == 0 ? mu : r == 1 ? mv : 1;
+          double v = 0;
+          v += t0 * s_gt[c]; v += t1 * s_gt[3 + c]; v += t2 * s_gt[6 + c];
+          s_hh[tid] = v;
+        }
+        __syncwarp();
+        if (tid < 9 && fabs(s_hh[8]) > 1e-12) S.Ha[tid] = (float)(s_hh[tid] / s_hh[8]);
       }
     }
     __syncthreads();
   }
   // anchor_model_free (acquire.c:2101-2118): the anchors' displacements about Ha, the robust rule at half a module
-  if (tid == 0) {
-    int np = 0;
-    for (int k = 0; k < kNA; k++) s_pos[k] = s_ok[k] ? np++ : -1;
-    s_np = np;
-  }
+  if (tid < kNA) s_pos[tid] = s_ok[tid] ? __popcll(found & ((1ull << tid) - 1)) : -1;
   __syncthreads();
   for (int k = tid; k < kNA; k += blockDim.x) {
     const int i = s_pos[k];
@@ -453,9 +547,9 @@ __global__ void __launch_bounds__(kFitThreads) reg_round_kernel(RegArgs a, uint8
     s_d[i][0] = ddx; s_d[i][1] = ddy; s_drop[i] = 0; s_at[i] = k;
   }
   __syncthreads();
-  const int np = s_np;
+  const int np = n;
   const int have = np >= 4 && block_lensm_fit(np, s_rx, s_ry, s_d, s_qx, s_qy, s_drop, true, 0.5 * (double)S.mpx, a.ax, a.ay, a.R, s_lens,
-                                              s_A, F, s_res, s_srt, s_flag);
+                                              s_A, F, s_res, s_srt);
   if (tid == 0) {
     S.have = have;
     a.have_mf[f] = have;
@@ -480,7 +574,7 @@ __global__ void __launch_bounds__(kFitThreads) reg_corners_kernel(RegArgs a) {
   __shared__ double s_res[kMaxPts], s_srt[kMaxPts], s_lens[kLensStride];
   __shared__ FitScratch F;
   __shared__ uint8_t s_drop[kMaxPts];
-  __shared__ int s_pos[kNA], s_np, s_flag[2], s_go;
+  __shared__ int s_pos[kNA], s_np, s_go;
   if (tid == 0) {
     s_go = S.have && S.nf >= kAnchMin;
     S.held = s_go;
@@ -517,7 +611,7 @@ __global__ void __launch_bounds__(kFitThreads) reg_corners_kernel(RegArgs a) {
     }
   }
   __syncthreads();
-  const int fit = block_lensm_fit(s_np, s_rx, s_ry, s_d, s_qx, s_qy, s_drop, false, 0, a.ax, a.ay, a.R, s_lens, s_A, F, s_res, s_srt, s_flag);
+  const int fit = block_lensm_fit(s_np, s_rx, s_ry, s_d, s_qx, s_qy, s_drop, false, 0, a.ax, a.ay, a.R, s_lens, s_A, F, s_res, s_srt);
   if (tid == 0) {
     S.mc_on = fit;
     a.on_mc[f] = fit;
@@ -534,13 +628,13 @@ __global__ void reg_redo_kernel(const RegState *st, int frames, uint8_t *redo) {
 
 // The corners searched again replace the measured ones (score 0.35 or more: the search's place, else the joint
 // model's), H made again from the four (acquire.c:2174-2195, homography 611-654), the anchors' displacements about H.
-// A thread a frame.
-__global__ void reg_finish_kernel(RegArgs a, int frames, float *quad_out) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= frames) return;
+// A CTA of kNA threads or more a frame: thread 0 the
+// corners and H, then an anchor a thread.
+__global__ void __launch_bounds__(64) reg_finish_kernel(RegArgs a, float *quad_out) {
+  const int f = blockIdx.x, tid = threadIdx.x;
   RegState &S = a.st[f];
   float *h = a.reg + (int64_t)f * a.hstride;
-  if (S.held) {
+  if (S.held && tid == 0) {
     const int nn = a.nn;
     int moved = 0;
     for (int c = 0; c < 4; c++) {
@@ -579,17 +673,18 @@ __global__ void reg_finish_kernel(RegArgs a, int frames, float *quad_out) {
         h[8] = 1;
       }
     }
-    const float ah = a.a * 0.5f;
-    for (int k = 0; k < kNA; k++) {
-      const int64_t o = (int64_t)f * kNA + k;
-      if (!a.ok[o]) continue;
-      float hu, hv;
-      project_f(h, (float)a.m0[k % 7] + ah, (float)a.m0[k / 7] + ah, &hu, &hv);
-      a.dx[o] = a.u[o] - hu; a.dy[o] = a.v[o] - hv;
-    }
   }
-  if (quad_out) for (int k = 0; k < 8; k++) quad_out[(int64_t)f * 8 + k] = S.quad[k];
+  __syncthreads();
+  const int64_t o = (int64_t)f * kNA + tid;
+  if (S.held && tid < kNA && a.ok[o]) {
+    const float ah = a.a * 0.5f;
+    float hu, hv;
+    project_f(h, (float)a.m0[tid % 7] + ah, (float)a.m0[tid / 7] + ah, &hu, &hv);
+    a.dx[o] = a.u[o] - hu; a.dy[o] = a.v[o] - hv;
+  }
+  if (quad_out && tid < 8) quad_out[(int64_t)f * 8 + tid] = S.quad[tid];
 }
+
 
 __global__ void reg_held_kernel(const RegState *st, int frames, int *held) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
@@ -743,7 +838,7 @@ int lizg_anchor_register_dev(lizg_refiner *r, const uint8_t *d_luma, const uint8
     const float *d_H0 = reinterpret_cast<const float *>(reinterpret_cast<const char *>(r->st) + offsetof(RegState, H0));
     e = border_corners_launch(r->span, d_rim ? d_rim : d_luma, w, h, frame_stride, d_H0, st_stride, r->mc, r->on_mc, r->redo, frames, r->nodes, st);
   }
-  if (e == cudaSuccess) { reg_finish_kernel<<<(frames + 127) / 128, 128, 0, st>>>(a, frames, d_quad); e = cudaGetLastError(); }
+  if (e == cudaSuccess) { reg_finish_kernel<<<frames, 64, 0, st>>>(a, d_quad); e = cudaGetLastError(); }
   if (e == cudaSuccess) { reg_held_kernel<<<(frames + 127) / 128, 128, 0, st>>>(r->st, frames, r->held); e = cudaGetLastError(); }
   if (e == cudaSuccess) {
     // the anchors' model about H (anchor_model) where the registration held, then the mesh
