@@ -198,11 +198,12 @@ def reference_estimate(value, kind):
             "measured": False}
 
 
-# Integer operations an edge update costs at the least in layered min-sum (liblizard/src/ldpc.c:141-192): the extrinsic
+# Operations an edge update costs at the least in layered min-sum (liblizard/src/ldpc.c:141-192): the extrinsic
 # q = L - R, its saturation to 8 bits, |q|, the running min1 / min2 (two min/max), the sign's XOR, the message's
 # sign select, the posterior L = q + R.
 OPS_PER_EDGE = 8
 ALU_LANES_PER_SM = 64   # 4 sub-partitions x 16 lanes: one ALU warp-instruction every 2 cycles each
+OPS_PER_LANE = 2        # the two-codeword form's operations are 16-bit pairs, a codeword a half
 
 
 def int_op_roofline(edges, launch_ms, sm_mhz, sms):
@@ -211,9 +212,9 @@ def int_op_roofline(edges, launch_ms, sm_mhz, sms):
     if not sm_mhz:
         return None
     achieved = edges / (launch_ms / 1e3) * OPS_PER_EDGE / 1e12
-    peak = sms * ALU_LANES_PER_SM * sm_mhz * 1e6 / 1e12
+    peak = sms * ALU_LANES_PER_SM * OPS_PER_LANE * sm_mhz * 1e6 / 1e12
     return {"achieved": round(achieved, 3), "peak": round(peak, 3), "unit": "Tops/s", "frac": round(achieved / peak, 4),
-            "ops_per_edge_update": OPS_PER_EDGE, "peak_from": "%d SMs x %d ALU lanes x the median SM clock under load (%.0f MHz)" % (sms, ALU_LANES_PER_SM, sm_mhz)}
+            "ops_per_edge_update": OPS_PER_EDGE, "peak_from": "%d SMs x %d ALU lanes x %d 16-bit operations x the median SM clock under load (%.0f MHz)" % (sms, ALU_LANES_PER_SM, OPS_PER_LANE, sm_mhz)}
 
 
 def picture_frames(fmt, count, seed, sigma):
@@ -1396,14 +1397,14 @@ def main():
                  "autotune": tune},
         "roofline": {"bound": "hbm", "achieved": round(achieved, 2), "peak": peak, "unit": "GB/s", "frac": round(achieved / peak, 5),
                      "traffic": None if traffic is None else int(traffic), "peak_source": peak_src,
-                     "kernel": "ldpc_decode_kernel<7/8,3/4,2/3,1/2> (the 4 launches of a step)",
+                     "kernel": "ldpc_dual_kernel<7/8,3/4,2/3,1/2> (the 4 launches of a step)",
                      "note": "not HBM bound: the min-sum minima issue on the ALU pipe (every min/max form does on sm_103a); "
                              "int_op is its roofline",
                      "int_op": int_op_roofline(edges, launch_ms, sm_mhz, sms),
-                     "alu_pipe": {"active_frac": 0.856, "measured": False,
-                                  "kernel": "ldpc_decode_kernel 7/8 code (41% of a step), 2 warps a codeword, pair form with the loop",
-                                  "source": "imported from one ncu capture (sm__pipe_alu_cycles_active, profiles/ldpc_decode_65536cw.md, "
-                                            "python bench.py --ldpc-variants --count 16384), not measured in this run"}},
+                     "alu_pipe": {"active_frac": 0.540, "measured": False,
+                                  "kernel": "ldpc_dual_kernel 7/8 code (34% of a step), two codewords to four warps",
+                                  "source": "imported from one ncu capture (sm__inst_executed_pipe_alu, profiles/ldpc_decode_65536cw.md, "
+                                            "python bench.py --count 32768), not measured in this run"}},
         "gpu_launches": launches,
         "clocks": clocks,
     }
