@@ -568,7 +568,7 @@ int lizg_encode_dev(lizg_encoder *x, const uint8_t *d_blocks, int frames, int pi
     err = cudaGetLastError();
   }
   // a copy for the grey page alone has its grey levels taken by the transform, a byte a sample written and read instead of
-  // four: the column pass 154 us against 145 (127 now), the paint's 302 MB of samples 75
+  // four: the column pass 154 us against 145 (117 now), the paint's 302 MB of samples 75
   const bool bytes = e.copy && !d_drive;
   if (err == cudaSuccess) err = enc_page_launch(x->xf, frames, x->signs, x->S, x->pic, bytes, st);
   if (err == cudaSuccess) {
