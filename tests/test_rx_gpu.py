@@ -159,3 +159,24 @@ def test_finish_coef_from_and_to_unaligned_buffers(turn):
     assert np.array_equal(blocks[1:1 + o["blocks"].numel()].cpu().numpy(), want["blocks"].ravel())
     for k in ("its", "ok", "est", "pilot", "sub_est", "sub_rms"):
         assert np.array_equal(o[k].cpu().numpy(), want[k], equal_nan=k == "pilot"), k
+
+
+@pytest.mark.parametrize("frames", [10, 24, 36, 60])
+def test_decode_of_many_frames_matches_oracle(frames):
+    """Tiers on both sides of one and of two codewords a CTA (152 SMs hold 608, 456, 456 and 304 CTAs of the four codes; the
+    tiers are of 57, 33, 17 and 17 blocks a frame): 10 frames keep every codeword alone, 60 take items of every code from
+    the counter. Frames of six noise levels in shuffled order, so that a half takes its next block through the bit map and
+    the whitening while its partner runs on, past declined blocks, among blocks that converge, stall and run to the cap."""
+    fmt = lz.Format(1024, 1024, 128)
+    o = oracle.Fmt(1024, 1024, 128)
+    res = [o.receive(synth.grids(fmt, 1, seed=int(s), sigma=s)[0][0]) for s in (3.0, 38.0, 45.0, 60.0, 75.0, 120.0)]
+    for kind in (-1, -2, -3):
+        assert any((r["its"] == kind).any() for r in res), kind
+    order = np.random.default_rng(frames).integers(0, len(res), frames)
+    rx = lz.Receiver(1024, 1024, 128, max_frames=frames)
+    out = rx.finish_coef(np.stack([res[k]["coef"] for k in order]))
+    for f, k in enumerate(order):
+        assert np.array_equal(out["its"][f], res[k]["its"].astype(np.int32)), f
+        assert np.array_equal(out["ok"][f], res[k]["ok"]), f
+        ok = res[k]["ok"].astype(bool)
+        assert np.array_equal(out["blocks"][f][ok], res[k]["blocks"][ok]), f
