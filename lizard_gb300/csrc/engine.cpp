@@ -9,6 +9,7 @@
 #include "lizard_gb300.h"
 #include "lizg_internal.h"
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <new>
 #include <string>
 #include <vector>
@@ -67,21 +68,30 @@ int run_mixed(lizg_engine *e, const lizg_engine_batch *b, int nb, cudaStream_t s
       return rc;
   int launches = 0;
   cudaError_t c;
-  auto grids = [&](cudaError_t (*fn)(const lizg::FftSegArgs *, int, cudaStream_t)) {
-    std::vector<lizg::FftSegArgs> segs;
-    for (int i0 = 0; i0 < nb; i0 += lizg::kFftMixSegs) {
-      segs.clear();
-      for (int i = i0; i < nb && i < i0 + lizg::kFftMixSegs; i++) segs.push_back(calls[i].fft);
-      const cudaError_t x = fn(segs.data(), (int)segs.size(), st);
+  auto grids = [&](cudaError_t (*fn)(const lizg::FftSegArgs *, int, cudaStream_t), const std::vector<lizg::FftSegArgs> &segs) {
+    for (size_t i0 = 0; i0 < segs.size(); i0 += lizg::kFftMixSegs) {
+      const cudaError_t x = fn(segs.data() + i0, (int)std::min<size_t>(lizg::kFftMixSegs, segs.size() - i0), st);
       if (x != cudaSuccess) return cuda_fail("lizg_engine_run_dev", x);
       launches++;
     }
     return 0;
   };
-  if (int rc = grids(lizg::fft_pre_mixed_launch)) return rc;
-  if (int rc = grids(lizg::fft_cols_mixed_launch)) return rc;
-  if (int rc = grids(lizg::fft_fac_mixed_launch)) return rc;
-  if (int rc = grids(lizg::fft_rows_mixed_launch)) return rc;
+  std::vector<lizg::FftSegArgs> segs;
+  for (const lizg::RxCall &x : calls) segs.push_back(x.fft);
+  // the samples' part in turns where a batch is past its receiver's workspace for them: turn k takes each format's k-th
+  for (int k = 0;; k++) {
+    std::vector<lizg::FftSegArgs> now;
+    for (const lizg::FftSegArgs &s : segs) {
+      const int turn = lizg::fft_turn(s);
+      if (turn < 1) return cuda_fail("lizg_engine_run_dev", cudaErrorInvalidValue);
+      if ((int64_t)k * turn < s.frames) now.push_back(lizg::fft_frames_of(s, k * turn, std::min(turn, s.frames - k * turn)));
+    }
+    if (now.empty()) break;
+    if (int rc = grids(lizg::fft_pre_mixed_launch, now)) return rc;
+    if (int rc = grids(lizg::fft_cols_mixed_launch, now)) return rc;
+  }
+  if (int rc = grids(lizg::fft_fac_mixed_launch, segs)) return rc;
+  if (int rc = grids(lizg::fft_rows_mixed_launch, segs)) return rc;
   {
     std::vector<lizg::DemapSeg> segs;
     for (int i0 = 0; i0 < nb; i0 += lizg::kDemapMixSegs) {

@@ -5,7 +5,8 @@
 //   hole_rhs_kernel   a CTA takes a band of the frame's every-eighth-sample rows: the shading fit's right-hand side
 //                     over the samples outside the anchors' squares, one partial sum a band (6 doubles); the frame's
 //                     last CTA to finish adds the bands and solves for the shading surface beta;
-//   sample16_kernel   (captured frames by the decode's read) the samples, 16 bits each;
+//   sample16_kernel   (captured frames by the decode's read) the samples, 16 bits each, in a bounded workspace: a batch
+//                     past it takes the kernels to here and the column pass in turns;
 //   cell_table_kernel (captured frames by the exact walk) each picture row's homography terms and the mesh displacement
 //                     line of each mesh cell along it, so the column pass reads them instead of walking the mesh per
 //                     sample;
@@ -1023,15 +1024,34 @@ int fft_y_map(CUtensorMap *map, float2 *Y, int n, int64_t rows) {
                      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
 }
 
-// The shading fit's partial sums, then (captured frames only) the sampler's row and cell table.
-cudaError_t fft_pre_launch(const FftSegArgs &a, int sms, cudaStream_t st) {
-  const int bands = fft_hole_bands(a.xd.n);
-  hole_rhs_kernel<<<a.frames * bands, kHoleThreads, 0, st>>>(a.xd, a.src, bands, a.b.hole, a.b.beta, a.b.ticket);
-  if (!a.src.grid && a.src.sd.read == LIZG_READ_DECODE) {
-    if (!a.b.g16) return cudaErrorInvalidValue;
+int fft_turn(const FftSegArgs &a) {
+  if (a.src.grid || a.src.sd.read != LIZG_READ_DECODE) return a.frames;
+  if (a.b.g16_frames < 1) return 0;
+  const int turns = (a.frames + a.b.g16_frames - 1) / a.b.g16_frames;
+  return (a.frames + turns - 1) / turns;   // alike: 128 frames of n = 1536 as 56, 56 and 16 had a short last grid
+}
+
+FftSegArgs fft_frames_of(const FftSegArgs &a, int f0, int count) {
+  FftSegArgs s = a;
+  s.frames = count;
+  if (f0 == 0) return s;
+  const int n = a.xd.n;
+  if (s.src.grid) s.src.grid += f0 * s.src.gstride;
+  if (s.src.luma) { s.src.luma += f0 * s.src.fstride; s.src.reg += (int64_t)f0 * s.src.regstride; }
+  s.b.hole += (int64_t)f0 * fft_hole_bands(n) * 6; s.b.beta += 6 * (int64_t)f0; s.b.ticket += f0;
+  s.b.part += (int64_t)f0 * (n / (2 * plan_of(n).lines)) * 5;
+  s.b.Y += (int64_t)f0 * a.xd.vrows * n;
+  return s;
+}
+
+// What the column pass reads of captured frames: the decode's samples or the exact walk's table.
+static cudaError_t fft_read_launch(const FftSegArgs &a, int sms, cudaStream_t st) {
+  if (a.src.grid) return cudaSuccess;
+  if (a.src.sd.read == LIZG_READ_DECODE) {
+    if (!a.b.g16 || a.frames > a.b.g16_frames) return cudaErrorInvalidValue;
     const int rows = sample_rows(a.xd.n, a.frames, sms);
     sample16_kernel<<<a.frames * sample_ctas(a.xd.n, rows), kSampleThreads, 0, st>>>(a.src, a.b.g16, rows);
-  } else if (!a.src.grid) {
+  } else {
     if (!a.b.ctab || a.src.sd.nx != a.src.sd.ny) return cudaErrorInvalidValue;
     const int per_frame = a.xd.n * a.src.sd.nx;
     cell_table_kernel<<<dim3((per_frame + 255) / 256, a.frames), 256, 0, st>>>(a.src, per_frame, a.b.ctab);
@@ -1039,7 +1059,7 @@ cudaError_t fft_pre_launch(const FftSegArgs &a, int sms, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-cudaError_t fft_fac_launch(const FftSegArgs &a, cudaStream_t st) {
+static cudaError_t fft_fac_launch(const FftSegArgs &a, cudaStream_t st) {
   fac_kernel<<<a.frames * kFacCtas, 256, 0, st>>>(a.xd, a.xd.n / (2 * plan_of(a.xd.n).lines), a.b.part, a.b.fac);
   return cudaGetLastError();
 }
@@ -1054,10 +1074,17 @@ static cudaError_t fft_launch_n(const FftDev &xd, int frames, const SrcDev &src,
   if ((e = opt_cols.set(reinterpret_cast<const void *>(fft_cols_kernel<N>), smem)) != cudaSuccess ||
       (e = opt_rows.set(reinterpret_cast<const void *>(fft_rows_kernel<N>), smem)) != cudaSuccess)
     return e;
-  const FftSegArgs a{xd, src, b, frames};
-  if ((e = fft_pre_launch(a, sms, st)) != cudaSuccess) return e;
-  fft_cols_kernel<N><<<frames * tiles, kThreads, smem, st>>>(xd, src, b.ctab, b.g16, b.beta, b.part, b.Y);
-  if ((e = fft_fac_launch(a, st)) != cudaSuccess) return e;
+  const FftSegArgs all{xd, src, b, frames};
+  const int turn = fft_turn(all);
+  if (turn < 1) return cudaErrorInvalidValue;
+  const int bands = fft_hole_bands(N);
+  hole_rhs_kernel<<<frames * bands, kHoleThreads, 0, st>>>(xd, src, bands, b.hole, b.beta, b.ticket);
+  for (int f0 = 0; f0 < frames; f0 += turn) {
+    const FftSegArgs a = fft_frames_of(all, f0, frames - f0 < turn ? frames - f0 : turn);
+    if ((e = fft_read_launch(a, sms, st)) != cudaSuccess) return e;
+    fft_cols_kernel<N><<<a.frames * tiles, kThreads, smem, st>>>(xd, a.src, a.b.ctab, a.b.g16, a.b.beta, a.b.part, a.b.Y);
+  }
+  if ((e = fft_fac_launch(all, st)) != cudaSuccess) return e;
   if (!b.ymap || !b.err) return cudaErrorInvalidValue;
   fft_rows_kernel<N><<<frames * ((xd.vrows + L - 1) / L), kThreads, smem, st>>>(xd, b.fac, *b.ymap, b.tpos, b.need, b.C, b.err);
   return cudaGetLastError();
@@ -1076,10 +1103,12 @@ static cudaError_t light_mix(const FftSegArgs *a, int count, FftLightMix &m) {
   m.nseg = count;
   for (int k = 0; k < count; k++) {
     const FftSegArgs &s = a[k];
-    if (!ladder_size(s.xd.n) || s.frames < 1 || s.src.grid || !s.b.ctab || s.src.sd.nx != s.src.sd.ny) return cudaErrorInvalidValue;
+    const bool sampled = s.src.sd.read == LIZG_READ_DECODE;
+    if (!ladder_size(s.xd.n) || s.frames < 1 || s.src.grid || s.src.sd.nx != s.src.sd.ny || !(sampled ? (void *)s.b.g16 : s.b.ctab))
+      return cudaErrorInvalidValue;
     FftLightSeg &g = m.seg[k];
     g.xd = s.xd; g.src = s.src; g.hole = s.b.hole; g.beta = s.b.beta; g.ticket = s.b.ticket; g.g16 = s.b.g16; g.part = s.b.part; g.ctab = s.b.ctab; g.fac = s.b.fac;
-    g.bands = fft_hole_bands(s.xd.n); g.per_frame = s.xd.n * s.src.sd.nx; g.tblocks = s.src.sd.read == LIZG_READ_DECODE ? sample_ctas(s.xd.n, 16) : (g.per_frame + kHoleThreads - 1) / kHoleThreads;
+    g.bands = fft_hole_bands(s.xd.n); g.per_frame = s.xd.n * s.src.sd.nx; g.tblocks = sampled ? sample_ctas(s.xd.n, 16) : (g.per_frame + kHoleThreads - 1) / kHoleThreads;
     g.tiles = s.xd.n / (2 * plan_of(s.xd.n).lines);
     m.hf[k + 1] = m.hf[k] + s.frames * g.bands;
     m.ff[k + 1] = m.ff[k] + s.frames * kFacCtas;
@@ -1092,6 +1121,8 @@ static cudaError_t light_mix(const FftSegArgs *a, int count, FftLightMix &m) {
 cudaError_t fft_pre_mixed_launch(const FftSegArgs *a, int count, cudaStream_t st) {
   FftLightMix m;
   if (cudaError_t e = light_mix(a, count, m)) return e;
+  for (int k = 0; k < count; k++)
+    if (a[k].frames > fft_turn(a[k])) return cudaErrorInvalidValue;
   fft_pre_mixed_kernel<<<m.tf[count], kHoleThreads, 0, st>>>(m);
   return cudaGetLastError();
 }

@@ -954,7 +954,7 @@ lizg_field *lizg_field_new(int n, int subch, int span, int chunk) {
   g->pt = static_cast<PilotTerms *>(up(nullptr, C * sizeof(PilotTerms)));
   g->skip = static_cast<uint8_t *>(up(nullptr, C));
   if (ok) {
-    g->rx = lizg_rx_new(n, subch, span, chunk);
+    g->rx = rx_new(n, subch, span, chunk, false);
     ok = g->rx != nullptr;
     if (ok) lizg_rx_set_read(g->rx, LIZG_READ_EXACT);   // the refinement's forward model: the float walk it differentiates
   }

@@ -279,7 +279,7 @@ lizg_gn *lizg_gn_new(int n, int subch, int span, int chunk) {
   if (ok) {
     a.pilot = static_cast<int32_t *>(p1); a.shat = static_cast<float2 *>(p2); a.group = static_cast<uint8_t *>(p3);
     g->grids = static_cast<float *>(p4); g->coef = static_cast<float2 *>(p5); g->state = static_cast<GnState *>(p6);
-    g->rx = lizg_rx_new(n, subch, span, chunk * kGnPics);
+    g->rx = rx_new(n, subch, span, chunk * kGnPics, false);   // grids only
     ok = g->rx != nullptr;
   }
   if (!ok) {

@@ -64,17 +64,19 @@ struct FftBufs {
   const int32_t *tpos;               // vrows x n: the pos index of spectrum point (u mod n, v), -1 where unused
   int need;                          // used coefficients a frame (subch x 320)
   float2 *C;                         // frames x need: the detrended spectrum's used coefficients in pos order
-  // frames x n x nx, filled before the column pass when captured frames are read by the exact walk: for each picture
-  // row y of a frame, the mesh displacement line of each cell i < nx - 1 (ex, cx, ey, cy, as cell_terms gives them) and
-  // at i = nx - 1 the homography's row terms (kw, ku, kv, 0)
+  // Filled before the column pass when captured frames are read, the two in one place (a batch is read one way). The
+  // exact walk's ctab, frames x n x nx: for each picture row y of a frame, the mesh displacement line of each cell
+  // i < nx - 1 (ex, cx, ey, cy, as cell_terms gives them) and at i = nx - 1 the homography's row terms (kw, ku, kv, 0).
+  // The decode's g16, g16_frames x n x n (0: the handle never reads so): the blend's whole numbers, by column tiles.
   float4 *ctab;
+  int16_t *g16;
+  int g16_frames;
   // Y as a 2D tensor (rows frames x vrows, each n complex as 2n floats; boxes of 128 complex by one row) for the row
   // pass's bulk tensor loads, and a device word the passes set when a bounded wait gave up
   const CUtensorMap *ymap;
   int *err;
   double *beta;                      // frames x 6: the shading surface
   int *ticket;                       // frames: the shading fit's CTAs done, 0 between calls
-  int16_t *g16;                      // frames x n x n: the decode's read, the blend's whole numbers, by column tiles
 };
 // Encodes the tensor map of a Y buffer of `rows` rows of n complex points (the row pass's loads). 0, or a CUresult.
 int fft_y_map(CUtensorMap *map, float2 *Y, int n, int64_t rows);
@@ -164,8 +166,7 @@ cudaError_t demap_mixed_launch(const DemapSeg *a, int count, cudaStream_t st);
 cudaError_t fft_row_table_launch(const FftDev &xd, float4 *rowc, cudaStream_t st);
 cudaError_t fft_launch(const FftDev &xd, int frames, const SrcDev &src, const FftBufs &b, int sms, cudaStream_t st);
 // One format's share of a transform stage run across formats (the engine's stage-wise run): its tables, source,
-// buffers and frames. fft_pre_launch: the shading fit's sums and the sampler's table; fft_fac_launch: the surface
-// factors; the mixed launches: one column (row) pass grid over count <= kFftMixSegs formats' tiles.
+// buffers and frames; one column (row) pass grid over count <= kFftMixSegs formats' tiles.
 constexpr int kFftMixSegs = 8;
 struct FftSegArgs {
   FftDev xd;
@@ -173,11 +174,14 @@ struct FftSegArgs {
   FftBufs b;
   int frames;
 };
-cudaError_t fft_pre_launch(const FftSegArgs &a, int sms, cudaStream_t st);
-cudaError_t fft_fac_launch(const FftSegArgs &a, cudaStream_t st);
+// The frames that a turn of reading captured frames and the column pass takes: all of them, or where the decode's
+// samples have not the room a like share in as few turns as they allow (0: they have none). fft_frames_of: the call's
+// frames f0 .. f0 + count - 1 as a call of their own.
+int fft_turn(const FftSegArgs &a);
+FftSegArgs fft_frames_of(const FftSegArgs &a, int f0, int count);
 cudaError_t fft_cols_mixed_launch(const FftSegArgs *a, int count, cudaStream_t st);
-// The light stages across formats (captured frames only): the shading sums and the sampler's tables in one launch,
-// the surface factors in one launch.
+// The light stages across formats (captured frames only): the shading sums and the decode's samples or the exact walk's
+// tables in one launch, the surface factors in one launch.
 cudaError_t fft_pre_mixed_launch(const FftSegArgs *a, int count, cudaStream_t st);
 cudaError_t fft_fac_mixed_launch(const FftSegArgs *a, int count, cudaStream_t st);
 cudaError_t fft_rows_mixed_launch(const FftSegArgs *a, int count, cudaStream_t st);
@@ -246,6 +250,8 @@ cudaError_t ldpc_mixed_launch(const LdpcMix &m, int sms, cudaStream_t st);
 int ldpc_variant_count(int code);
 int ldpc_choice(int code);   // the device's choice for the code (lizg_ldpc_autotune, lizg_ldpc_set_variant)
 cudaError_t ldpc_launch_variant(int code, int v, const LdpcLaunch &a, int sms, cudaStream_t st);
+// lizg_rx_new; with decode 0 a handle that never takes captured frames by the decode's read (no workspace for its samples).
+lizg_rx *rx_new(int n, int subch, int span, int max_frames, bool decode);
 // Row (b) alone from captured frames: the handle's read through each frame's registration, the anchors' erase, the
 // detrend and the 2D transform, the used coefficients into d_coef (frames x subch x 320 complex, pos order); no soft
 // stage. For the registration's refinements, which measure their mismatch where the receiver measures it.

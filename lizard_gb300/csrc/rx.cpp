@@ -5,6 +5,7 @@
 #include "lizard_codes.h"
 #include "lizg_internal.h"
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <new>
@@ -31,13 +32,13 @@ struct lizg_rx {
   int *counters = nullptr;
   double *hole = nullptr, *beta = nullptr, *part = nullptr;
   int *ticket = nullptr;
-  int16_t *g16 = nullptr;               // the decode's read of a batch's frames
   float2 *fac = nullptr;
   lizg::SampleDev sd{};
   float *node_xy = nullptr;
   float4 *sample_t = nullptr;
   float2 *Y = nullptr, *C = nullptr;   // column transforms' kept rows; the spectrum's used coefficients in pos order
-  float4 *ctab = nullptr;              // the sampler's row and mesh-cell terms, frames x n x nx
+  void *samples = nullptr;             // what the column pass reads of captured frames: see samples_alloc
+  int g16_frames = 0;
   int32_t *tpos = nullptr;             // vrows x n: the pos index of each kept spectrum point, -1 where unused
   CUtensorMap ymap;                    // Y as the row pass's bulk tensor loads see it
   int *dev_err = nullptr;              // set by a pass whose bounded wait gave up
@@ -82,6 +83,27 @@ cudaError_t dev_alloc(lizg_rx *r, T **dst, size_t count) {
   return e;
 }
 
+// The samples' workspace: the exact walk's table of every frame (16 n nx bytes each) or, in the same place, the decode's
+// 16-bit samples (2 n^2 bytes a frame, at n = 1536 as much as the column transforms' rows) of as many frames as
+// kSampleBytes hold: 56 of n = 1536, past which a call takes the sampler and the column pass in turns of as many. Where
+// the device has not that much left, of half as many, down to one; none where the handle never reads so.
+constexpr size_t kSampleBytes = 256u << 20;
+cudaError_t samples_alloc(lizg_rx *r, bool decode) {
+  const size_t frame = 2 * (size_t)r->f.n * r->f.n, table = (size_t)r->max_frames * r->f.n * r->sd.nx * sizeof(float4);
+  for (int held = decode ? (int)std::max<size_t>(1, std::min<size_t>(r->max_frames, kSampleBytes / frame)) : 0;; held /= 2) {
+    char *p = nullptr;
+    const cudaError_t e = dev_alloc(r, &p, std::max(table, held * frame));
+    if (e == cudaErrorMemoryAllocation && held > 1) { cudaGetLastError(); continue; }
+    r->samples = p; r->g16_frames = held;
+    return e;
+  }
+}
+
+lizg::FftBufs fft_bufs(const lizg_rx *r, float2 *C) {
+  return lizg::FftBufs{r->hole, r->part, r->fac, r->Y, r->tpos, r->f.subch * lizg::kSub, C, static_cast<float4 *>(r->samples),
+                       static_cast<int16_t *>(r->samples), r->g16_frames, &r->ymap, r->dev_err, r->beta, r->ticket};
+}
+
 lizg::FmtDev fmt_dev(const lizg_rx *r, int frames) {
   lizg::FmtDev d{};
   const lizg::Format &f = r->f;
@@ -99,9 +121,7 @@ lizg::FmtDev fmt_dev(const lizg_rx *r, int frames) {
 
 }  // namespace
 
-extern "C" {
-
-lizg_rx *lizg_rx_new(int n, int subch, int span, int max_frames) {
+lizg_rx *lizg::rx_new(int n, int subch, int span, int max_frames, bool decode) {
   if (max_frames < 1 || max_frames > 4096) { lizg::record_error(LIZG_E_ARG, "lizg_rx_new: max_frames must be 1..4096"); return nullptr; }
   int sms = 0;
   if (lizg::device_ready(&sms)) return nullptr;
@@ -180,7 +200,6 @@ lizg_rx *lizg_rx_new(int n, int subch, int span, int max_frames) {
   ok(dev_alloc(r, &r->hole, F * lizg::fft_hole_bands(n) * 6));
   ok(dev_alloc(r, &r->beta, F * 6));
   ok(dev_alloc(r, &r->ticket, F));
-  ok(dev_alloc(r, &r->g16, F * n * n));
   if (e == cudaSuccess) e = cudaMemset(r->ticket, 0, F * sizeof(int));
   ok(dev_alloc(r, &r->fac, F * (2 * (size_t)n + r->xd.vrows)));
   ok(dev_alloc(r, &r->part, F * (size_t)(n / 2) * 5));   // column tiles (at most n / 2) x 5
@@ -188,7 +207,6 @@ lizg_rx *lizg_rx_new(int n, int subch, int span, int max_frames) {
   ok(dev_alloc(r, &r->dev_err, 1));
   if (e == cudaSuccess) e = cudaMemset(r->dev_err, 0, sizeof(int));
   if (e == cudaSuccess && lizg::fft_y_map(&r->ymap, r->Y, n, F * (int64_t)r->xd.vrows)) e = cudaErrorInvalidValue;
-  ok(dev_alloc(r, &r->ctab, F * n * (size_t)r->sd.nx));
   ok(dev_alloc(r, &r->C, F * need));
   {
     std::vector<int32_t> tp((size_t)r->xd.vrows * n, -1);
@@ -203,6 +221,7 @@ lizg_rx *lizg_rx_new(int n, int subch, int span, int max_frames) {
   ok(dev_alloc(r, &r->align, F * 3));
   ok(dev_alloc(r, &r->decl, F * f.blocks));
   ok(dev_alloc(r, &r->counters, 4));
+  ok(samples_alloc(r, decode));   // last: it takes what is left
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&r->fork, cudaEventDisableTiming);
   for (int t = 0; t < 4 && e == cudaSuccess; t++) {
     if ((e = cudaStreamCreateWithFlags(&r->side[t], cudaStreamNonBlocking)) == cudaSuccess)
@@ -215,6 +234,10 @@ lizg_rx *lizg_rx_new(int n, int subch, int span, int max_frames) {
   }
   return r;
 }
+
+extern "C" {
+
+lizg_rx *lizg_rx_new(int n, int subch, int span, int max_frames) { return lizg::rx_new(n, subch, span, max_frames, true); }
 
 void lizg_rx_free(lizg_rx *r) {
   if (!r) return;
@@ -386,10 +409,13 @@ int lizg_rx_finish_coef_dev(lizg_rx *r, const float *d_coef, int frames, const l
 static int finish_src(lizg_rx *r, const lizg::SrcDev &src, int frames, const lizg_rx_out *out, float *d_coef, cudaStream_t st, int sms) {
   const int need = r->f.subch * lizg::kSub;
   float2 *C = d_coef ? reinterpret_cast<float2 *>(d_coef) : r->C;   // the caller's spectrum buffer when given
-  const lizg::FftBufs b{r->hole, r->part, r->fac, r->Y, r->tpos, need, C, r->ctab, &r->ymap, r->dev_err, r->beta, r->ticket, r->g16};
+  const lizg::FftBufs b = fft_bufs(r, C);
   cudaError_t e = lizg::fft_launch(r->xd, frames, src, b, sms, st);
   if (e != cudaSuccess) return lizg::record_error(LIZG_E_CUDA, (std::string("transform: ") + cudaGetErrorString(e)).c_str());
-  r->launches += src.grid ? 4 : 5;   // sampling in the column pass adds the sampler's row and cell table
+  // captured frames add the decode's sampler or the exact walk's table; each turn past the first the sampler and the
+  // column pass again
+  const int turn = lizg::fft_turn(lizg::FftSegArgs{r->xd, src, b, frames});
+  r->launches += (src.grid ? 4 : 5) + 2 * ((frames + turn - 1) / turn - 1);
   return finish_spec(r, C, need, frames, out, st, sms);
 }
 
@@ -411,8 +437,7 @@ int lizg_rx_spectrum_grid_dev(lizg_rx *r, const float *d_grid, int frames, float
   if (int rc = lizg::device_ready(&sms)) return rc;
   lizg::SrcDev src{};
   src.grid = d_grid; src.gstride = (int64_t)r->f.n * r->f.n; src.sd = r->sd;
-  const int need = r->f.subch * lizg::kSub;
-  const lizg::FftBufs b{r->hole, r->part, r->fac, r->Y, r->tpos, need, reinterpret_cast<float2 *>(d_coef), r->ctab, &r->ymap, r->dev_err, r->beta, r->ticket, r->g16};
+  const lizg::FftBufs b = fft_bufs(r, reinterpret_cast<float2 *>(d_coef));
   cudaError_t e = lizg::fft_launch(r->xd, frames, src, b, sms, static_cast<cudaStream_t>(stream));
   r->launches = 4;
   return e == cudaSuccess ? 0 : lizg::record_error(LIZG_E_CUDA, (std::string("lizg_rx_spectrum_grid_dev: ") + cudaGetErrorString(e)).c_str());
@@ -455,7 +480,7 @@ int lizg::rx_spectrum_luma(lizg_rx *r, const uint8_t *d_luma, int w, int h, int 
   src.sd = r->sd;
   src.luma = d_luma; src.w = w; src.h = h; src.pitch = pitch; src.fstride = frame_stride; src.reg = d_reg;
   src.regstride = 9 + 2 * r->sd.nx * r->sd.ny;
-  const lizg::FftBufs b{r->hole, r->part, r->fac, r->Y, r->tpos, r->f.subch * lizg::kSub, reinterpret_cast<float2 *>(d_coef), r->ctab, &r->ymap, r->dev_err, r->beta, r->ticket, r->g16};
+  const lizg::FftBufs b = fft_bufs(r, reinterpret_cast<float2 *>(d_coef));
   const cudaError_t e = lizg::fft_launch(r->xd, frames, src, b, sms, st);
   return e == cudaSuccess ? 0 : lizg::record_error(LIZG_E_CUDA, (std::string("spectrum from frames: ") + cudaGetErrorString(e)).c_str());
 }
@@ -474,7 +499,7 @@ int lizg::rx_call(lizg_rx *r, const uint8_t *d_luma, int w, int h, int pitch, in
   src.sd = r->sd;
   src.luma = d_luma; src.w = w; src.h = h; src.pitch = pitch; src.fstride = frame_stride; src.reg = d_reg;
   src.regstride = 9 + 2 * r->sd.nx * r->sd.ny;
-  c.fft.b = FftBufs{r->hole, r->part, r->fac, r->Y, r->tpos, r->f.subch * lizg::kSub, r->C, r->ctab, &r->ymap, r->dev_err, r->beta, r->ticket, r->g16};
+  c.fft.b = fft_bufs(r, r->C);
   c.fd = fmt_dev(r, frames);
   c.tiers = r->f.tiers;
   c.out = out;

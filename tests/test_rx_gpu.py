@@ -180,3 +180,98 @@ def test_decode_of_many_frames_matches_oracle(frames):
         assert np.array_equal(out["ok"][f], res[k]["ok"]), f
         ok = res[k]["ok"].astype(bool)
         assert np.array_equal(out["blocks"][f][ok], res[k]["blocks"][ok]), f
+
+
+def _held(make):
+    """Device memory that a handle takes, in bytes."""
+    import torch
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    h = make()
+    after = torch.cuda.mem_get_info()[0]
+    del h
+    return before - after
+
+
+def test_handles_hold_no_samples_they_do_not_read():
+    """A handle's device memory a frame is its transform's, spectrum's and soft values' buffers: the decode's 16-bit samples
+    are a bounded workspace (it does not grow past 256 MB), and the handles that never read a frame by it (field
+    refinement: the exact walk; eight-parameter refinement: grids) hold none."""
+    n, subch = 1536, 1024
+    need, vrows, nx = subch * lz.SUB, int(lz.Format(n, subch, 128).uv[1::2].max()) + 1, synth.layout_nodes(128).size
+    rx = 8 * vrows * n + 8 * need + 2 * need + 16 * n * nx + 8 * (2 * n + vrows) + 20 * n + 64 * 1024   # Y, C, soft values, the walk's table, the rest
+    slack = 64 << 20   # allocations rounded up
+    lz.Receiver(n, subch, 128, max_frames=1)   # the module, the tables
+    grown = _held(lambda: lz.Receiver(n, subch, 128, max_frames=192)) - _held(lambda: lz.Receiver(n, subch, 128, max_frames=64))
+    assert grown <= 128 * rx + slack
+    assert _held(lambda: lz.Receiver(n, subch, 128, max_frames=192)) <= 192 * rx + (256 << 20) + slack
+    # field refinement: its own pictures, spectra, half-planes and partial sums beside the receiver's
+    field = rx + 4 * n * n + 8 * need + 8 * vrows * n + (1 << 20)
+    lz.FieldRefiner(n, subch, 128, chunk=1)
+    grown = _held(lambda: lz.FieldRefiner(n, subch, 128, chunk=48)) - _held(lambda: lz.FieldRefiner(n, subch, 128, chunk=16))
+    assert grown <= 32 * field + slack
+    # nine pictures a frame, with their spectra, beside the receiver's
+    gn = 9 * (rx + 4 * n * n + 8 * need)
+    lz.PilotRefiner(n, subch, 128, chunk=1)
+    grown = _held(lambda: lz.PilotRefiner(n, subch, 128, chunk=6)) - _held(lambda: lz.PilotRefiner(n, subch, 128, chunk=2))
+    assert grown <= 4 * gn + slack
+
+
+def test_batches_past_the_samples_workspace():
+    """60 frames of n = 1536 by the decode's read: more than the samples' workspace holds, so the transform takes them in
+    turns; every output as from two batches that fit, and as the engine's stage-wise run gives them."""
+    import ctypes
+    import torch
+    P = ctypes.c_void_p
+    n, subch, span, W, H, F = 1536, 1024, 128, 640, 480, 60
+    rng = np.random.default_rng(60)
+    side = span + 30
+    luma = torch.from_numpy(rng.integers(0, 256, (F, H, W), dtype=np.uint8)).cuda()
+    luma[3:5] = 128   # and frames of one grey level
+    nn = synth.layout_nodes(span).size
+    reg = np.zeros((F, 9 + 2 * nn * nn), np.float32)
+    for f in range(F):
+        s = 440.0 / side * (1 + 0.02 * rng.uniform(-1, 1))
+        reg[f, :9] = [s, 0.02 * rng.uniform(-1, 1), 90.0, 0.02 * rng.uniform(-1, 1), s, 12.0, 1e-5 * rng.uniform(-1, 1), 1e-5 * rng.uniform(-1, 1), 1]
+        reg[f, 9:] = rng.normal(0, 0.3, 2 * nn * nn)
+    reg = torch.from_numpy(reg).cuda()
+    rx = lz.Receiver(n, subch, span, max_frames=F)
+    fmt = lz.Format(n, subch, span)
+    want, _ = lz.rx_outputs(fmt, F, keep=True)
+    wcoef = torch.empty((F, subch * lz.SUB, 2), device="cuda")
+
+    def finish(f0, f1, o, coef):
+        out, s = o
+        lz._check(lz.lib().lizg_rx_finish_luma_dev(rx._h, P(luma[f0:f1].data_ptr()), W, H, W, W * H, P(reg[f0:f1].data_ptr()), f1 - f0,
+                                                   ctypes.byref(s), None, P(coef.data_ptr()), None), "lizg_rx_finish_luma_dev")
+        torch.cuda.synchronize()
+        return out
+
+    for f0 in (0, 30):
+        part = finish(f0, f0 + 30, lz.rx_outputs(fmt, 30, keep=True), wcoef[f0:f0 + 30])
+        for k in want:
+            want[k][f0:f0 + 30] = part[k]
+    coef = torch.empty_like(wcoef)
+    got = finish(0, F, lz.rx_outputs(fmt, F, keep=True), coef)
+    assert torch.equal(coef.view(torch.int32), wcoef.view(torch.int32))
+    for k in want:
+        assert np.array_equal(got[k].cpu().numpy(), want[k].cpu().numpy(), equal_nan=k in ("pilot", "est", "sub_est")), k
+    assert rx.launches == 5 + 2 + 3 + fmt.tiers   # two turns
+    # stage-wise, beside a format whose frames fit
+    eng = lz.Engine()
+    a, b = eng.add_format(n, subch, span, F), eng.add_format(384, 64, span, 4)
+    eng.set_mixed(1)
+    big, sb = lz.rx_outputs(fmt, F, keep=True)
+    small, ss = lz.rx_outputs(lz.Format(384, 64, span), 4, keep=True)
+    eng.run_dev([(a, luma.data_ptr(), W, H, W, W * H, reg.data_ptr(), F, sb),
+                 (b, luma.data_ptr(), W, H, W, W * H, reg.data_ptr(), 4, ss)], 0)
+    torch.cuda.synchronize()
+    for k in want:
+        assert np.array_equal(big[k].cpu().numpy(), want[k].cpu().numpy(), equal_nan=k in ("pilot", "est", "sub_est")), k
+    rs = lz.Receiver(384, 64, span, max_frames=4)
+    one, so = lz.rx_outputs(lz.Format(384, 64, span), 4, keep=True)
+    lz._check(lz.lib().lizg_rx_finish_luma_dev(rs._h, P(luma.data_ptr()), W, H, W, W * H, P(reg.data_ptr()), 4, ctypes.byref(so), None, None, None),
+              "lizg_rx_finish_luma_dev")
+    torch.cuda.synchronize()
+    for k in one:
+        assert np.array_equal(small[k].cpu().numpy(), one[k].cpu().numpy(), equal_nan=k in ("pilot", "est", "sub_est")), k
