@@ -388,8 +388,8 @@ struct lizg_encoder {
   int max_frames = 0, fps = 0;
   std::vector<void *> owned;
   float2 *S = nullptr;      // the row transforms, by column tiles
-  uint32_t *signs = nullptr; // the half-plane's signs
-  float *pic = nullptr, *tmp = nullptr;
+  float *pic = nullptr, *tmp = nullptr;   // the picture; the resampler's intermediate
+  uint32_t *signs = nullptr;   // the half-plane's signs, in tmp's place: read by the row transforms, before tmp is written
   uint8_t *kind = nullptr;
 };
 
@@ -513,12 +513,13 @@ lizg_encoder *lizg_encoder_new(int n, int subch, int span, int max_frames) {
   x->xf.lim = 2.0f * 2.0f * std::sqrt(0.5f * (float)(subch * kSub));   // LIZARD_CLIP 2, twice the half-plane's rms
   x->xf.sc = 0.5f / x->xf.lim;
   ok = ok && alloc(x, reinterpret_cast<void **>(&x->S), sizeof(float2) * (size_t)max_frames * e.vrows * n) &&
-       alloc(x, reinterpret_cast<void **>(&x->signs), sizeof(uint32_t) * (size_t)((max_frames + kFrameGroup - 1) / kFrameGroup) * e.vrows * n) &&
        alloc(x, reinterpret_cast<void **>(&x->pic), sizeof(float) * (size_t)max_frames * n * n) &&
        alloc(x, reinterpret_cast<void **>(&x->tmp), sizeof(float) * (size_t)max_frames * e.q * n) &&
        alloc(x, reinterpret_cast<void **>(&x->kind), (size_t)e.side * e.side);
   e.kind = x->kind;
-  ok = ok && paint_kind(x);
+  // signs: vrows n words for every kFrameGroup frames; tmp: q n floats a frame, q >= n >= 2 vrows
+  x->signs = reinterpret_cast<uint32_t *>(x->tmp);
+  ok = ok && e.q >= e.vrows && paint_kind(x);
   if (!ok) {
     lizg_encoder_free(x);
     record_error(LIZG_E_NOMEM, "lizg_encoder_new: device allocation or copy failed");

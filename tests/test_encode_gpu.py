@@ -94,3 +94,21 @@ def test_grey_alone_is_the_drive_pages_grey(n, subch, span):
         got = out.cpu().numpy()
         assert np.array_equal(got[at:at + want.size].reshape(want.shape), want), at
         assert not got[:at].any() and not got[at + want.size:].any()
+
+
+def test_encoder_holds_no_more_than_its_pictures():
+    """An encoder's device memory a frame is its transform's rows, its picture and the resampler's intermediate."""
+    import torch
+    n, subch, span = 1536, 1024, 128
+
+    def held(frames):
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        enc = lz.Encoder(n, subch, span, max_frames=frames)
+        after = torch.cuda.mem_get_info()[0]
+        del enc
+        return before - after
+
+    held(1)   # the module, the tables
+    vrows, q = int(lz.Format(n, subch, span).uv[1::2].max()) + 1, (span + 6) * 12
+    assert held(256) - held(64) <= 192 * (8 * vrows * n + 4 * n * n + 4 * q * n) + (32 << 20)
