@@ -254,3 +254,20 @@ def test_two_codeword_form_at_its_edges(rate, count, mi, si):
     wild = np.random.default_rng(count).integers(-128, 128, n, dtype=np.int64).astype(np.int8)
     llr[(count // 2) * n:(count // 2 + 1) * n] = wild
     check_against_oracle({**b, "llr": llr}, mi, si, 0.95)
+
+
+def test_variant_indices_name_their_forms():
+    """The forms a variant index names (warps a codeword; 1 the loop form, 2 the pair form, 4 the two-codeword form): an index
+    chosen by hand or saved keeps its form, the default's place apart and the one that the earlier default took."""
+    import ctypes
+    want = {6: [(4, 5), (1, 1), (2, 3), (2, 1), (2, 2), (1, 3)], 4: [(4, 5), (2, 0), (4, 0), (2, 1), (2, 2), (1, 2)],
+            3: [(4, 5), (2, 0), (4, 0), (2, 2), (1, 2)], 2: [(4, 5), (2, 0), (4, 0), (2, 2), (1, 2)]}
+    w, form = ctypes.c_int32(), ctypes.c_int32()
+    for r, forms in want.items():
+        try:
+            for v, f in enumerate(forms):
+                lz.ldpc_set_variant(r, v)
+                assert lz.lib().lizg_ldpc_variant(r, ctypes.byref(w), ctypes.byref(form)) == v
+                assert (w.value, form.value) == f, (r, v)
+        finally:
+            lz.ldpc_set_variant(r, 0)
