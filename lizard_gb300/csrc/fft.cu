@@ -295,20 +295,24 @@ __device__ __forceinline__ bool in_square(const FftDev &xd, int t) {
 // in order. A warp takes a row: its samples outside the squares summed in float as z, z c(x), z q(x) (the basis is
 // separable: 1, c(x), q(x), c(y), q(y), c(x) c(y)), then the row's six terms added in double, rows w and w + 8, then w in
 // order. The decode's read is the reference's one call over every eighth column (liblizard/src/lizard_phy.c:1611): lane l
-// takes columns l, l + 32, ..., so its homography lane is walked on eight steps from one to the next, and the at most
-// six samples' loads are in flight together. Bound: latency. A frame of n = 1536: 26 us with two rows a warp, each sample
+// takes columns l, l + 32, ..., so its homography lane is walked on eight steps from one to the next, and its G
+// samples' loads (hole_cols: 2 at n = 384, 6 at 1536) are in flight together. Bound: latency. A frame of n = 1536: 26 us with two rows a warp, each sample
 // walked from the first column, 15 so; and the column pass no longer adds the bands in every CTA (39 us, 35).
-constexpr int kHoleThreads = 32 * kHoleBand, kHoleCols = 6;
+constexpr int kHoleThreads = 32 * kHoleBand;
 static_assert(kHoleBand == 16, "rows w and w + 8 of a band share a sum");
+__host__ __device__ constexpr int hole_cols(int n) { return (n / 8 + 31) / 32; }   // a lane's columns
+struct HoleShared {
+  double red[8][6], rhs[6];
+  float row[kHoleBand][3];
+  bool last;
+};
+template <int G>
 __device__ __forceinline__ void hole_rhs_band(const FftDev &xd, const SrcDev &src, int bands, double *hole, double *beta, int *ticket, int f,
-                                              int band) {
-  __shared__ float s_row[kHoleBand][3];
-  __shared__ double s_red[8][6], s_rhs[6];
-  __shared__ bool s_last;
+                                              int band, HoleShared &sh) {
   const int n = xd.n, c = n / 8, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ky = band * kHoleBand + warp, y = 8 * ky;
   if (ky < c) {
     const bool ysq = in_square(xd, y);
-    float v[kHoleCols];
+    float v[G];
     if (src.luma && src.sd.read == LIZG_READ_DECODE) {
       const float *H = src.reg + (int64_t)f * src.regstride;
       const uint8_t *px = src.luma + f * src.fstride;
@@ -317,7 +321,7 @@ __device__ __forceinline__ void hole_rhs_band(const FftDev &xd, const SrcDev &sr
       LinNum s = lin_start(lc, r.kw, r.ku, r.kv);
       lin_steps(lc, s, lc.g);
 #pragma unroll
-      for (int m = 0; m < kHoleCols; m++) {
+      for (int m = 0; m < G; m++) {
         const int x = 8 * min(lane + 32 * m, c - 1);
         v[m] = lin_point(px, src.w, src.h, src.pitch, s, lin_cell(src.sd, H + 9, src.sd.colt[x], r.j), r.v);
 #pragma unroll
@@ -325,11 +329,11 @@ __device__ __forceinline__ void hole_rhs_band(const FftDev &xd, const SrcDev &sr
       }
     } else {
 #pragma unroll
-      for (int m = 0; m < kHoleCols; m++) v[m] = shade_at(src, f, 8 * min(lane + 32 * m, c - 1), y);
+      for (int m = 0; m < G; m++) v[m] = shade_at(src, f, 8 * min(lane + 32 * m, c - 1), y);
     }
     float s0 = 0, s1 = 0, s2 = 0;
 #pragma unroll
-    for (int m = 0; m < kHoleCols; m++) {
+    for (int m = 0; m < G; m++) {
       const int kx = lane + 32 * m, x = 8 * kx;
       if (kx < c && !(ysq && in_square(xd, x))) { s0 += v[m]; s1 += __ldg(xd.cx + x) * v[m]; s2 += __ldg(xd.qx + x) * v[m]; }
     }
@@ -338,7 +342,7 @@ __device__ __forceinline__ void hole_rhs_band(const FftDev &xd, const SrcDev &sr
       s1 += __shfl_xor_sync(0xffffffffu, s1, o);
       s2 += __shfl_xor_sync(0xffffffffu, s2, o);
     }
-    if (lane == 0) { s_row[warp][0] = s0; s_row[warp][1] = s1; s_row[warp][2] = s2; }
+    if (lane == 0) { sh.row[warp][0] = s0; sh.row[warp][1] = s1; sh.row[warp][2] = s2; }
   }
   __syncthreads();
   if (tid < 48) {
@@ -347,25 +351,25 @@ __device__ __forceinline__ void hole_rhs_band(const FftDev &xd, const SrcDev &sr
     for (int row = w; row < kHoleBand; row += 8) {
       const int kr = band * kHoleBand + row;
       if (kr >= c) break;
-      const double sv = s_row[row][k], b = r < 3 ? 1.0 : r == 4 ? xd.qx[8 * kr] : xd.cx[8 * kr];
+      const double sv = sh.row[row][k], b = r < 3 ? 1.0 : r == 4 ? xd.qx[8 * kr] : xd.cx[8 * kr];
       acc = fma(b, sv, acc);
     }
-    s_red[w][r] = acc;
+    sh.red[w][r] = acc;
   }
   __syncthreads();
   if (tid < 6) {
     double acc = 0;
-    for (int w = 0; w < 8; w++) acc += s_red[w][tid];
+    for (int w = 0; w < 8; w++) acc += sh.red[w][tid];
     __stcg(hole + ((int64_t)f * bands + band) * 6 + tid, acc);
     __threadfence();
   }
   __syncthreads();
   if (tid == 0) {
-    s_last = atomicAdd(ticket + f, 1) == bands - 1;
+    sh.last = atomicAdd(ticket + f, 1) == bands - 1;
     __threadfence();
   }
   __syncthreads();
-  if (!s_last || tid >= 32) return;
+  if (!sh.last || tid >= 32) return;
   if (tid < 6) {
     double acc = 0;
     for (int b0 = 0; b0 < bands; b0 += 12) {   // the bands' loads in flight, then added in order
@@ -375,19 +379,21 @@ __device__ __forceinline__ void hole_rhs_band(const FftDev &xd, const SrcDev &sr
 #pragma unroll
       for (int k = 0; k < 12; k++) if (b0 + k < bands) acc += v[k];
     }
-    s_rhs[tid] = acc;
+    sh.rhs[tid] = acc;
   }
   __syncwarp();
   if (tid < 6) {
     double acc = 0;
 #pragma unroll
-    for (int k = 0; k < 6; k++) acc += xd.hole_inv[tid * 6 + k] * s_rhs[k];
+    for (int k = 0; k < 6; k++) acc += xd.hole_inv[tid * 6 + k] * sh.rhs[k];
     beta[6 * f + tid] = acc;
   }
   if (tid == 0) ticket[f] = 0;   // as the next call finds it
 }
+template <int G>
 __global__ void __launch_bounds__(kHoleThreads) hole_rhs_kernel(FftDev xd, SrcDev src, int bands, double *hole, double *beta, int *ticket) {
-  hole_rhs_band(xd, src, bands, hole, beta, ticket, blockIdx.x / bands, blockIdx.x % bands);
+  __shared__ HoleShared sh;
+  hole_rhs_band<G>(xd, src, bands, hole, beta, ticket, blockIdx.x / bands, blockIdx.x % bands, sh);
 }
 
 // The transform CTA's shared memory: the lines, the twiddles, the moments' reduction.
@@ -857,12 +863,19 @@ __device__ __forceinline__ int seg_at(const int *first, int nseg, int b) {
   return k;
 }
 __global__ void __launch_bounds__(kHoleThreads, 2) fft_pre_mixed_kernel(const __grid_constant__ FftLightMix m) {
+  __shared__ HoleShared sh;
   const int b = blockIdx.x;
   if (b < m.hf[m.nseg]) {
     const int k = seg_at(m.hf, m.nseg, b);
     const FftLightSeg &g = m.seg[k];
     const int lb = b - m.hf[k];
-    hole_rhs_band(g.xd, g.src, g.bands, g.hole, g.beta, g.ticket, lb / g.bands, lb % g.bands);
+    switch (hole_cols(g.xd.n)) {
+      case 2: hole_rhs_band<2>(g.xd, g.src, g.bands, g.hole, g.beta, g.ticket, lb / g.bands, lb % g.bands, sh); break;
+      case 3: hole_rhs_band<3>(g.xd, g.src, g.bands, g.hole, g.beta, g.ticket, lb / g.bands, lb % g.bands, sh); break;
+      case 4: hole_rhs_band<4>(g.xd, g.src, g.bands, g.hole, g.beta, g.ticket, lb / g.bands, lb % g.bands, sh); break;
+      case 5: hole_rhs_band<5>(g.xd, g.src, g.bands, g.hole, g.beta, g.ticket, lb / g.bands, lb % g.bands, sh); break;
+      default: hole_rhs_band<6>(g.xd, g.src, g.bands, g.hole, g.beta, g.ticket, lb / g.bands, lb % g.bands, sh); break;
+    }
   } else {
     const int k = seg_at(m.tf, m.nseg, b);
     const FftLightSeg &g = m.seg[k];
@@ -1068,6 +1081,7 @@ template <int N>
 static cudaError_t fft_launch_n(const FftDev &xd, int frames, const SrcDev &src, const FftBufs &b, int sms, cudaStream_t st) {
   constexpr int L = plan_of(N).lines, smem = smem_bytes_of(N), tiles = N / (2 * L);
   static_assert(smem <= kFftSmemMax, "transform CTA's shared memory");
+  static_assert(hole_cols(N) >= 2 && hole_cols(N) <= 6, "the shading fit's columns a lane");
   static_assert(N % (2 * L) == 0 && L * N <= kFftPoints && kThreads % L == 0 && L <= 32, "transform plan");
   static SmemOptIn opt_cols, opt_rows;
   cudaError_t e;
@@ -1078,7 +1092,7 @@ static cudaError_t fft_launch_n(const FftDev &xd, int frames, const SrcDev &src,
   const int turn = fft_turn(all);
   if (turn < 1) return cudaErrorInvalidValue;
   const int bands = fft_hole_bands(N);
-  hole_rhs_kernel<<<frames * bands, kHoleThreads, 0, st>>>(xd, src, bands, b.hole, b.beta, b.ticket);
+  hole_rhs_kernel<hole_cols(N)><<<frames * bands, kHoleThreads, 0, st>>>(xd, src, bands, b.hole, b.beta, b.ticket);
   for (int f0 = 0; f0 < frames; f0 += turn) {
     const FftSegArgs a = fft_frames_of(all, f0, frames - f0 < turn ? frames - f0 : turn);
     if ((e = fft_read_launch(a, sms, st)) != cudaSuccess) return e;
