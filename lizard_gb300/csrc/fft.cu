@@ -396,21 +396,15 @@ __global__ void __launch_bounds__(kHoleThreads) hole_rhs_kernel(FftDev xd, SrcDe
   hole_rhs_band<G>(xd, src, bands, hole, beta, ticket, blockIdx.x / bands, blockIdx.x % bands, sh);
 }
 
-// The transform CTA's shared memory: the lines, the twiddles, the moments' reduction.
+// The transform CTA's dynamic shared memory: the lines, the twiddles.
 struct SmemMap {
   float2 *buf, *tw;
-  double *red;
 };
-__host__ __device__ constexpr int smem_bytes_of(int n) {
-  return (plan_of(n).lines * lstride_of(n) + n) * (int)sizeof(float2) + (kThreads / 32) * 6 * plan_of(n).lines * (int)sizeof(double);
-}
+__host__ __device__ constexpr int smem_bytes_of(int n) { return (plan_of(n).lines * lstride_of(n) + n) * (int)sizeof(float2); }
 template <int N>
 __device__ __forceinline__ SmemMap smem_map(unsigned char *raw) {
-  SmemMap m;
-  m.buf = reinterpret_cast<float2 *>(raw);
-  m.tw = m.buf + plan_of(N).lines * lstride_of(N);
-  m.red = reinterpret_cast<double *>(m.tw + N);
-  return m;
+  float2 *buf = reinterpret_cast<float2 *>(raw);
+  return SmemMap{buf, buf + plan_of(N).lines * lstride_of(N)};
 }
 
 __host__ __device__ constexpr int cmax_i(int x, int y) { return x > y ? x : y; }
@@ -1309,7 +1303,7 @@ __global__ void __launch_bounds__(kThreads, 3) enc_rows_kernel(EncFft e, const f
 
 template <int N, bool PAGE, bool GREY>
 static cudaError_t enc_fft_launch_n(const EncFft &e, int frames, const uint32_t *signs, float2 *S, void *pic, cudaStream_t st) {
-  constexpr int L = plan_of(N).lines, smem = (L * lstride_of(N) + N) * (int)sizeof(float2);
+  constexpr int L = plan_of(N).lines, smem = smem_bytes_of(N);
   static SmemOptIn opt_cols, opt_rows;
   cudaError_t err;
   if ((err = opt_cols.set(reinterpret_cast<const void *>(enc_cols_kernel<N, PAGE>), smem)) != cudaSuccess ||
