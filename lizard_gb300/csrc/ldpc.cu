@@ -789,6 +789,22 @@ template <int C> struct FullRows {
                                              Code<C>::MB, Code<C>::NDMAX);
   static constexpr bool all = mask == (uint32_t)((1ull << Code<C>::MB) - 1);
 };
+// The most messages that add into a data column's posterior (a parity column takes two).
+__host__ __device__ constexpr int most_messages(const uint8_t *rowptr, const uint16_t *circ, int mb) {
+  int most = 2;
+  for (int col = 0; col < 31; col++) {
+    int k = 0;
+    for (int e = 0; e < rowptr[mb]; e++) k += circ[e] >> 8 == col;
+    most = k > most ? k : most;
+  }
+  return most;
+}
+constexpr int kMessageMost = 13 * 127 / 16, kWholeMost = 2048;   // f16 holds every whole number up to the second
+static_assert(128 + kMessageMost * most_messages(LIZG_R78_ROWPTR, LIZG_R78_CIRC, Code<0>::MB) + kMessageMost < kWholeMost &&
+              128 + kMessageMost * most_messages(LIZG_R34_ROWPTR, LIZG_R34_CIRC, Code<1>::MB) + kMessageMost < kWholeMost &&
+              128 + kMessageMost * most_messages(LIZG_R23_ROWPTR, LIZG_R23_CIRC, Code<2>::MB) + kMessageMost < kWholeMost &&
+              128 + kMessageMost * most_messages(LIZG_R12_ROWPTR, LIZG_R12_CIRC, Code<3>::MB) + kMessageMost < kWholeMost,
+              "posteriors, and those less a message, are whole numbers that f16 holds exactly");
 // A row's message words: the staircase's two slots, then the circulants two a word.
 template <int C> __host__ __device__ constexpr int row_words() { return 1 + (Code<C>::NDMAX + 1) / 2; }
 
