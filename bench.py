@@ -1388,7 +1388,7 @@ def main():
     out = {
         "metric": METRIC, "value": round(value, 4), "unit": UNIT, "n_gpus": ws, "steps": args.steps, "warmup": max(args.warmup, 3),
         "ms_per_step": round(ms, 4), "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": "int8/int16", "data": "synthetic (seeded blocks over a simulated AWGN channel)", "config": workload(args.count),
+        "dtype": "int8/f16 (whole numbers, exact)", "data": "synthetic (seeded blocks over a simulated AWGN channel)", "config": workload(args.count),
         "payload_MBps": round(ws * float(ok[its > 0].sum()) * 472 / (ms / 1e3) / 1e6, 2),
         "codewords_per_s": round(ws * args.count / (ms / 1e3), 1),
         "ldpc": {"decoded": int((its > 0).sum()), "crc_ok": int(ok[its > 0].sum()), "stalled": int((its == -3).sum()),

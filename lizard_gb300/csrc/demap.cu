@@ -335,11 +335,11 @@ __device__ __forceinline__ void demap_block(const FmtDev &fd, const float2 *spec
     const float kk = (float)(0.7 * 2 * sqrt(2 * m.a2) / m.nv);
     s_k8[lane] = 8 * kk;
   }
-  asm volatile("bar.sync 1, 224;" ::: "memory");   // every warp but the second
+  asm volatile("bar.sync 1, %0;" ::"n"(kDemapThreads - 32) : "memory");   // every warp but warp 2, which has left
   int8_t *out = llrf + ((int64_t)f * fd.subch + j0) * 2 * kSubDev;
   // four coefficients in, eight soft values out, in the widest accesses the caller's buffers allow
   const bool wide = ((reinterpret_cast<uintptr_t>(src) & 15) | (reinterpret_cast<uintptr_t>(out) & 7)) == 0;
-  const int at = warp > 2 ? tid - 32 : tid;
+  const int at = warp > 2 ? tid - 32 : tid;   // this thread among the seven warps'
 #pragma unroll 4
   for (int c = at; c < subs * kSubDev / 4; c += kDemapThreads - 32) {
     float2 y[4];

@@ -30,7 +30,9 @@ namespace lizg {
 constexpr int kEncThreads = 256, kCp = 3, kQuiet = 2, kMaxCheckRows = 30;
 
 struct EncTier {
-  const uint32_t *bit;   // per coefficient that carries codeword bits: its two bits' places, 16 bits each (data bits in order, parity bit k + i mb + r at k + 128 r + i)
+  // per coefficient that carries codeword bits: its two bits' places, 16 bits each (data bits in order, parity bit
+  // k + i mb + r at k + 128 r + i)
+  const uint32_t *bit;
   const uint8_t *rowptr;
   const uint16_t *circ;
   int nt, k, m, slots, mb;
@@ -68,11 +70,12 @@ __device__ __forceinline__ uint32_t crc_mul(uint32_t a, uint32_t b) {
 
 // A block of kFrameGroup frames, one CTA: their bits, their codewords, their slots, their coefficients' signs into the
 // half-plane, a byte a frame of a word a point (the frames of a group share the place, and the scattered stores, a
-// sector each, are what a byte a store is bound by). Everything is words: a column of 128 data bits is four, a check row's
-// data bits the XOR of its circulants' columns rotated (check c = i mb + r holds data bit col z + (i - shift) mod z of row
-// r's circulants), CRC-32C (Castagnoli, reflected 0x82F63B78, liblizard/src/layout.c:44-54) a word a thread times its
-// place, the parity's running XOR over the checks (i, then r) a prefix over the rows and one over the 128 bits of their sum. 3,968 blocks (32 pages of n = 1536): 140 us a bit a byte with
-// the CRC on one thread, 92 in words a frame at a time (the stores), 27 four frames at a time.
+// sector each, are what a byte a store is bound by). Everything is words: a column of 128 data bits is four, a check
+// row's data bits the XOR of its circulants' columns rotated (check c = i mb + r holds data bit col z + (i - shift) mod
+// z of row r's circulants), CRC-32C (Castagnoli, reflected 0x82F63B78, liblizard/src/layout.c:44-54) a word a thread
+// times its place, the parity's running XOR over the checks (i, then r) a prefix over the rows and one over the 128 bits
+// of their sum. 3,968 blocks (32 pages of n = 1536): 140 us a bit a byte with the CRC on one thread, 92 in words a frame
+// at a time (the stores), 27 four frames at a time.
 constexpr int kBlockThreads = 128 * kFrameGroup, kBlockWords = 244;
 __global__ void __launch_bounds__(kBlockThreads) enc_blocks_kernel(EncDev e, const uint8_t *blocks, int frames, int pilots, uint32_t *signs) {
   // frame g's word w at [w][g]: bit t of the codeword at bit t & 31 of word t >> 5, the parity rows of 128 past the data

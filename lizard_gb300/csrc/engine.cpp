@@ -54,10 +54,10 @@ int fork_each(lizg_engine *e, const lizg_engine_batch *b, int nb, cudaStream_t s
   return 0;
 }
 
-// The stage-wise run, queued on st, every stage one launch over every format's work items (kFftMixSegs formats a
-// launch; more formats take more launches): the shading sums with the sampler's tables, the column pass, the surface
-// factors, the row pass, the pilots' fit, the soft values, the block stage, then the decode over every format's tiers,
-// the 1/2 code's first, then 2/3, 3/4, 7/8.
+// The stage-wise run, queued on st, every stage one launch over every format's work items (kFftMixSegs formats a launch;
+// more formats take more launches, and a batch past its samples' workspace the first two in turns): the shading sums
+// with the sampler or the exact walk's tables, the column pass, the surface factors, the row pass, the pilots' fit, the
+// soft values, the block stage, then the decode over every format's tiers, the 1/2 code's first, then 2/3, 3/4, 7/8.
 int run_mixed(lizg_engine *e, const lizg_engine_batch *b, int nb, cudaStream_t st) {
   int sms = 0;
   if (int rc = lizg::device_ready(&sms)) return rc;

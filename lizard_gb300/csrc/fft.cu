@@ -11,8 +11,9 @@
 //                     line of each mesh cell along it, so the column pass reads them instead of walking the mesh per
 //                     sample;
 //   fft_cols_kernel   a CTA takes 2L picture columns of a frame (L complex lines: column x0 + l real, x0 + L + l
-//                     imaginary), erases the anchors' squares to the shading surface, loads the rest, sums each column's detrend moments, transforms the L lines along y in shared
-//                     memory and separates the two real columns of each, writing Y[v][x] for the kept rows v;
+//                     imaginary), erases the anchors' squares to the shading surface, loads the rest, sums each
+//                     column's detrend moments, transforms the L lines along y in shared memory and separates the two
+//                     real columns of each, writing Y[v][x] for the kept rows v;
 //   fac_kernel        kFacCtas CTAs a frame: the five projections from the columns' moments, then the surface spectrum's
 //                     per-column and per-row factors (the double products the reference rounds to float);
 //   fft_rows_kernel   a CTA takes L kept rows v of a frame, transforms along x and subtracts the surface's spectrum
@@ -291,13 +292,14 @@ __device__ __forceinline__ bool in_square(const FftDev &xd, int t) {
 }
 
 // The shading fit's right-hand side (liblizard/src/lizard_phy.c:1609-1623) over kHoleBand of the frame's every-eighth
-// rows, hole[f][band][0..5], then, by the frame's last CTA to finish (its ticket), the surface beta[f][0..5] from the bands
-// in order. A warp takes a row: its samples outside the squares summed in float as z, z c(x), z q(x) (the basis is
-// separable: 1, c(x), q(x), c(y), q(y), c(x) c(y)), then the row's six terms added in double, rows w and w + 8, then w in
-// order. The decode's read is the reference's one call over every eighth column (liblizard/src/lizard_phy.c:1611): lane l
-// takes columns l, l + 32, ..., so its homography lane is walked on eight steps from one to the next, and its G
-// samples' loads (hole_cols: 2 at n = 384, 6 at 1536) are in flight together. Bound: latency. A frame of n = 1536: 26 us with two rows a warp, each sample
-// walked from the first column, 15 so; and the column pass no longer adds the bands in every CTA (39 us, 35).
+// rows, hole[f][band][0..5], then, by the frame's last CTA to finish (its ticket), the surface beta[f][0..5] from the
+// bands in order. A warp takes a row: its samples outside the squares summed in float as z, z c(x), z q(x) (the basis is
+// separable: 1, c(x), q(x), c(y), q(y), c(x) c(y)), then the row's six terms added in double, rows w and w + 8, then w
+// in order. The decode's read is the reference's one call over every eighth column (liblizard/src/lizard_phy.c:1611):
+// lane l takes columns l, l + 32, ..., so its homography lane is walked on eight steps from one to the next, and its G
+// samples' loads (hole_cols: 2 at n = 384, 6 at 1536) are in flight together. Bound: latency. A frame of n = 1536: 26 us
+// with two rows a warp, each sample walked from the first column, 15 so; and the column pass no longer adds the bands in
+// every CTA (39 us, 35).
 constexpr int kHoleThreads = 32 * kHoleBand;
 static_assert(kHoleBand == 16, "rows w and w + 8 of a band share a sum");
 __host__ __device__ constexpr int hole_cols(int n) { return (n / 8 + 31) / 32; }   // a lane's columns
@@ -721,9 +723,10 @@ __device__ __forceinline__ void erase_tile(const FftDev &xd, int x0, float2 *buf
   __syncthreads();
 }
 
-// The column pass on one tile (frame f, columns x0 = 2 L tile .. x0 + 2L - 1): the tile's samples (erased, projections summed: part[f][tile][0..4]), the L lines' transforms along
-// y, and the two real columns of each line separated: A(v) = (Z(v) + conj Z(n - v)) / 2, B(v) = -i (Z(v) - conj
-// Z(n - v)) / 2, written to Y[f][v][x] for the kept rows v. Every thread of the CTA takes part.
+// The column pass on one tile (frame f, columns x0 = 2 L tile .. x0 + 2L - 1): the tile's samples (erased, projections
+// summed: part[f][tile][0..4]), the L lines' transforms along y, and the two real columns of each line separated: A(v) =
+// (Z(v) + conj Z(n - v)) / 2, B(v) = -i (Z(v) - conj Z(n - v)) / 2, written to Y[f][v][x] for the kept rows v. Every
+// thread of the CTA takes part.
 template <int N>
 __device__ __forceinline__ void cols_tile(const FftDev &xd, const SrcDev &src, const float4 *ctab, const int16_t *g16, const double *beta,
                                           double *part, float2 *Y, int f, int tile, unsigned char *smraw, ColsShared &s) {
@@ -798,9 +801,11 @@ __global__ void __launch_bounds__(kThreads, 3) fft_cols_mixed_kernel(const __gri
 
 // The five projections of each frame from its column tiles' sums, normalised (liblizard/src/lizard_phy.c:1697), then the
 // surface spectrum's factors (liblizard/src/lizard_phy.c:1702-1716), rounded to float as there: fac[f] = xy[u] (pxy
-// X1[u]) for u < n, x0[u] (n (px X1[u] + pxx X2[u])) for u < n, y0[v] (n (py X1[v] + pyy X2[v])) for v < vrows. Each of a
-// frame's kFacCtas CTAs adds the tiles itself (a warp a projection, as a tree) and takes its share of the factors: one CTA
-// a frame adding the tiles in a chain held one SM's double pipe 27 us at n = 1536; 6 so (9 for 32 frames).
+// X1[u]) for u < n, x0[u] (n (px X1[u] + pxx X2[u])) for u < n, y0[v] (n (py X1[v] + pyy X2[v])) for v < vrows. Each of
+// a frame's kFacCtas CTAs adds the tiles itself (a warp a projection, as a tree) and takes its share of the factors: one
+// CTA a frame adding the tiles in a chain held one SM's double pipe 27 us at n = 1536; 6 so (9 for 32 frames). The tiles
+// are this pass's own, so no order of the reference's is at stake; the tree's sums (at most 6 in a lane, then 5 steps)
+// are nearer the exact ones than the chain's of up to 192, and both have rounded to the same factors wherever compared.
 constexpr int kFacCtas = 8;
 __device__ __forceinline__ void fac_frame(const FftDev &xd, int tiles, const double *part, float2 *fac, int f, int piece) {
   const int n = xd.n, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -832,7 +837,8 @@ __global__ void __launch_bounds__(256) fac_kernel(FftDev xd, int tiles, const do
   fac_frame(xd, tiles, part, fac, blockIdx.x / kFacCtas, blockIdx.x % kFacCtas);
 }
 
-// The shading sums, the sampler's tables and the surface factors over several formats' batches, one launch a stage:
+// The shading sums, the sampler or the exact walk's tables and the surface factors over several formats' batches, one
+// launch a stage:
 // format k's shading-band CTAs at [hf[k], hf[k + 1]), then its table CTAs at [tf[k], tf[k + 1]) (one launch takes
 // both), its frames' factor CTAs at [ff[k], ff[k + 1]).
 struct FftLightSeg {
@@ -1187,9 +1193,9 @@ cudaError_t fft_rows_mixed_launch(const FftSegArgs *a, int count, cudaStream_t s
 //
 // The half-plane spectrum's rows (v < vrows, each along u), then the picture's columns, in one of two forms. Over rows
 // (the refinement's adjoint): the spectrum complex, transformed in place, the picture row-major. PAGE (the sender): the
-// spectrum a byte a point and frame (its two signs), and both results by column tiles, a line's two columns side by side, so that
-// the column pass reads and writes runs of bytes (row by row they are 16 to 32 bytes a cache line, and the pass is bound
-// by the lines it touches: 250 us over 32 pages of n = 1536, 145 so).
+// spectrum a byte a point and frame (its two signs), and both results by column tiles, a line's two columns side by
+// side, so that the column pass reads and writes runs of bytes (row by row they are 16 to 32 bytes a cache line, and the
+// pass is bound by the lines it touches: 250 us over 32 pages of n = 1536, 145 so).
 
 // The half-plane spectrum's rows inverse-transformed: S[v][x] = sum_u S[v][u] e^{+2 pi i u x / n}, as the conjugate of the
 // forward transform of the conjugate. L rows a CTA.
@@ -1232,12 +1238,11 @@ __global__ void __launch_bounds__(kThreads, 3) enc_cols_kernel(EncFft e, const u
   static_assert(!PAGE || to % C == 0, "a butterfly's outputs in like places of their tiles");
 }
 
-// The picture's columns: 2L of them a CTA, columns xa = x0 + l and xb = x0 + L + l sharing line l as H_a + i H_b, each
-// H the column's Hermitian completion over v (H(0) = 2 Re T(0), H(v) = T(v), H(n - v) = conj T(v) for 0 < v < vrows,
-// zero between), inverse-transformed along v: the real part column xa, the imaginary part column xb
+// The picture's columns: 2L of them a CTA, columns xa = x0 + l and xb = x0 + L + l sharing line l as H_a + i H_b, each H
+// the column's Hermitian completion over v (H(0) = 2 Re T(0), H(v) = T(v), H(n - v) = conj T(v) for 0 < v < vrows, zero
+// between), inverse-transformed along v: the real part column xa, the imaginary part column xb
 // (liblizard/src/lizard_phy.c:733-773 turn_pack). Then clipped at +-lim and mapped to 0.5 + v sc (clip_row, :775-782),
-// into pic[y][x], or by column tiles (pic_at), then as they
-// are or (GREY) as the page's grey levels.
+// into pic[y][x], or by column tiles (pic_at), as they are or (GREY) as the page's grey levels.
 template <int N, bool PAGE, bool GREY>
 __global__ void __launch_bounds__(kThreads, 3) enc_rows_kernel(EncFft e, const float2 *T, void *pic) {
   extern __shared__ __align__(16) unsigned char smraw[];

@@ -7,8 +7,8 @@
 //     table, each 2 x 2 quad averaged when binned by 2.
 // Compiled with -fmad=false (the develop's float order is the reference's). The pixel formats: a CTA takes a band of
 // kBand rows, a thread four output pixels (one 16-byte load where aligned). The develop: a CTA takes a tile, its
-// source rows staged into shared memory with 16-byte loads, the gamma table beside them. Bytes in and bytes out,
-// bound by HBM.
+// source rows staged into shared memory with 16-byte loads, the gamma table beside them. The pixel formats are bound by
+// HBM, the develop by instruction issue (DRAM a third to a half busy).
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <algorithm>

@@ -752,7 +752,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) ldpc_mixed_kernel(const __grid
 // messages in registers instead, 30-80 KB of code, the instruction fetch bound the kernel (no_instruction the top
 // stall; the 1/2 code 3.75 ms on the case below).
 //
-// Bound: instruction issue (62-77% of cycles issue, ALU pipe 43-56%, shared memory 45%), 25 instructions an edge of
+// Bound: instruction issue (60-76% of cycles issue, ALU pipe 41-54%, shared memory up to 45%), 25 instructions an edge of
 // two codewords against 37-58 an edge of one in the integer forms. Measured, 16,384 codewords of one code at Eb/N0
 // 1.0-4.0 dB, the best integer form and this one, ms: 7/8 4.77, 1.71; 3/4 4.37, 1.71; 2/3 4.01, 1.79; 1/2 4.14, 2.31;
 // and 12 codewords (one a CTA, latency alone), us: 410, 73; 384, 93; 323, 112; 310, 128.

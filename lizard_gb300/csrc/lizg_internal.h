@@ -99,7 +99,7 @@ struct SampleDev {
 };
 
 // Where the transform reads a frame's picture samples from: a grid (grid set; frame f at grid + f gstride, row-major
-// n x n) or the captured frames through their registrations (the sampler fused in).
+// n x n) or the captured frames through their registrations (sampled by the handle's read).
 struct SrcDev {
   const float *grid;
   int64_t gstride;

@@ -8,8 +8,8 @@
 // 1630-1669; lens_rows 1506-1512, solve_lens 1491-1504): the four corner nodes (no displacement) and the anchors found
 // (their displacement about H), x and y about the frame's centre over its half-diagonal; the normal equations of the
 // 8 + 3 term model summed once in the points' order; each model of 0..3 radial terms solved by Gauss-Jordan; the one
-// of least AICc kept. One warp a frame: lane l sums entries l, l + 32, l + 64 of the 77 (upper triangle and right
-// side) over the points in order; lane 0 solves.
+// of least AICc kept. A block of four warps a frame: the 77 entries (upper triangle and right side) a thread each over the
+// points in order, then a warp a model.
 #include <cuda_runtime.h>
 #include <cstddef>
 #include <math.h>
@@ -628,8 +628,7 @@ __global__ void reg_redo_kernel(const RegState *st, int frames, uint8_t *redo) {
 
 // The corners searched again replace the measured ones (score 0.35 or more: the search's place, else the joint
 // model's), H made again from the four (acquire.c:2174-2195, homography 611-654), the anchors' displacements about H.
-// A CTA of kNA threads or more a frame: thread 0 the
-// corners and H, then an anchor a thread.
+// A CTA of kNA threads or more a frame: thread 0 the corners and H, then an anchor a thread.
 __global__ void __launch_bounds__(64) reg_finish_kernel(RegArgs a, float *quad_out) {
   const int f = blockIdx.x, tid = threadIdx.x;
   RegState &S = a.st[f];

@@ -84,9 +84,9 @@ cudaError_t dev_alloc(lizg_rx *r, T **dst, size_t count) {
 }
 
 // The samples' workspace: the exact walk's table of every frame (16 n nx bytes each) or, in the same place, the decode's
-// 16-bit samples (2 n^2 bytes a frame, at n = 1536 as much as the column transforms' rows) of as many frames as
-// kSampleBytes hold: 56 of n = 1536, past which a call takes the sampler and the column pass in turns of as many. Where
-// the device has not that much left, of half as many, down to one; none where the handle never reads so.
+// 16-bit samples (2 n^2 bytes a frame, 4.7 MB at n = 1536) of as many frames as kSampleBytes hold: 56 of n = 1536, past
+// which a call takes the sampler and the column pass in turns (128 frames in 3.21 ms, in one turn 3.16). Where the device
+// has not that much left, of half as many, down to one; none where the handle never reads so.
 constexpr size_t kSampleBytes = 256u << 20;
 cudaError_t samples_alloc(lizg_rx *r, bool decode) {
   const size_t frame = 2 * (size_t)r->f.n * r->f.n, table = (size_t)r->max_frames * r->f.n * r->sd.nx * sizeof(float4);
@@ -444,7 +444,7 @@ int lizg_rx_spectrum_grid_dev(lizg_rx *r, const float *d_grid, int frames, float
 }
 
 // Rows (a) to (e) on a batch of captured luma frames, each with its registration (H, then the node mesh). The
-// sampler runs inside the transform's passes (no grid in HBM) unless the caller asks for the grid.
+// samples stay the transform's own (16 bits each, or read inside its column pass) unless the caller asks for the grid.
 int lizg_rx_finish_luma_dev(lizg_rx *r, const uint8_t *d_luma, int w, int h, int pitch, int64_t frame_stride, const float *d_reg,
                             int frames, const lizg_rx_out *out, float *d_grid, float *d_coef, void *stream) {
   int sms = 0;
