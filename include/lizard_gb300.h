@@ -257,7 +257,7 @@ int lizg_rx_finish_luma_host(lizg_rx *r, const uint8_t *luma, int w, int h, int 
 // block) items of all four codes (the 1/2 code's first); 8 launches for up to 8 formats. The whole run is one CUDA
 // graph, captured on the first run with those batches. The outputs are the same bit for bit either way. That decode runs
 // the forms of one codeword, so on a GB300 a graph a format, whose decode takes two at once, is the faster (the
-// five-format tick 0.71 ms against 1.02): the choice is for fewer launches.
+// five-format tick 0.69 ms against 1.00): the choice is for fewer launches.
 // Returns the previous setting. lizg_engine_autotune first tunes each format's decode on its batch
 // (lizg_rx_autotune on the format's handle), then runs the batches both ways (each four times, the first not timed),
 // keeps the faster and returns it (0 or 1); ms (may be NULL) gets the two best times, per format first.
